@@ -17,6 +17,7 @@
 #include <string.h>
 #include <stdio.h>
 #include <math.h>
+#include <limits.h>
 #include <string>
 #include <vector>
 #include <algorithm>
@@ -206,6 +207,143 @@ static int dev_alloc(DevArr<T> &d, size_t n)
         return B200JK_OK;
 }
 
+// Streams the class kernels of one build are spread over: a class of few
+// quartets leaves most SMs idle until its longest chunk ends, so the classes
+// run side by side between a fork from and a join to the caller's stream.
+// Kernels of different classes only add to the same accumulators.
+// With one count and scan for all classes and the longest chunks drawn first
+// (ChunkLoop) a build of H2O/cc-pVDZ went from 3.66 to 0.34 ms, (H2O)8/cc-pVDZ
+// 11.5 -> 5.5 ms, (H2O)3/cc-pVTZ with two general densities 22.2 -> 7.3 ms,
+// (H2O)16/cc-pVTZ, which fills the GPU class by class, 405 -> 380 ms.
+struct StreamFan {
+        static const int N = 7;     // besides the caller's stream
+        cudaStream_t st[N] = {};
+        cudaEvent_t forked = nullptr, done[N] = {};
+        int used = 0;               // lanes of st with work since the fork
+        int lane = 0;
+        bool ready = false;
+        int create()
+        {
+                if (ready) return B200JK_OK;
+                if (!forked) CUDA_TRY(cudaEventCreateWithFlags(&forked, cudaEventDisableTiming));
+                for (int i = 0; i < N; i++) {
+                        if (!st[i]) CUDA_TRY(cudaStreamCreateWithFlags(&st[i], cudaStreamNonBlocking));
+                        if (!done[i]) CUDA_TRY(cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming));
+                }
+                ready = true;
+                return B200JK_OK;
+        }
+        int fork(cudaStream_t s)
+        {
+                CUDA_TRY(cudaEventRecord(forked, s));
+                used = 0;
+                lane = 0;
+                return B200JK_OK;
+        }
+        // the next lane in turn (the caller's stream is one of them)
+        int take(cudaStream_t s, cudaStream_t &out)
+        {
+                if (lane == N) {
+                        lane = 0;
+                        out = s;
+                        return B200JK_OK;
+                }
+                out = st[lane++];
+                if (lane > used) {
+                        used = lane;
+                        CUDA_TRY(cudaStreamWaitEvent(out, forked, 0));
+                }
+                return B200JK_OK;
+        }
+        int join(cudaStream_t s)
+        {
+                for (int i = 0; i < used; i++) {
+                        CUDA_TRY(cudaEventRecord(done[i], st[i]));
+                        CUDA_TRY(cudaStreamWaitEvent(s, done[i], 0));
+                }
+                used = 0;
+                return B200JK_OK;
+        }
+        void release()
+        {
+                for (int i = 0; i < N; i++) {
+                        if (done[i]) cudaEventDestroy(done[i]);
+                        if (st[i]) cudaStreamDestroy(st[i]);
+                        done[i] = nullptr;
+                        st[i] = nullptr;
+                }
+                if (forked) cudaEventDestroy(forked);
+                forked = nullptr;
+                ready = false;
+        }
+};
+
+// The fans of a device, lent to one build at a time (a build returns after
+// its work has ended, so a fan comes back idle).  Builds in several threads
+// hold one each; at most KEEP idle ones are kept, none once the device has no
+// plan left.  (Seven streams in every plan made creating the next plan 1.5-2
+// ms slower.)
+struct FanPool {
+        static const int KEEP = 4;
+        std::mutex mu;
+        std::vector<StreamFan *> idle;
+        int plans = 0;
+        int take(StreamFan *&out)
+        {
+                out = nullptr;
+                {
+                        std::lock_guard<std::mutex> lk(mu);
+                        if (!idle.empty()) {
+                                out = idle.back();
+                                idle.pop_back();
+                        }
+                }
+                if (!out) out = new StreamFan();
+                const int rc = out->create();
+                if (rc) give(out);
+                return rc;
+        }
+        void give(StreamFan *f)
+        {
+                if (!f) return;
+                {
+                        std::lock_guard<std::mutex> lk(mu);
+                        if (f->ready && plans > 0 && (int)idle.size() < KEEP) {
+                                idle.push_back(f);
+                                return;
+                        }
+                }
+                f->release();
+                delete f;
+        }
+        void plan_added()
+        {
+                std::lock_guard<std::mutex> lk(mu);
+                plans++;
+        }
+        void plan_removed()
+        {
+                std::vector<StreamFan *> gone;
+                {
+                        std::lock_guard<std::mutex> lk(mu);
+                        if (--plans == 0) gone.swap(idle);
+                }
+                for (StreamFan *f : gone) {
+                        f->release();
+                        delete f;
+                }
+        }
+};
+static FanPool g_fans[64];   // per device
+
+// a fan for the length of one build
+struct FanLease {
+        FanPool &pool;
+        StreamFan *fan = nullptr;
+        explicit FanLease(int device) : pool(g_fans[device]) {}
+        ~FanLease() { pool.give(fan); }
+};
+
 struct PairClassDev {
         int la = 0, lb = 0, n = 0;
         int boff[B2_NBUCKET + 1] = {0, 0, 0, 0, 0};
@@ -343,9 +481,13 @@ struct b200jk_plan {
         long long ws_gen = 0;
         DevArr<double> D, Dc, Ds, Jacc, Kacc, outJ, outK;
         DevArr<unsigned long long> dmax, stats;
+        // segments of all classes and passes of a build, counted in one launch
         DevArr<int> nkl, kst;
         DevArr<long long> nchunk, chunk_off;
         DevArr<unsigned char> cub_tmp;
+        DevArr<CountDesc> cdesc;
+        std::vector<CountDesc> h_cdesc;   // what cdesc holds
+        bool counted = false;             // among its device's plans (FanPool)
         cudaStream_t stream = nullptr;
         cudaEvent_t ev0 = nullptr, ev1 = nullptr;
         int nsm = 148;
@@ -367,6 +509,8 @@ struct b200jk_plan {
                 i1_S.release(); i1_H.release(); i1_zero.release(); i1_out.release();
                 release_fill();
                 dmax.release(); stats.release(); nkl.release(); kst.release(); nchunk.release(); chunk_off.release(); cub_tmp.release();
+                cdesc.release();
+                if (counted) g_fans[device].plan_removed();
                 for (auto e : cls_ev) cudaEventDestroy(e);
                 if (ev0) cudaEventDestroy(ev0);
                 if (ev1) cudaEventDestroy(ev1);
@@ -776,6 +920,8 @@ int b200jk_plan_create(const int32_t *atm, int natm, const int32_t *bas, int nba
         if (cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreate(&P->ev0) != cudaSuccess || cudaEventCreate(&P->ev1) != cudaSuccess)
                 return bail(fail(B200JK_ECUDA, "stream/event creation failed"));
+        g_fans[device].plan_added();   // (ensure_tables checked the index)
+        P->counted = true;
 
         // segment info and basis maps
         std::vector<int4> seg_info(segs.size());
@@ -1180,7 +1326,7 @@ int b200jk_get_q_cond(const b200jk_plan *plan, double *q_cond)
 static std::vector<const void *> workspace_key(const b200jk_plan *P)
 {
         return {P->D.p, P->Dc.p, P->Ds.p, P->Jacc.p, P->Kacc.p, P->outJ.p, P->outK.p, P->dm_cond.p, P->dmax.p,
-                P->stats.p, P->Dpk.p, P->Jpk.p, P->nkl.p, P->kst.p, P->nchunk.p, P->chunk_off.p, P->cub_tmp.p};
+                P->stats.p, P->Dpk.p, P->Jpk.p};
 }
 
 static int ensure_workspace(b200jk_plan *P, int n_dm)
@@ -1192,20 +1338,120 @@ static int ensure_workspace(b200jk_plan *P, int n_dm)
             (rc = dev_alloc(P->Ds, nc * n_dm)) || (rc = dev_alloc(P->Jacc, nc * n_dm)) ||
             (rc = dev_alloc(P->Kacc, nc * n_dm * 2)) || (rc = dev_alloc(P->outJ, nn * n_dm)) ||
             (rc = dev_alloc(P->outK, nn * n_dm)) || (rc = dev_alloc(P->dm_cond, (size_t)P->nbas * P->nbas)) ||
-            (rc = dev_alloc(P->dmax, 1)) || (rc = dev_alloc(P->stats, 4 * 64)) ||
+            (rc = dev_alloc(P->dmax, 1)) || (rc = dev_alloc(P->stats, 6 * 64)) ||
             (rc = dev_alloc(P->Dpk, (size_t)std::max<long long>(1, P->pk_total) * n_dm)) ||
             (rc = dev_alloc(P->Jpk, (size_t)std::max<long long>(1, P->pk_total) * n_dm)))
                 return rc;
-        int maxn = 1;
-        for (auto &c : P->pc) maxn = std::max(maxn, c.n * B2_NBUCKET);
-        if ((rc = dev_alloc(P->nkl, maxn)) || (rc = dev_alloc(P->kst, maxn)) || (rc = dev_alloc(P->nchunk, maxn + 1)) ||
-            (rc = dev_alloc(P->chunk_off, maxn + 1)))
-                return rc;
-        size_t tmp = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, tmp, P->nchunk.p, P->chunk_off.p, maxn + 1);
-        if ((rc = dev_alloc(P->cub_tmp, tmp + 16))) return rc;
         P->ws_ndm = std::max(P->ws_ndm, n_dm);
         if (workspace_key(P) != key0) P->ws_gen++;
+        return B200JK_OK;
+}
+
+// One launch of a build: a quartet class in one precision pass.
+struct ClassPass {
+        size_t t;                  // quartet class
+        int pass, variant;
+        CountDesc d;
+        long long nscan, max_chunk;
+};
+
+// How finely the long contractions of a class are cut (split_log2): level 2
+// where the class has fewer quartets than about four per resident lane (2048
+// lanes or 64 lane groups an SM), level 1 otherwise.
+static int split_level(const PairClassDev &bra, const PairClassDev &ket, int same, bool thread, int nsm)
+{
+        const double nq = same ? 0.5 * bra.n * (bra.n + 1.0) : (double)bra.n * ket.n;
+        return nq < 4.0 * nsm * (thread ? 512 : 64) ? 2 : 1;
+}
+
+// The passes of a build with work, their segment ranges and chunk bounds.
+static std::vector<ClassPass> class_passes(const b200jk_plan *P, int mixed, int n_dm, int nk, long long &nseg,
+                                           long long &nscan)
+{
+        std::vector<ClassPass> v;
+        auto qcs = quartet_classes();
+        nseg = nscan = 0;
+        for (size_t t = 0; t < qcs.size(); t++) {
+                const PairClassDev &bra = P->pc[qcs[t].X], &ket = P->pc[qcs[t].Y];
+                if (bra.n == 0 || ket.n == 0) continue;
+                const int la = bra.la, lb = bra.lb, lc = ket.la, ld = ket.lb;
+                const bool thread = family_is_thread(la, lb, lc, ld);
+                // pass 0: float64 quartets (all of them unless mixed);
+                // pass 1: the float32 quartets of mixed precision
+                const double tau = mixed ? class_tau(P, t) : 0.0;
+                for (int pass = 0; pass < (tau > 0 ? 2 : 1); pass++) {
+                        ClassPass c;
+                        c.t = t;
+                        c.pass = pass;
+                        // tiled chunk order for unsharded plans (with shards the
+                        // stride over bra pairs would leave tile slots idle)
+                        const int tiled = P->nshard == 1 && P->tile_b > 0;
+                        // chunk size of the family the dispatcher will pick; bra
+                        // runs (variant 2) need the tiled float64 pass of one
+                        // symmetric density, else the class runs variant 0
+                        c.variant = class_variant(P, t, pass);
+                        const int brun = family_bra_run(la, lb, lc, ld);
+                        if (c.variant == 2 && (pass == 1 || !tiled || n_dm != 1 || nk != 1 || brun <= 1 ||
+                                               P->tile_b % brun != 0))
+                                c.variant = 0;
+                        CountDesc &d = c.d;
+                        memset(&d, 0, sizeof(d));   // compared bytewise with the uploaded list
+                        d.bra = bra.view();
+                        d.ket = ket.view();
+                        d.same = qcs[t].X == qcs[t].Y;
+                        d.pass = pass;
+                        d.tau = tau;
+                        d.chunk = family_chunk(la, lb, lc, ld, c.variant);
+                        // several kets per lane and bra runs keep whole quartets on a lane
+                        d.split = thread && c.variant != 0 ? 0 : split_level(bra, ket, d.same, thread, P->nsm);
+                        d.most = thread ? 5 : 3;
+                        d.tiled = tiled;
+                        d.tile_b = P->tile_b;
+                        d.ntb = (bra.n + P->tile_b - 1) / std::max(1, P->tile_b);
+                        d.nslot = c.variant == 2 ? P->tile_b / brun : P->tile_b;
+                        d.seg0 = nseg;
+                        d.scan0 = nscan;
+                        c.nscan = tiled ? (long long)B2_NBUCKET * d.ntb : (long long)bra.n * B2_NBUCKET;
+                        c.max_chunk = 0;
+                        for (int b = 0; b < B2_NBUCKET; b++) {
+                                const int lg = d.split ? std::min(d.most, split_log2(d.split, B2_NBUCKET - 1, b)) : 0;
+                                const int len = d.chunk >> lg, nket = ket.boff[b + 1] - ket.boff[b];
+                                c.max_chunk += (long long)((nket + len - 1) / len) * (tiled ? (long long)d.ntb * d.nslot : bra.n);
+                        }
+                        nseg += (long long)bra.n * B2_NBUCKET;
+                        nscan += c.nscan;
+                        v.push_back(c);
+                }
+        }
+        return v;
+}
+
+// Buffers of the count and scan, and the class list on the device (uploaded
+// when it differs from the one there).
+static int ensure_count(b200jk_plan *P, const std::vector<ClassPass> &passes, long long nseg, long long nscan,
+                        cudaStream_t s)
+{
+        int rc;
+        if (nscan + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one build");
+        if ((rc = dev_alloc(P->nkl, (size_t)std::max(1ll, nseg))) || (rc = dev_alloc(P->kst, (size_t)std::max(1ll, nseg))) ||
+            (rc = dev_alloc(P->nchunk, (size_t)nscan + 1)) || (rc = dev_alloc(P->chunk_off, (size_t)nscan + 1)))
+                return rc;
+        size_t tmp = 0;
+        cub::DeviceScan::ExclusiveSum(nullptr, tmp, P->nchunk.p, P->chunk_off.p, (int)(nscan + 1));
+        if ((rc = dev_alloc(P->cub_tmp, tmp + 16))) return rc;
+        const bool there = P->cdesc.p && P->h_cdesc.size() == passes.size();
+        bool same = there;
+        for (size_t i = 0; same && i < passes.size(); i++) same = !memcmp(&P->h_cdesc[i], &passes[i].d, sizeof(CountDesc));
+        if (!same) {
+                std::vector<CountDesc> h;
+                for (auto &c : passes) h.push_back(c.d);
+                P->h_cdesc.clear();
+                if ((rc = dev_alloc(P->cdesc, std::max<size_t>(1, h.size())))) return rc;
+                // pageable memory: staged before the call returns
+                if (!h.empty())
+                        CUDA_TRY(cudaMemcpyAsync(P->cdesc.p, h.data(), sizeof(CountDesc) * h.size(), cudaMemcpyHostToDevice, s));
+                P->h_cdesc.swap(h);
+        }
         return B200JK_OK;
 }
 
@@ -1230,6 +1476,11 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
         cudaStream_t s = stream ? (cudaStream_t)stream : P->stream;
         const size_t nn = (size_t)P->nao * P->nao, nc = (size_t)P->naoc * P->naoc;
         const int nk = hermi == 1 ? 1 : 2;
+        long long nseg = 0, nscan = 0;
+        const std::vector<ClassPass> passes = class_passes(P, mixed, n_dm, nk, nseg, nscan);
+        FanLease lease(P->device);
+        if ((rc = ensure_count(P, passes, nseg, nscan, s)) || (rc = lease.pool.take(lease.fan))) return rc;
+        StreamFan &lanes = *lease.fan;
         CUDA_TRY(cudaEventRecord(P->ev0, s));
         const double *dD = dms;
         if (!dev_ptrs) {
@@ -1238,7 +1489,8 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
         }
         // screening data
         CUDA_TRY(cudaMemsetAsync(P->dmax.p, 0, sizeof(unsigned long long), s));
-        CUDA_TRY(cudaMemsetAsync(P->stats.p, 0, 4 * 64 * sizeof(unsigned long long), s));
+        // statistics, then the chunk queues
+        CUDA_TRY(cudaMemsetAsync(P->stats.p, 0, 6 * 64 * sizeof(unsigned long long), s));
         {
                 const long long npair = (long long)P->nbas * (P->nbas + 1) / 2;
                 dm_cond_kernel<<<grid_for(npair, 256), 256, 0, s>>>(dD, n_dm, P->nao, P->ao_loc_d.p, P->nbas,
@@ -1285,80 +1537,66 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
                 for (auto &e : P->cls_ev) CUDA_TRY(cudaEventCreate(&e));
         }
         std::vector<char> ran(qcs.size(), 0);
-        {
-                for (size_t t = 0; t < qcs.size(); t++) {
-                        const PairClassDev &bra = P->pc[qcs[t].X], &ket = P->pc[qcs[t].Y];
-                        if (bra.n == 0 || ket.n == 0) continue;
-                        int la = bra.la, lb = bra.lb, lc = ket.la, ld = ket.lb;
-                        const int same = qcs[t].X == qcs[t].Y;
-                        const int nseg = bra.n * B2_NBUCKET;
-                        if (P->profiling) CUDA_TRY(cudaEventRecord(P->cls_ev[2 * t], s));
-                        // pass 0: float64 quartets (all of them unless mixed);
-                        // pass 1: the float32 quartets of mixed precision
-                        const double tau_c = mixed ? class_tau(P, t) : 0.0;
-                        for (int pass = 0; pass < (tau_c > 0 ? 2 : 1); pass++) {
-                                // tiled chunk order for unsharded plans (with shards the
-                                // stride over bra pairs would leave tile slots idle)
-                                const int tiled = P->nshard == 1 && P->tile_b > 0;
-                                // chunk size of the family the dispatcher will pick; bra
-                                // runs (variant 2) need the tiled float64 pass of one
-                                // symmetric density, else the class runs variant 0
-                                int variant = class_variant(P, t, pass);
-                                const int brun = family_bra_run(la, lb, lc, ld);
-                                if (variant == 2 && (pass == 1 || !tiled || n_dm != 1 || nk != 1 || brun <= 1 ||
-                                                     P->tile_b % brun != 0))
-                                        variant = 0;
-                                const int chunk = family_chunk(la, lb, lc, ld, variant);
-                                count_kernel<<<grid_for(nseg, 256), 256, 0, s>>>(
-                                        bra.view(), ket.view(), same, P->tol > 0 ? P->tol : 0.0, (const double *)P->dmax.p,
-                                        chunk, tau_c, pass, P->shard, P->nshard, P->nkl.p, P->kst.p,
-                                        P->nchunk.p);
-                                CUDA_TRY(cudaGetLastError());
-                                const int ntb = (bra.n + P->tile_b - 1) / std::max(1, P->tile_b);
-                                const int nscan = tiled ? B2_NBUCKET * ntb : nseg;
-                                if (tiled) {
-                                        const int nslot = variant == 2 ? P->tile_b / brun : P->tile_b;
-                                        tile_count_kernel<<<grid_for(nscan, 256), 256, 0, s>>>(P->nkl.p, bra.n, chunk, P->tile_b,
-                                                                                             ntb, nslot, P->nchunk.p);
-                                        CUDA_TRY(cudaGetLastError());
-                                }
-                                CUDA_TRY(cudaMemsetAsync(P->nchunk.p + nscan, 0, sizeof(long long), s));
-                                size_t tmp = P->cub_tmp.n;
-                                CUDA_TRY(cub::DeviceScan::ExclusiveSum(P->cub_tmp.p, tmp, P->nchunk.p, P->chunk_off.p,
-                                                                       nscan + 1, s));
-                                JKArgs a;
-                                a.tiled = tiled;
-                                a.tile_b = P->tile_b;
-                                a.ntile = nscan;
-                                a.ntb = ntb;
-                                a.bra = bra.view();
-                                a.ket = ket.view();
-                                a.PP = P->PP.p; a.PK = P->PK.p;
-                                a.chunk_off = P->chunk_off.p;
-                                a.nkl = P->nkl.p;
-                                a.kst = P->kst.p;
-                                a.dm_cond = P->dm_cond.p;
-                                a.table = tbl;
-                                a.table_f = tbl_f;
-                                a.goff = P->goff_all.p + P->goff_at[t];
-                                a.Jacc = P->Jacc.p; a.Kacc = P->Kacc.p;
-                                a.Ds = P->Ds.p; a.Dk = P->Dc.p;
-                                a.Dpk = P->Dpk.p + P->pk_off[qcs[t].Y];
-                                a.Jpk = P->Jpk.p + P->pk_off[qcs[t].Y];
-                                a.pk_stride = P->pk_total;
-                                a.stats = P->stats.p + 2 * (64 * pass + t);
-                                a.tol = P->tol > 0 ? P->tol : -1.0;
-                                a.nbas = P->nbas; a.naoc = P->naoc; a.n_dm = n_dm; a.nk = nk;
-                                a.with_j = with_j; a.with_k = with_k; a.same = same;
-                                a.screen = P->screen;
-                                a.omega2 = P->omega2;
-                                if ((rc = dispatch_jk(P, la, lb, lc, ld, a, pass, s, nullptr, nullptr, 0, variant))) return rc;
-                                launches += 2;   // count + class kernel (the scan is a CUB library kernel)
-                        }
-                        if (P->profiling) CUDA_TRY(cudaEventRecord(P->cls_ev[2 * t + 1], s));
-                        ran[t] = 1;
-                }
+        // chunks of every class and pass: one count, one scan
+        if (nseg > 0) {
+                CUDA_TRY(cudaMemsetAsync(P->nchunk.p, 0, sizeof(long long) * (nscan + 1), s));
+                count_all_kernel<<<grid_for(nseg, 256), 256, 0, s>>>(
+                        P->cdesc.p, (int)passes.size(), nseg, P->tol > 0 ? P->tol : 0.0, (const double *)P->dmax.p,
+                        P->shard, P->nshard, P->nkl.p, P->kst.p, (unsigned long long *)P->nchunk.p);
+                CUDA_TRY(cudaGetLastError());
+                size_t tmp = P->cub_tmp.n;
+                CUDA_TRY(cub::DeviceScan::ExclusiveSum(P->cub_tmp.p, tmp, P->nchunk.p, P->chunk_off.p, (int)(nscan + 1), s));
+                launches++;
         }
+        // with class timing on, the classes run one after the other
+        const bool fan = !P->profiling;
+        if (fan && (rc = lanes.fork(s))) return rc;
+        for (size_t i = 0; i < passes.size(); i++) {
+                const ClassPass &c = passes[i];
+                const size_t t = c.t;
+                const PairClassDev &bra = P->pc[qcs[t].X], &ket = P->pc[qcs[t].Y];
+                if (P->profiling && c.pass == 0) CUDA_TRY(cudaEventRecord(P->cls_ev[2 * t], s));
+                JKArgs a;
+                a.tiled = c.d.tiled;
+                a.tile_b = P->tile_b;
+                a.ntile = c.d.tiled ? (int)c.nscan : 0;
+                a.ntb = c.d.ntb;
+                a.split = c.d.split;
+                a.max_chunk = c.max_chunk;
+                a.next = P->stats.p + 4 * 64 + 64 * c.pass + t;
+                a.bra = bra.view();
+                a.ket = ket.view();
+                a.PP = P->PP.p; a.PK = P->PK.p;
+                a.chunk_off = P->chunk_off.p + c.d.scan0;
+                a.nkl = P->nkl.p + c.d.seg0;
+                a.kst = P->kst.p + c.d.seg0;
+                a.dm_cond = P->dm_cond.p;
+                a.table = tbl;
+                a.table_f = tbl_f;
+                a.goff = P->goff_all.p + P->goff_at[t];
+                a.Jacc = P->Jacc.p; a.Kacc = P->Kacc.p;
+                a.Ds = P->Ds.p; a.Dk = P->Dc.p;
+                a.Dpk = P->Dpk.p + P->pk_off[qcs[t].Y];
+                a.Jpk = P->Jpk.p + P->pk_off[qcs[t].Y];
+                a.pk_stride = P->pk_total;
+                a.stats = P->stats.p + 2 * (64 * c.pass + t);
+                a.tol = P->tol > 0 ? P->tol : -1.0;
+                a.nbas = P->nbas; a.naoc = P->naoc; a.n_dm = n_dm; a.nk = nk;
+                a.with_j = with_j; a.with_k = with_k; a.same = c.d.same;
+                a.screen = P->screen;
+                a.omega2 = P->omega2;
+                cudaStream_t cs = s;
+                if (fan && (rc = lanes.take(s, cs))) { lanes.join(s); return rc; }
+                if ((rc = dispatch_jk(P, bra.la, bra.lb, ket.la, ket.lb, a, c.pass, cs, nullptr, nullptr, 0, c.variant))) {
+                        if (fan) lanes.join(s);
+                        return rc;
+                }
+                launches++;
+                if (P->profiling && (i + 1 == passes.size() || passes[i + 1].t != t))
+                        CUDA_TRY(cudaEventRecord(P->cls_ev[2 * t + 1], s));
+                ran[t] = 1;
+        }
+        if (fan && (rc = lanes.join(s))) return rc;
         // ket-side J from the packed blocks, then back to the output basis
         if (with_j && P->pk_total > 0) {
                 for (int d = 0; d < n_dm; d++) {
@@ -2296,7 +2534,7 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                     (rc = dev_alloc(B->segoff, std::max<size_t>(1, tot_seg))) || (rc = dev_alloc(B->nkl, max_segs)) ||
                     (rc = dev_alloc(B->kst, max_segs)) || (rc = dev_alloc(B->nchunk, max_segs + 1)) ||
                     (rc = dev_alloc(B->chunk_off, max_segs + 1)) || (rc = dev_alloc(B->mchunk, nmol + 1)) ||
-                    (rc = dev_alloc(B->stats, 4 * 64)))
+                    (rc = dev_alloc(B->stats, 6 * 64)))
                         return rc;
                 size_t cub_bytes = 0;
                 cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, B->nchunk.p, B->chunk_off.p, max_segs + 1);
@@ -2333,7 +2571,8 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                 if (with_k) CUDA_TRY(cudaMemsetAsync(P->Kacc.p, 0, sizeof(double) * nc * nk, s));
                 launches += 3;
         }
-        CUDA_TRY(cudaMemsetAsync(B->stats.p, 0, 4 * 64 * sizeof(unsigned long long), s));
+        // statistics, then the chunk queues
+        CUDA_TRY(cudaMemsetAsync(B->stats.p, 0, 6 * 64 * sizeof(unsigned long long), s));
         const double *tbl = B->tbl;
         const float *tbl_f = B->tbl_f;
         // argument arrays (pointers only depend on the workspaces): fill and upload once
@@ -2369,6 +2608,7 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                                 a.with_j = with_j; a.with_k = with_k; a.same = qcs[t].X == qcs[t].Y;
                                 a.screen = P->screen;
                                 a.omega2 = P->omega2;
+                                a.split = 1;
                                 ha[k] = a;
                                 hs[k] = seg;
                                 k++;
@@ -2395,7 +2635,8 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                         const JKArgs *dargs = B->args.p + at[2 * t + pass];
                         const int *dseg = B->segoff.p + sat[2 * t + pass];
                         const int segs = h_segoff[sat[2 * t + pass] + nm];
-                        count_kernel_multi<<<grid_for(segs, 256), 256, 0, s>>>(dargs, dseg, nm, chunk, tau,
+                        const int most = family_is_thread(la, lb, lc, ld) ? (variant == 0 ? 5 : 0) : 3;
+                        count_kernel_multi<<<grid_for(segs, 256), 256, 0, s>>>(dargs, dseg, nm, chunk, most, tau,
                                                                               pass, B->nkl.p, B->kst.p, B->nchunk.p);
                         CUDA_TRY(cudaGetLastError());
                         CUDA_TRY(cudaMemsetAsync(B->nchunk.p + segs, 0, sizeof(long long), s));
@@ -2403,7 +2644,8 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                         CUDA_TRY(cub::DeviceScan::ExclusiveSum(B->cub_tmp.p, tmp, B->nchunk.p, B->chunk_off.p, segs + 1, s));
                         batch_chunk_starts<<<grid_for(nm + 1, 128), 128, 0, s>>>(B->chunk_off.p, dseg, nm, B->mchunk.p);
                         CUDA_TRY(cudaGetLastError());
-                        const JKArgs &a0 = h_args[at[2 * t + pass]];
+                        JKArgs a0 = h_args[at[2 * t + pass]];
+                        a0.next = B->stats.p + 4 * 64 + 64 * pass + t;
                         if ((rc = dispatch_jk(B->plans[0], la, lb, lc, ld, a0, pass, s, dargs, B->mchunk.p, nm, variant)))
                                 return rc;
                         launches += 3;

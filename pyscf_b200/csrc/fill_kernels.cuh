@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(128) fill_kernel(FillArgs f, int chunk_q)
         group_load_goff<LA, LB, LC, LD, GS, double>(a.goff, gl, goff_r);
         for (long long chunk = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; chunk < total;
              chunk += nwarps) {
-                int sgi, kc;
-                if (!map_chunk(a, chunk, chunk_q, sgi, kc)) continue;
+                int sgi, kc, lg;
+                if (!map_chunk(a, chunk, chunk_q, 0, sgi, kc, lg)) continue;
                 const int ij = sgi / B2_NBUCKET;
                 const int kb = a.ket.boff[sgi % B2_NBUCKET] + a.kst[sgi];
                 const int kl0 = kb + kc * chunk_q;

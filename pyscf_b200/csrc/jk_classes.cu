@@ -12,6 +12,13 @@ namespace b200jk {
 
 namespace {
 
+// blocks of a launch: no more than its chunks can occupy
+inline int grid_of(int grid, int block, long long max_chunk)
+{
+        const long long need = (max_chunk + block / 32 - 1) / (block / 32);
+        return max_chunk > 0 && need < grid ? (int)(need > 0 ? need : 1) : grid;
+}
+
 struct LaunchCfg {
         int grid = 0, block = 128;
         size_t smem = 0;
@@ -66,9 +73,9 @@ int launch_one(const JKArgs &a, const JKArgs *margs, const long long *mchunk, in
                 return 1;
         }
         if constexpr (thread) {
-                jk_thread_kernel<LA, LB, LC, LD, NP, R, MULTI, KR><<<cfg.grid, cfg.block, cfg.smem, s>>>(a, margs, mchunk, nmol);
+                jk_thread_kernel<LA, LB, LC, LD, NP, R, MULTI, KR><<<grid_of(cfg.grid, cfg.block, a.max_chunk), cfg.block, cfg.smem, s>>>(a, margs, mchunk, nmol);
         } else {
-                jk_warp_kernel<LA, LB, LC, LD, R, MULTI, GSX><<<cfg.grid, cfg.block, cfg.smem, s>>>(
+                jk_warp_kernel<LA, LB, LC, LD, R, MULTI, GSX><<<grid_of(cfg.grid, cfg.block, a.max_chunk), cfg.block, cfg.smem, s>>>(
                         a, 8 * (32 / GSX), margs, mchunk, nmol);
         }
         cudaError_t e = cudaGetLastError();
@@ -106,7 +113,7 @@ int launch_run(const JKArgs &a, cudaStream_t s, int nsm, std::string &err)
                 err = std::string("kernel configuration: ") + cudaGetErrorString(cfg.status);
                 return 1;
         }
-        jk_thread_run_kernel<LA, LB, LC, LD, BR><<<cfg.grid, cfg.block, cfg.smem, s>>>(a);
+        jk_thread_run_kernel<LA, LB, LC, LD, BR><<<grid_of(cfg.grid, cfg.block, a.max_chunk), cfg.block, cfg.smem, s>>>(a);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
                 err = std::string("kernel launch: ") + cudaGetErrorString(e);

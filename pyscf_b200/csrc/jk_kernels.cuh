@@ -87,6 +87,16 @@ struct JKArgs {
         int screen = 0;
         // omega^2 of the long-range operator erf(omega r12)/r12, 0 = Coulomb
         double omega2 = 0.0;
+        // Dynamic chunk queue (optional): warps draw chunk numbers from this
+        // zeroed counter, last chunk first; nullptr = grid stride.
+        unsigned long long *next = nullptr;
+        // how finely segments of many primitives are cut (split_log2): 0 not,
+        // 1 the heaviest, 2 every contracted segment (classes too small to
+        // fill the GPU)
+        int split = 0;
+        // host-side bound on the chunks of the launch (0: unknown); launchers
+        // start no more warps than that
+        long long max_chunk = 0;
 };
 
 // Packed ket blocks: src[e] is the Cartesian matrix offset of packed entry e
@@ -150,6 +160,76 @@ __device__ __forceinline__ bool quartet_passes(const JKArgs &a, int4 sb, double 
 // 2 pi^{5/2}
 #define B2_TWO_PI_2P5 34.98683665524972497
 
+// A segment (bra pair, ket bucket) of long contractions is the longest serial
+// chain of a build: an (ss|ss) quartet of two 8-primitive shells evaluates
+// 64 x 64 primitive quartets, 1.06 ms on one lane, while everything else of
+// one H2O/cc-pVDZ build takes less.  The register family therefore spreads
+// the primitive quartets of such a quartet over 2^split_log2 lanes of the
+// warp (a chunk then holds that many times fewer quartets), and the group
+// family cuts its chunks down to one quartet per group.  The line is drawn by
+// the expected primitive quartets of the two buckets: at level 1 only where a
+// lane would run hundreds of them (the contraction, done by one lane of the
+// 2^s, stays below a tenth of the work); at level 2, for classes with too few
+// quartets to occupy every lane, wherever there is more than one.
+__host__ __device__ inline int split_log2(int level, int bra_bucket, int ket_bucket)
+{
+        if (level == 0) return 0;
+        // typical primitive pairs per bucket: 1, 3, 9, 30 (log2, rounded)
+        const int l2[B2_NBUCKET] = {0, 2, 3, 5};
+        const int e = l2[bra_bucket] + l2[ket_bucket];
+        if (level == 1) return e >= 10 ? 5 : (e >= 8 ? 3 : 0);
+        return e >= 5 ? 5 : e;
+}
+
+// bucket of pair ij of a class
+__device__ __forceinline__ int bucket_of(const PairView &v, int ij)
+{
+        int b = 0;
+        while (b < B2_NBUCKET - 1 && ij >= v.boff[b + 1]) b++;
+        return b;
+}
+
+// log2 of the cut of the chunks of segment sgi: at most 5 in the register
+// family (32 lanes per quartet), 3 in the group family (8 quartets per group
+// down to 1)
+__device__ __forceinline__ int segment_split(const JKArgs &a, int sgi, int most)
+{
+        if (a.split == 0) return 0;
+        return min(most, split_log2(a.split, bucket_of(a.bra, sgi / B2_NBUCKET), sgi % B2_NBUCKET));
+}
+
+// The chunks of a warp.  With a queue the chunks are drawn from the end: the
+// last ket bucket and the last bra pairs hold the longest contractions, so
+// the longest work starts first and the shortest fills the tail.
+struct ChunkLoop {
+        long long first, total, stride, cur;
+        unsigned long long *next;
+        __device__ __forceinline__ ChunkLoop(unsigned long long *next_, long long first_, long long total_)
+                : first(first_), total(total_), stride(((long long)gridDim.x * blockDim.x) >> 5),
+                  cur(first_ + (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5)), next(next_)
+        {
+        }
+        // whether any warp of this block has work (blocks past the last chunk
+        // leave before they stage their tables)
+        __device__ __forceinline__ bool block_has_work() const
+        {
+                return first + (((long long)blockIdx.x * blockDim.x) >> 5) < total;
+        }
+        __device__ __forceinline__ bool get(long long &chunk)
+        {
+                if (next) {
+                        unsigned long long k = 0;
+                        if ((threadIdx.x & 31) == 0) k = atomicAdd(next, 1ull);
+                        k = __shfl_sync(0xffffffffu, k, 0);
+                        chunk = total - 1 - (long long)k;
+                        return chunk >= first;
+                }
+                chunk = cur;
+                cur += stride;
+                return chunk < total;
+        }
+};
+
 // ---------------------------------------------------------------------------
 // Count kernel: for bra pair ij and ket bucket b, the prefix of the bucket
 // that can pass the screen, split at the mixed-precision threshold: kets with
@@ -162,25 +242,16 @@ __device__ __forceinline__ bool quartet_passes(const JKArgs &a, int4 sb, double 
 // bucket, so striding spreads the cost evenly.
 // Tiled chunk order: tile t gets tile_b x (the most chunks of its bra pairs)
 // chunk slots; slots past a bra pair's own chunks stay idle.
-// nslot chunk slots per ket chunk of a tile: tile_b (one bra pair per slot)
-// or tile_b / BR (bra runs of the register family's variant 2)
-static __global__ void tile_count_kernel(const int *__restrict__ nkl, int nbra, int chunk, int tile_b, int ntb,
-                                         int nslot, long long *tile_cnt)
-{
-        const int t = blockIdx.x * blockDim.x + threadIdx.x;
-        if (t >= B2_NBUCKET * ntb) return;
-        const int b = t / ntb, t0 = (t % ntb) * tile_b;
-        int m = 0;
-        for (int ij = t0; ij < min(nbra, t0 + tile_b); ij++) m = max(m, (nkl[ij * B2_NBUCKET + b] + chunk - 1) / chunk);
-        tile_cnt[t] = (long long)m * nslot;
-}
 
-// chunk -> (segment, chunk of the segment); false for an idle slot
-__device__ __forceinline__ bool map_chunk(const JKArgs &a, long long chunk, int chunk_len, int &sgi, int &kc)
+// chunk -> (segment, chunk of the segment, log2 of the segment's cut); the
+// segment's chunks hold chunk_len >> lg quartets.  false for an idle slot.
+__device__ __forceinline__ bool map_chunk(const JKArgs &a, long long chunk, int chunk_len, int most, int &sgi, int &kc,
+                                          int &lg)
 {
         if (!a.tiled) {
                 sgi = find_bra(a.chunk_off, a.bra.n * B2_NBUCKET, chunk);
                 kc = (int)(chunk - a.chunk_off[sgi]);
+                lg = segment_split(a, sgi, most);
                 return true;
         }
         const int t = find_bra(a.chunk_off, a.ntile, chunk);
@@ -189,7 +260,8 @@ __device__ __forceinline__ bool map_chunk(const JKArgs &a, long long chunk, int 
         const int ij = (t % a.ntb) * a.tile_b + l % a.tile_b;
         if (ij >= a.bra.n) return false;
         sgi = ij * B2_NBUCKET + t / a.ntb;
-        return kc * chunk_len < a.nkl[sgi];
+        lg = segment_split(a, sgi, most);
+        return kc * (chunk_len >> lg) < a.nkl[sgi];
 }
 
 // one (bra pair, ket bucket) segment t of a class: its ket range and chunks
@@ -251,7 +323,8 @@ static __global__ void count_kernel(PairView bra, PairView ket, int same, double
 // molecule m owns segments [segoff[m], segoff[m+1]) of the concatenated
 // nkl/kst/nchunk arrays.
 static __global__ void count_kernel_multi(const JKArgs *__restrict__ margs, const int *__restrict__ segoff, int nmol,
-                                          int chunk, double tau32, int pass, int *nkl, int *kst, long long *nchunk)
+                                          int chunk, int most, double tau32, int pass, int *nkl, int *kst,
+                                          long long *nchunk)
 {
         const int t = blockIdx.x * blockDim.x + threadIdx.x;
         if (t >= segoff[nmol]) return;
@@ -262,8 +335,9 @@ static __global__ void count_kernel_multi(const JKArgs *__restrict__ margs, cons
                 else hi = mid;
         }
         const JKArgs &a = margs[lo];
-        count_segment(a.bra, a.ket, a.same, a.tol > 0 ? a.tol : 0.0, *a.dmax4, chunk, tau32, pass, 0, 1,
-                      t - segoff[lo], nkl[t], kst[t], nchunk[t]);
+        const int sgi = t - segoff[lo];
+        count_segment(a.bra, a.ket, a.same, a.tol > 0 ? a.tol : 0.0, *a.dmax4, chunk >> segment_split(a, sgi, most),
+                      tau32, pass, 0, 1, sgi, nkl[t], kst[t], nchunk[t]);
 }
 
 // first chunk of every molecule of a batch: mchunk[m] = chunk_off[segoff[m]]
@@ -271,6 +345,43 @@ static __global__ void batch_chunk_starts(const long long *chunk_off, const int 
 {
         const int m = blockIdx.x * blockDim.x + threadIdx.x;
         if (m <= nmol) mchunk[m] = chunk_off[segoff[m]];
+}
+
+// All quartet classes (and precision passes) of one build counted in one
+// launch: segment t of the flat list belongs to the pass whose seg0 range
+// holds it.  cnt (zeroed by the caller) receives the chunk slots, per tile
+// (tiled: the most chunks of its bra pairs times the slots per ket chunk) or
+// per segment; one scan over cnt then gives every pass its chunk offsets.
+struct CountDesc {
+        PairView bra, ket;
+        long long seg0, scan0;       // first segment, first entry of cnt
+        double tau;
+        int same, pass, chunk, split, most;
+        int tiled, tile_b, ntb, nslot;
+};
+
+static __global__ void count_all_kernel(const CountDesc *__restrict__ desc, int nd, long long nseg, double tol,
+                                        const double *dmax4, int shard, int nshard, int *nkl, int *kst,
+                                        unsigned long long *cnt)
+{
+        const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+        if (t >= nseg) return;
+        int lo = 0, hi = nd;   // desc[lo].seg0 <= t < desc[hi].seg0
+        while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (desc[mid].seg0 <= t) lo = mid;
+                else hi = mid;
+        }
+        const CountDesc &d = desc[lo];
+        const int sgi = (int)(t - d.seg0);
+        const int ij = sgi / B2_NBUCKET, b = sgi % B2_NBUCKET;
+        const int lg = d.split ? min(d.most, split_log2(d.split, bucket_of(d.bra, ij), b)) : 0;
+        long long nc;
+        count_segment(d.bra, d.ket, d.same, tol, *dmax4, d.chunk >> lg, d.tau, d.pass, shard, nshard, sgi, nkl[t],
+                      kst[t], nc);
+        if (!d.tiled) cnt[d.scan0 + sgi] = (unsigned long long)nc;
+        else if (nc > 0)
+                atomicMax(cnt + d.scan0 + (long long)b * d.ntb + ij / d.tile_b, (unsigned long long)(nc * d.nslot));
 }
 
 // ---------------------------------------------------------------------------
@@ -340,6 +451,9 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk
         // small (float64 up to four roots, <= 59 KB; float32 always, <= 27 KB),
         // read from global memory otherwise
         extern __shared__ __align__(32) double smem_dyn[];
+        ChunkLoop loop(a0.next, MULTI ? 0 : a0.chunk_off[0],
+                       MULTI ? mchunk[nmol] : a0.chunk_off[a0.tiled ? a0.ntile : a0.bra.n * B2_NBUCKET]);
+        if (!loop.block_has_work()) return;
         const R *tab = table_of<R>(a0) + RysLayout<R>::offset(K::NR);
         if constexpr (stage_table<R>(K::NR)) {
                 constexpr int NS = rys_slice_elems<R>(K::NR);
@@ -349,18 +463,16 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk
                 __syncthreads();
                 tab = reinterpret_cast<const R *>(smem_dyn);
         }
-        const long long total = MULTI ? mchunk[nmol] : a0.chunk_off[a0.tiled ? a0.ntile : a0.bra.n * B2_NBUCKET];
-        const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
         unsigned long long nq = 0, npq = 0;
-        for (long long chunk = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; chunk < total;
-             chunk += nwarps) {
+        long long chunk;
+        while (loop.get(chunk)) {
               auto body = [&](const JKArgs &a) {
-                const int nseg = a.bra.n * B2_NBUCKET;
                 const size_t n = (size_t)a.naoc, nn = n * n;
                 constexpr int M = KR;
-                int sgi, kc;
-                if (!map_chunk(a, chunk, 32 * M, sgi, kc)) return;
-                (void)nseg;
+                // 2^lg lanes share a quartet's primitive quartets (one ket per lane only)
+                int sgi, kc, lg;
+                if (!map_chunk(a, chunk, 32 * M, M == 1 ? 5 : 0, sgi, kc, lg)) return;
+                const int nsub = 1 << lg, sub = lane & (nsub - 1);
                 const int ij = sgi / B2_NBUCKET;
                 const bool carry = M > 1 && a.n_dm == 1 && a.nk == 1 && a.with_k;
                 double acc_a[K::NA * K::NC], acc_b[K::NB * K::NC];
@@ -380,7 +492,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk
                                         atomicAdd(a.Kacc + (sb0.y + b) * n + cur_c + c, acc_b[b * K::NC + c]);
                 };
               for (int jk = 0; jk < M; jk++) {
-                const int pos = kc * (32 * M) + lane * M + jk;
+                const int pos = M == 1 ? kc * (32 >> lg) + (lane >> lg) : kc * (32 * M) + lane * M + jk;
                 const int kl = a.ket.boff[sgi % B2_NBUCKET] + a.kst[sgi] + pos;
                 const int4 sb = a.bra.sh[ij];
                 const int2 pb = a.bra.pr[ij];
@@ -409,9 +521,13 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk
                         if (a.same && ij == kl) fac *= (R)0.5;
                         C[0] = (R)(Ak.x - Ab.x); C[1] = (R)(Ak.y - Ab.y); C[2] = (R)(Ak.z - Ab.z);
                         CD[0] = (R)CDk.x; CD[1] = (R)CDk.y; CD[2] = (R)CDk.z;
-                        nq++;
-                        npq += (unsigned long long)pb.y * pk.y;
+                        if (sub == 0) {
+                                nq++;
+                                npq += (unsigned long long)pb.y * pk.y;
+                        }
                 }
+                // the lane that contracts the quartet
+                const bool lead = active && sub == 0;
                 const int ia = sb.x, ib = sb.y, ic = sk.x, id = sk.y;
                 if (carry && active && ic != cur_c) {
                         flush();
@@ -428,12 +544,15 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk
 #pragma unroll
                         for (int t = 0; t < NGP; t++) Gp[t] = (R)0;
                         if (active) {
-                                for (int ip = 0; ip < pb.y; ip++) {
+                                // primitive quartets sub, sub + nsub, ... of the bra-major list
+                                int ip = 0, kp = sub;
+                                while (kp >= pk.y) { kp -= pk.y; ip++; }
+                                while (ip < pb.y) {
                                         const double4 P = a.PP[pb.x + ip];
                                         const double2 KP = a.PK[pb.x + ip];
                                         const R Kab = (R)KP.x * fac;
                                         const R Pv[3] = {(R)(P.x - Ab.x), (R)(P.y - Ab.y), (R)(P.z - Ab.z)};
-                                        for (int kp = 0; kp < pk.y; kp++) {
+                                        for (; kp < pk.y; kp += nsub) {
                                                 const double4 Q = a.PP[pk.x + kp];
                                                 const double2 KQ = a.PK[pk.x + kp];
                                                 const R Qv[3] = {(R)(Q.x - Ab.x), (R)(Q.y - Ab.y), (R)(Q.z - Ab.z)};
@@ -442,14 +561,20 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk
                                                               Kab * (R)KQ.x, (R)a.omega2);
                                                 add_prim_quartet_part<LA, LB, LC, LD, PART * NGP, NGP, R>(Gp, tab, sq, AB, CD);
                                         }
+                                        while (kp >= pk.y) { kp -= pk.y; ip++; }
                                 }
+                        }
+                        if constexpr (M == 1) {
+                                for (int o = 1; o < nsub; o <<= 1)
+#pragma unroll
+                                        for (int t = 0; t < NGP; t++) Gp[t] += __shfl_xor_sync(0xffffffffu, Gp[t], o);
                         }
                         // Gp[((x*NB + b)*NC + c)*ND + d] holds bra component A0 + x
                         for (int s = 0; s < a.n_dm; s++) {
                                 if (a.with_j) {
                                         const double *Ds = a.Ds + s * nn;
                                         double *J = a.Jacc + s * nn;
-                                        if (active) {
+                                        if (lead) {
                                                 double dab[NAP * K::NB];
 #pragma unroll
                                                 for (int x = 0; x < NAP; x++)
@@ -472,7 +597,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk
                                         for (int x = 0; x < K::NC; x++)
 #pragma unroll
                                                 for (int y = 0; y < K::ND; y++)
-                                                        dcd[x * K::ND + y] = !active ? 0.0
+                                                        dcd[x * K::ND + y] = !lead ? 0.0
                                                                 : (a.Dpk ? __ldg(a.Dpk + s * a.pk_stride + (long long)kl * K::NCD + x * K::ND + y)
                                                                          : __ldg(Ds + (ic + x) * n + id + y));
 #pragma unroll
@@ -485,7 +610,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk
                                                         atomicAdd(J + (ia + A0 + t / K::NB) * n + ib + t % K::NB, v);
                                         }
                                 }
-                                if (a.with_k && active) {
+                                if (a.with_k && lead) {
                                         for (int tk = 0; tk < a.nk; tk++) {
                                                 const double *X = a.Dk + (s * a.nk + tk) * nn;
                                                 double *Kt = a.Kacc + (s * a.nk + tk) * nn;
@@ -620,6 +745,8 @@ __global__ void __launch_bounds__(128, B2_THREAD_MINB) jk_thread_run_kernel(JKAr
         constexpr int NG = K::NG;
         const int lane = threadIdx.x & 31;
         extern __shared__ __align__(32) double smem_dyn[];
+        ChunkLoop loop(a.next, a.chunk_off[0], a.chunk_off[a.ntile]);
+        if (!loop.block_has_work()) return;
         const double *tab = a.table + RysLayout<double>::offset(K::NR);
         if constexpr (stage_table<double>(K::NR)) {
                 constexpr int NS = rys_slice_elems<double>(K::NR);
@@ -631,11 +758,9 @@ __global__ void __launch_bounds__(128, B2_THREAD_MINB) jk_thread_run_kernel(JKAr
         }
         const size_t n = (size_t)a.naoc;
         const int nrun = a.tile_b / BR;   // runs per tile
-        const long long total = a.chunk_off[a.ntile];
-        const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
         unsigned long long nq = 0, npq = 0;
-        for (long long chunk = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; chunk < total;
-             chunk += nwarps) {
+        long long chunk;
+        while (loop.get(chunk)) {
                 const int t = find_bra(a.chunk_off, a.ntile, chunk);
                 const int l = (int)(chunk - a.chunk_off[t]);
                 const int kc = l / nrun, run = l % nrun;
@@ -1073,8 +1198,9 @@ __global__ void __launch_bounds__(128, (warp_min_blocks<LA, LB, LC, LD, R, GS_>(
         const unsigned gmask = GS == 32 ? 0xffffffffu : (((1u << GS) - 1u) << (grp * GS));
         const int wib = threadIdx.x >> 5;
         double *sm = smem_dyn + (size_t)(wib * NGRP + grp) * S::SIZE;
-        const long long total = MULTI ? mchunk[nmol] : a0.chunk_off[a0.tiled ? a0.ntile : a0.bra.n * B2_NBUCKET];
-        const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+        ChunkLoop loop(a0.next, MULTI ? 0 : a0.chunk_off[0],
+                       MULTI ? mchunk[nmol] : a0.chunk_off[a0.tiled ? a0.ntile : a0.bra.n * B2_NBUCKET]);
+        if (!loop.block_has_work()) return;
         unsigned long long nq = 0, npq = 0;
         // offsets of this lane's components (the same for every molecule of a batch)
         int goff_r[group_goff_regs<LA, LB, LC, LD, GS, R>()];
@@ -1083,18 +1209,17 @@ __global__ void __launch_bounds__(128, (warp_min_blocks<LA, LB, LC, LD, R, GS_>(
         // each lane sums its J[a,b] components over the chunk and the groups
         // of the warp combine them before one atomic per element
         constexpr int NJB = sizeof(R) == 8 ? (K::NAB + GS - 1) / GS : 1;
-        for (long long chunk = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; chunk < total;
-             chunk += nwarps) {
+        long long chunk;
+        while (loop.get(chunk)) {
               auto body = [&](const JKArgs &a) {
-                const int nseg = a.bra.n * B2_NBUCKET;
                 const size_t n = (size_t)a.naoc, nn = n * n;
-                int sgi, kc;
-                if (!map_chunk(a, chunk, chunk_q, sgi, kc)) return;
-                (void)nseg;
+                int sgi, kc, lg;
+                if (!map_chunk(a, chunk, chunk_q, 3, sgi, kc, lg)) return;
+                const int cq = chunk_q >> lg;
                 const int ij = sgi / B2_NBUCKET;
                 const int kb = a.ket.boff[sgi % B2_NBUCKET] + a.kst[sgi];
-                const int kl0 = kb + kc * chunk_q;
-                const int kl1 = kb + min(kc * chunk_q + chunk_q, a.nkl[sgi]);
+                const int kl0 = kb + kc * cq;
+                const int kl1 = kb + min(kc * cq + cq, a.nkl[sgi]);
                 const int4 sb = a.bra.sh[ij];
                 const int2 pb = a.bra.pr[ij];
                 const double qij = a.bra.q[ij];

@@ -1,0 +1,109 @@
+"""The J/K build's chunking and scheduling: long contractions whose primitive
+quartets are spread over lanes, every chunk order, builds in several threads.
+
+Reference: the CPU oracle.  Tolerance 1e-10 on elements of order 1-10, the
+parity bound of the FP64 kernels (sums of ~1e5 terms of 1e-16 relative
+rounding each stay three orders below it)."""
+import threading
+
+import numpy
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-10
+
+
+@pytest.fixture(scope='module')
+def b2():
+    from pyscf_b200 import lib
+    if lib.device_count() == 0:
+        pytest.skip('no GPU')
+    return lib
+
+
+def contracted_molecule(nprims, l_of, ncopy=1, nctr=1):
+    """atm, bas, env: one shell of nprims[k] primitives and angular momentum
+    l_of[k] on its own atom, `ncopy` times over, about 1.5 Bohr apart."""
+    rng = numpy.random.default_rng(42)
+    env = [0.0] * 20
+    atm, bas = [], []
+    for c in range(ncopy):
+        for k, (n, l) in enumerate(zip(nprims, l_of)):
+            r = numpy.array([1.5 * k, 1.7 * c, 0.3 * (k + c)]) + rng.uniform(-0.1, 0.1, 3)
+            atm.append([1, len(env), 1, len(env) + 3, 0, 0])
+            env += list(r) + [0.0]
+            e = 0.25 * 2.3 ** numpy.arange(n)
+            bas.append([len(atm) - 1, l, n, nctr, 0, len(env), len(env) + n, 0])
+            env += list(e) + list(rng.uniform(0.2, 1.0, n * nctr) / n)
+    return (numpy.array(atm, dtype=numpy.int32), numpy.array(bas, dtype=numpy.int32), numpy.array(env))
+
+
+def densities(nao, n):
+    rng = numpy.random.default_rng(7)
+    return rng.standard_normal((n, nao, nao)) / numpy.sqrt(nao)
+
+
+# primitive pairs 1, 2, 4, 5, 16, 17, 81: both sides of every bucket's edge
+@pytest.mark.parametrize('nprims,l_of,nctr', [
+    ((1, 2, 4, 9), (0, 0, 0, 0), 1),
+    ((1, 3, 5, 9), (1, 0, 1, 0), 1),
+    ((2, 4, 1, 9), (2, 1, 0, 0), 1),
+    ((4, 17, 1), (1, 0, 2), 2),
+])
+@pytest.mark.parametrize('hermi,n_dm', [(1, 1), (0, 2)])
+def test_long_contractions(b2, nprims, l_of, nctr, hermi, n_dm):
+    atm, bas, env = contracted_molecule(nprims, l_of, nctr=nctr)
+    plan = b2.Plan(atm, bas, env, direct_scf_tol=1e-13)
+    d = densities(plan.nao, n_dm)
+    if hermi == 1:
+        d = d + d.transpose(0, 2, 1)
+    vj, vk = plan.get_jk(d, hermi=hermi)
+    for s in range(n_dm):
+        rj, rk, _ = oracle.get_jk(d[s], atm, bas, env, hermi=hermi)
+        assert abs(vj[s] - rj).max() < TOL
+        assert abs(vk[s] - rk).max() < TOL
+
+
+@pytest.mark.parametrize('tile', [0, 1, 5, 64])
+@pytest.mark.parametrize('precision', [0, 1])
+def test_chunk_orders(b2, tile, precision):
+    """Every tile size, both precisions and a J-only / K-only build give the
+    default order's J and K (mixed: every quartet in float64, tau = 0)."""
+    atm, bas, env = contracted_molecule((1, 3, 9, 1), (1, 0, 0, 2), ncopy=6)
+    plan = b2.Plan(atm, bas, env, direct_scf_tol=1e-13)
+    d = densities(plan.nao, 1)[0]
+    d = d + d.T
+    rj, rk = plan.get_jk(d, hermi=1)
+    nq = plan.stats()['quartets']
+    plan.set_tile(tile)
+    plan.set_mixed_threshold(0.0)
+    for kw in ({}, {'with_k': False}, {'with_j': False}):
+        vj, vk = plan.get_jk(d, hermi=1, precision=precision, **kw)
+        assert plan.stats()['quartets'] == nq
+        assert vj is None or abs(vj - rj).max() < TOL
+        assert vk is None or abs(vk - rk).max() < TOL
+
+
+def test_threads(b2):
+    """Builds of different plans in several threads at once (each holds its
+    own set of streams) give what they give alone."""
+    atm, bas, env = contracted_molecule((1, 3, 9, 1), (1, 0, 0, 2), ncopy=3)
+    plans = [b2.Plan(atm, bas, env, direct_scf_tol=1e-13) for _ in range(6)]
+    d = densities(plans[0].nao, 6)
+    want = [plans[0].get_jk(x + x.T, hermi=1) for x in d]
+    bad = []
+
+    def work(k):
+        for _ in range(5):
+            vj, vk = plans[k].get_jk(d[k] + d[k].T, hermi=1)
+            if abs(vj - want[k][0]).max() > TOL or abs(vk - want[k][1]).max() > TOL:
+                bad.append(k)
+
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(6)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
