@@ -388,6 +388,7 @@ struct GradPlan {
         DevArr<int> nkl, kst;
         DevArr<long long> nchunk, chunk_off;
         DevArr<unsigned char> cub_tmp;
+        DevArr<CountDesc> cdesc;
         int64_t quartets = 0, prim_quartets = 0, launches = 0;
         double last_ms = 0;
         std::vector<b200jk_class_stat_t> cls;   // per (bra class, ket class)
@@ -401,7 +402,7 @@ struct GradPlan {
                 q0.release(); goff.release(); D.release(); Dc.release(); Ds.release(); V.release(); out.release();
                 de.release(); shell_atom.release();
                 dmc.release(); fac.release(); dmax.release(); stats.release(); nkl.release(); kst.release();
-                nchunk.release(); chunk_off.release(); cub_tmp.release();
+                nchunk.release(); chunk_off.release(); cub_tmp.release(); cdesc.release();
         }
 };
 
@@ -2176,21 +2177,64 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
         if ((rc = ensure_grad(P, tol))) return rc;
         GradPlan &g = P->grad;
         const size_t nn = (size_t)P->nao * P->nao, nc = (size_t)P->naoc * P->naoc;
-        int maxn = 1;
-        for (auto &c : g.bra) maxn = std::max(maxn, c.n * B2_NBUCKET);
+        // every (bra class, ket class) with work: segments and chunks counted in
+        // one launch, as in b200jk_get_jk
+        struct Pass {
+                int X, Y;
+                CountDesc d;
+                long long max_chunk;
+        };
+        std::vector<Pass> passes;
+        long long nseg_all = 0;
+        for (int X = 0; X < NPAIRCLASS; X++)
+                for (int Y = 0; Y < NPAIRCLASS; Y++) {
+                        const PairClassDev &bra = g.bra[X], &ket = g.ket[Y];
+                        if (bra.n == 0 || ket.n == 0) continue;
+                        Pass p;
+                        p.X = X;
+                        p.Y = Y;
+                        CountDesc &d = p.d;
+                        memset(&d, 0, sizeof(d));
+                        d.bra = bra.view();
+                        d.ket = ket.view();
+                        d.chunk = grad_chunk(bra.la, bra.lb, ket.la, ket.lb, fused);
+                        d.split = split_level(bra, ket, 0, grad_register_family(bra.la, bra.lb, ket.la, ket.lb, fused), P->nsm);
+                        d.most = d.chunk == 32 ? 5 : (d.chunk == 16 ? 4 : 3);
+                        d.seg0 = d.scan0 = nseg_all;
+                        p.max_chunk = 0;
+                        for (int b = 0; b < B2_NBUCKET; b++) {
+                                const int len = d.chunk >> std::min(d.most, split_log2(d.split, B2_NBUCKET - 1, b));
+                                p.max_chunk += (long long)((ket.boff[b + 1] - ket.boff[b] + len - 1) / len) * bra.n;
+                        }
+                        nseg_all += (long long)bra.n * B2_NBUCKET;
+                        passes.push_back(p);
+                }
+        if (nseg_all + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one build");
+        const size_t NQ = NPAIRCLASS * NPAIRCLASS;
         if (fused && ((rc = dev_alloc(g.de, (size_t)3 * P->natm)) || (!g.shell_atom.p && (rc = dev_upload(g.shell_atom, P->shell_atom)))))
                 return rc;
         if ((rc = dev_alloc(g.D, nn * n_dm)) || (rc = dev_alloc(g.Dc, nc * n_dm)) || (rc = dev_alloc(g.Ds, nc * n_dm)) ||
             (rc = dev_alloc(g.V, fused ? 1 : 6 * nc * n_dm)) || (rc = dev_alloc(g.out, dev_ptrs || fused ? 1 : 6 * nn * n_dm)) ||
             (rc = dev_alloc(g.dmc, (size_t)P->nbas * P->nbas)) || (rc = dev_alloc(g.fac, 1)) ||
-            (rc = dev_alloc(g.dmax, 1)) || (rc = dev_alloc(g.stats, 2 * NPAIRCLASS * NPAIRCLASS)) || (rc = dev_alloc(g.nkl, maxn)) ||
-            (rc = dev_alloc(g.kst, maxn)) || (rc = dev_alloc(g.nchunk, maxn + 1)) || (rc = dev_alloc(g.chunk_off, maxn + 1)))
+            (rc = dev_alloc(g.dmax, 1)) || (rc = dev_alloc(g.stats, 3 * NQ)) ||
+            (rc = dev_alloc(g.nkl, (size_t)std::max(1ll, nseg_all))) || (rc = dev_alloc(g.kst, (size_t)std::max(1ll, nseg_all))) ||
+            (rc = dev_alloc(g.nchunk, (size_t)nseg_all + 1)) || (rc = dev_alloc(g.chunk_off, (size_t)nseg_all + 1)) ||
+            (rc = dev_alloc(g.cdesc, std::max<size_t>(1, passes.size()))))
                 return rc;
         size_t cub_bytes = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, g.nchunk.p, g.chunk_off.p, maxn + 1);
+        cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, g.nchunk.p, g.chunk_off.p, (int)(nseg_all + 1));
         if ((rc = dev_alloc(g.cub_tmp, cub_bytes + 16))) return rc;
+        FanLease lease(P->device);
+        if ((rc = lease.pool.take(lease.fan))) return rc;
+        StreamFan &lanes = *lease.fan;
 
         cudaStream_t s = stream ? (cudaStream_t)stream : P->stream;
+        if (!passes.empty()) {
+                std::vector<CountDesc> h;
+                for (const Pass &p : passes) h.push_back(p.d);
+                // pageable memory: staged before the call returns
+                CUDA_TRY(cudaMemcpyAsync(g.cdesc.p, h.data(), sizeof(CountDesc) * h.size(), cudaMemcpyHostToDevice, s));
+        }
         CUDA_TRY(cudaEventRecord(P->ev0, s));
         const double *dD = dms;
         if (!dev_ptrs) {
@@ -2198,7 +2242,8 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
                 dD = g.D.p;
         }
         CUDA_TRY(cudaMemsetAsync(g.dmax.p, 0, sizeof(unsigned long long), s));
-        CUDA_TRY(cudaMemsetAsync(g.stats.p, 0, 2 * NPAIRCLASS * NPAIRCLASS * sizeof(unsigned long long), s));
+        // statistics, then the chunk queues
+        CUDA_TRY(cudaMemsetAsync(g.stats.p, 0, 3 * NQ * sizeof(unsigned long long), s));
         if (P->profiling && g.cls_ev.empty()) {
                 g.cls_ev.resize(2 * NPAIRCLASS * NPAIRCLASS);
                 for (auto &e : g.cls_ev) CUDA_TRY(cudaEventCreate(&e));
@@ -2224,50 +2269,59 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
         if (fused) CUDA_TRY(cudaMemsetAsync(g.de.p, 0, sizeof(double) * 3 * P->natm, s));
         else CUDA_TRY(cudaMemsetAsync(g.V.p, 0, sizeof(double) * 6 * nc * n_dm, s));
         double *Vj = fused ? nullptr : g.V.p, *Vk = fused ? nullptr : g.V.p + 3 * nc * n_dm;
-        for (int X = 0; X < NPAIRCLASS; X++) {
-                const PairClassDev &bra = g.bra[X];
-                if (bra.n == 0) continue;
-                for (int Y = 0; Y < NPAIRCLASS; Y++) {
-                        const PairClassDev &ket = g.ket[Y];
-                        if (ket.n == 0) continue;
-                        const int nseg = bra.n * B2_NBUCKET;
-                        const int chunk = grad_chunk(bra.la, bra.lb, ket.la, ket.lb, fused);
-                        count_kernel<<<grid_for(nseg, 256), 256, 0, s>>>(bra.view(), ket.view(), 0, tol, g.fac.p, chunk,
-                                                                        0.0, 0, P->shard, P->nshard, g.nkl.p, g.kst.p,
-                                                                        g.nchunk.p);
-                        CUDA_TRY(cudaGetLastError());
-                        CUDA_TRY(cudaMemsetAsync(g.nchunk.p + nseg, 0, sizeof(long long), s));
-                        size_t tmp = g.cub_tmp.n;
-                        CUDA_TRY(cub::DeviceScan::ExclusiveSum(g.cub_tmp.p, tmp, g.nchunk.p, g.chunk_off.p, nseg + 1, s));
-                        GradArgs a;
-                        a.bra = bra.view();
-                        a.ket = ket.view();
-                        a.PP = P->PP.p; a.PK = P->PK.p; a.PE = P->PE.p;
-                        a.chunk_off = g.chunk_off.p;
-                        a.nkl = g.nkl.p;
-                        a.kst = g.kst.p;
-                        a.q0 = g.q0.p;
-                        a.q1 = P->qcond.p;
-                        a.dmc = g.dmc.p;
-                        a.table = table_ptr();
-                        a.goff = g.goff.p + g.goff_at[X * NPAIRCLASS + Y];
-                        a.Vj = Vj; a.Vk = Vk;
-                        a.Ds = g.Ds.p; a.Dc = g.Dc.p;
-                        a.stats = g.stats.p + 2 * (X * NPAIRCLASS + Y);
-                        a.tol = tol > 0 ? tol : -1.0;
-                        a.nbas = P->nbas; a.naoc = P->naoc; a.n_dm = n_dm;
-                        a.with_j = with_j; a.with_k = with_k;
-                        a.de = fused ? g.de.p : nullptr;
-                        a.omega2 = P->omega2;
-                        a.shell_atom = fused ? g.shell_atom.p : nullptr;
-                        std::string err;
-                        if (P->profiling) CUDA_TRY(cudaEventRecord(g.cls_ev[2 * (X * NPAIRCLASS + Y)], s));
-                        if (g_grad_launch[X](ket.la, ket.lb, a, s, P->nsm, err)) return fail(B200JK_ECUDA, err);
-                        if (P->profiling) CUDA_TRY(cudaEventRecord(g.cls_ev[2 * (X * NPAIRCLASS + Y) + 1], s));
-                        ran[X * NPAIRCLASS + Y] = 1;
-                        launches += 2;   // count + class kernel (the scan is a CUB library kernel)
-                }
+        if (nseg_all > 0) {
+                CUDA_TRY(cudaMemsetAsync(g.nchunk.p + nseg_all, 0, sizeof(long long), s));
+                count_all_kernel<<<grid_for(nseg_all, 256), 256, 0, s>>>(g.cdesc.p, (int)passes.size(), nseg_all, tol, g.fac.p,
+                                                                        P->shard, P->nshard, g.nkl.p, g.kst.p,
+                                                                        (unsigned long long *)g.nchunk.p);
+                CUDA_TRY(cudaGetLastError());
+                size_t tmp = g.cub_tmp.n;
+                CUDA_TRY(cub::DeviceScan::ExclusiveSum(g.cub_tmp.p, tmp, g.nchunk.p, g.chunk_off.p, (int)(nseg_all + 1), s));
+                launches++;
         }
+        // with class timing on, the classes run one after the other
+        const bool fan = !P->profiling;
+        if (fan && (rc = lanes.fork(s))) return rc;
+        for (const Pass &p : passes) {
+                const PairClassDev &bra = g.bra[p.X], &ket = g.ket[p.Y];
+                const int t = p.X * NPAIRCLASS + p.Y;
+                GradArgs a;
+                a.bra = bra.view();
+                a.ket = ket.view();
+                a.PP = P->PP.p; a.PK = P->PK.p; a.PE = P->PE.p;
+                a.chunk_off = g.chunk_off.p + p.d.scan0;
+                a.nkl = g.nkl.p + p.d.seg0;
+                a.kst = g.kst.p + p.d.seg0;
+                a.q0 = g.q0.p;
+                a.q1 = P->qcond.p;
+                a.dmc = g.dmc.p;
+                a.table = table_ptr();
+                a.goff = g.goff.p + g.goff_at[t];
+                a.Vj = Vj; a.Vk = Vk;
+                a.Ds = g.Ds.p; a.Dc = g.Dc.p;
+                a.stats = g.stats.p + 2 * t;
+                a.next = g.stats.p + 2 * NQ + t;
+                a.split = p.d.split;
+                a.max_chunk = p.max_chunk;
+                a.tol = tol > 0 ? tol : -1.0;
+                a.nbas = P->nbas; a.naoc = P->naoc; a.n_dm = n_dm;
+                a.with_j = with_j; a.with_k = with_k;
+                a.de = fused ? g.de.p : nullptr;
+                a.omega2 = P->omega2;
+                a.shell_atom = fused ? g.shell_atom.p : nullptr;
+                std::string err;
+                cudaStream_t cs = s;
+                if (fan && (rc = lanes.take(s, cs))) { lanes.join(s); return rc; }
+                if (P->profiling) CUDA_TRY(cudaEventRecord(g.cls_ev[2 * t], s));
+                if (g_grad_launch[p.X](ket.la, ket.lb, a, cs, P->nsm, err)) {
+                        if (fan) lanes.join(s);
+                        return fail(B200JK_ECUDA, err);
+                }
+                if (P->profiling) CUDA_TRY(cudaEventRecord(g.cls_ev[2 * t + 1], s));
+                ran[t] = 1;
+                launches++;
+        }
+        if (fan && (rc = lanes.join(s))) return rc;
         // to the output basis.  The kernels differentiate with respect to the
         // centre (d/dA = -nabla_r of int2e_ip1), so the accumulators already
         // hold the negated contraction grad.rhf.get_jk returns

@@ -26,6 +26,13 @@ struct GradCfg {
 // largest dynamic shared memory a block may request on sm_100
 constexpr size_t SMEM_MAX = 227 * 1024;
 
+// blocks of a launch: no more than its chunks can occupy
+inline int grid_of(int grid, int block, long long max_chunk)
+{
+        const long long need = (max_chunk + block / 32 - 1) / (block / 32);
+        return max_chunk > 0 && need < grid ? (int)(need > 0 ? need : 1) : grid;
+}
+
 template <int LA, int LB, int LC, int LD, bool FUSED>
 int launch_grad_impl(const GradArgs &a, cudaStream_t s, int nsm, std::string &err)
 {
@@ -50,7 +57,7 @@ int launch_grad_impl(const GradArgs &a, cudaStream_t s, int nsm, std::string &er
                         err = std::string("gradient kernel configuration: ") + cudaGetErrorString(cfg.status);
                         return 1;
                 }
-                grad_force_kernel<LA, LB, LC, LD><<<cfg.grid, cfg.block, 0, s>>>(a);
+                grad_force_kernel<LA, LB, LC, LD><<<grid_of(cfg.grid, cfg.block, a.max_chunk), cfg.block, 0, s>>>(a);
                 cudaError_t e = cudaGetLastError();
                 if (e != cudaSuccess) {
                         err = std::string("gradient kernel launch: ") + cudaGetErrorString(e);
@@ -73,7 +80,7 @@ int launch_grad_impl(const GradArgs &a, cudaStream_t s, int nsm, std::string &er
                         err = std::string("gradient kernel configuration: ") + cudaGetErrorString(cfg.status);
                         return 1;
                 }
-                grad_thread_kernel<LA, LB, LC, LD, FUSED><<<cfg.grid, cfg.block, 0, s>>>(a);
+                grad_thread_kernel<LA, LB, LC, LD, FUSED><<<grid_of(cfg.grid, cfg.block, a.max_chunk), cfg.block, 0, s>>>(a);
                 cudaError_t e = cudaGetLastError();
                 if (e != cudaSuccess) {
                         err = std::string("gradient kernel launch: ") + cudaGetErrorString(e);
@@ -106,7 +113,7 @@ int launch_grad_impl(const GradArgs &a, cudaStream_t s, int nsm, std::string &er
                 err = std::string("gradient kernel configuration: ") + cudaGetErrorString(cfg.status);
                 return 1;
         }
-        grad_jk_kernel<LA, LB, LC, LD, FUSED><<<cfg.grid, cfg.block, cfg.smem, s>>>(a, 8 * (32 / GS));
+        grad_jk_kernel<LA, LB, LC, LD, FUSED><<<grid_of(cfg.grid, cfg.block, a.max_chunk), cfg.block, cfg.smem, s>>>(a, 8 * (32 / GS));
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
                 err = std::string("gradient kernel launch: ") + cudaGetErrorString(e);

@@ -144,7 +144,23 @@ struct GradArgs {
         const int *shell_atom = nullptr;
         // omega^2 of the long-range operator erf(omega r12)/r12, 0 = Coulomb
         double omega2 = 0.0;
+        // chunk queue, cut of long contractions and chunk bound, as in JKArgs
+        unsigned long long *next = nullptr;
+        int split = 0;
+        long long max_chunk = 0;
 };
+
+// log2 of the cut of segment sgi's chunks (split_log2).  Everything a
+// quartet contributes is linear in its integrals, so lanes (register
+// families) or groups that share a quartet's primitive quartets contract
+// their partial sums on their own.  (Gradient J/K of (H2O)6/cc-pVDZ: 67.6 ms
+// with the 36 class pairs one after the other and 8 quartets of up to 192
+// primitive quartets in a row per group, 29.3 ms side by side with the cut.)
+__device__ __forceinline__ int grad_segment_split(const GradArgs &a, int sgi)
+{
+        if (a.split == 0) return 0;
+        return split_log2(a.split, bucket_of(a.bra, sgi / B2_NBUCKET), sgi % B2_NBUCKET);
+}
 
 // Weight of one Cartesian element (ab|cd) in the two-electron force of a
 // symmetric density D (Cartesian, Ds = D + D^T): grad_elec adds
@@ -190,10 +206,11 @@ __device__ __forceinline__ bool grad_side_passes(const GradArgs &a, int i, int j
 // Mode 0: components 0..2 = d/dA_{x,y,z}, 3..5 = d/dB_{x,y,z}.  Mode 1 (bra =
 // ket pair): components 0..2 = d/dA_x d/dC_x (same x), 3..5 = d/dB_x d/dD_x.
 // P and Q are taken relative to the origin O; A = 0, C relative to O.
+// Primitive quartets sub, sub + nsub, ... of the bra-major list.
 template <int LA, int LB, int LC, int LD, int MODE, int GS>
 __device__ __forceinline__ void grad_eval_pass(double *sm, const GradArgs &a, int2 pb, int2 pk, const double4 O,
                                                const double AB[3], const double C[3], const double CD[3], double fac,
-                                               int c0, int gl, unsigned gmask)
+                                               int c0, int gl, unsigned gmask, int sub, int nsub)
 {
         using GC = GClass<LA, LB, LC, LD, MODE>;
         using S = GradSmem<LA, LB, LC, LD, MODE>;
@@ -203,14 +220,15 @@ __device__ __forceinline__ void grad_eval_pass(double *sm, const GradArgs &a, in
         const double *table = a.table + rys_padded_offset(NR);
         const double A[3] = {0.0, 0.0, 0.0};
         for (int t = gl; t < NCP * NG; t += GS) G[t] = 0.0;
-        for (int ip = 0; ip < pb.y; ip++) {
+        for (int ip = 0, kp = sub; ip < pb.y; ip++, kp -= pk.y) {
+                if (kp >= pk.y) continue;
                 const double4 P = a.PP[pb.x + ip];
                 const double2 KP = a.PK[pb.x + ip];
                 const double2 EP = a.PE[pb.x + ip];
                 const double Kab = KP.x * fac;
                 const double Pv[3] = {P.x - O.x, P.y - O.y, P.z - O.z};
                 const double ta = 2.0 * EP.x, tb = 2.0 * EP.y;
-                for (int kp = 0; kp < pk.y; kp++) {
+                for (; kp < pk.y; kp += nsub) {
                         const double4 Q = a.PP[pk.x + kp];
                         const double2 KQ = a.PK[pk.x + kp];
                         const double2 EQ = a.PE[pk.x + kp];
@@ -281,7 +299,8 @@ __device__ __forceinline__ void grad_eval_pass(double *sm, const GradArgs &a, in
 template <int LA, int LB, int LC, int LD, int GS>
 __device__ __forceinline__ void grad_eval_force(double *sm, const GradArgs &a, int2 pb, int2 pk, const double4 O,
                                                 const double AB[3], const double C[3], const double CD[3],
-                                                double fac, const double *w, int gl, unsigned gmask, double fq[6])
+                                                double fac, const double *w, int gl, unsigned gmask, double fq[6],
+                                                int sub, int nsub)
 {
         using GC = GClass<LA, LB, LC, LD, 0>;
         using S = GradSmem<LA, LB, LC, LD, 0, true>;
@@ -290,14 +309,15 @@ __device__ __forceinline__ void grad_eval_force(double *sm, const GradArgs &a, i
         double *E = sm + S::E;
         const double *table = a.table + rys_padded_offset(NR);
         const double A[3] = {0.0, 0.0, 0.0};
-        for (int ip = 0; ip < pb.y; ip++) {
+        for (int ip = 0, kp = sub; ip < pb.y; ip++, kp -= pk.y) {
+                if (kp >= pk.y) continue;
                 const double4 P = a.PP[pb.x + ip];
                 const double2 KP = a.PK[pb.x + ip];
                 const double2 EP = a.PE[pb.x + ip];
                 const double Kab = KP.x * fac;
                 const double Pv[3] = {P.x - O.x, P.y - O.y, P.z - O.z};
                 const double ta = 2.0 * EP.x, tb = 2.0 * EP.y;
-                for (int kp = 0; kp < pk.y; kp++) {
+                for (; kp < pk.y; kp += nsub) {
                         const double4 Q = a.PP[pk.x + kp];
                         const double2 KQ = a.PK[pk.x + kp];
                         const double Qv[3] = {Q.x - O.x, Q.y - O.y, Q.z - O.z};
@@ -378,17 +398,21 @@ __global__ void __launch_bounds__(128) grad_jk_kernel(GradArgs a, int chunk_q)
         const int wib = threadIdx.x >> 5;
         double *sm = smem_dyn + (size_t)(wib * NGRP + grp) * S::SIZE;
         const int nseg = a.bra.n * B2_NBUCKET;
-        const long long total = a.chunk_off[nseg];
-        const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+        ChunkLoop loop(a.next, a.chunk_off[0], a.chunk_off[nseg]);
+        if (!loop.block_has_work()) return;
         const size_t n = (size_t)a.naoc, nn = n * n;
         unsigned long long nq = 0, npq = 0;
-        for (long long chunk = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; chunk < total;
-             chunk += nwarps) {
+        long long chunk;
+        while (loop.get(chunk)) {
                 const int sgi = find_bra(a.chunk_off, nseg, chunk);
                 const int ij = sgi / B2_NBUCKET;
+                // quartets of this segment's chunks; below one per group, gsub
+                // groups share the primitive quartets of each
+                const int cq = max(1, chunk_q >> grad_segment_split(a, sgi));
+                const int gsub = cq < NGRP ? NGRP / cq : 1, sub = grp % gsub, nsub = gsub;
                 const int kb = a.ket.boff[sgi % B2_NBUCKET] + a.kst[sgi];
-                const int kl0 = kb + (int)(chunk - a.chunk_off[sgi]) * chunk_q;
-                const int kl1 = kb + min((int)(chunk - a.chunk_off[sgi]) * chunk_q + chunk_q, a.nkl[sgi]);
+                const int kl0 = kb + (int)(chunk - a.chunk_off[sgi]) * cq;
+                const int kl1 = kb + min((int)(chunk - a.chunk_off[sgi]) * cq + cq, a.nkl[sgi]);
                 const int4 sb = a.bra.sh[ij];
                 const int2 pb = a.bra.pr[ij];
                 const double4 Ab = a.bra.A[ij];
@@ -397,7 +421,7 @@ __global__ void __launch_bounds__(128) grad_jk_kernel(GradArgs a, int chunk_q)
                 const int ia = sb.x, ib = sb.y;
                 const bool bra_one_segment = Ab.w != 0.0;
                 double fs[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-                for (int kl = kl0 + grp; kl < kl1; kl += NGRP) {
+                for (int kl = kl0 + grp / gsub; kl < kl1; kl += NGRP / gsub) {
                         const int4 sk = a.ket.sh[kl];
                         const int kk = max(sk.z, sk.w), ll = min(sk.z, sk.w);
                         const bool sideA = grad_side_passes(a, sb.z, sb.w, kk, ll);
@@ -409,7 +433,7 @@ __global__ void __launch_bounds__(128) grad_jk_kernel(GradArgs a, int chunk_q)
                         const double fac = Ak.w != 0.0 ? 0.5 : 1.0;
                         const double C[3] = {Ak.x - Ab.x, Ak.y - Ab.y, Ak.z - Ab.z};
                         const double CD[3] = {CDk.x, CDk.y, CDk.z};
-                        if (gl == 0) {
+                        if (gl == 0 && sub == 0) {
                                 nq += (unsigned long long)sideA + (unsigned long long)sideB;
                                 npq += (unsigned long long)pb.y * pk.y;
                         }
@@ -437,7 +461,7 @@ __global__ void __launch_bounds__(128) grad_jk_kernel(GradArgs a, int chunk_q)
                                 }
                                 __syncwarp(gmask);
                                 double fq[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-                                grad_eval_force<LA, LB, LC, LD, GS>(sm, a, pb, pk, Ab, AB, C, CD, fac, w, gl, gmask, fq);
+                                grad_eval_force<LA, LB, LC, LD, GS>(sm, a, pb, pk, Ab, AB, C, CD, fac, w, gl, gmask, fq, sub, nsub);
 #pragma unroll
                                 for (int q = 0; q < 6; q++)
                                         if (q < 3 ? sideA : sideB) fs[q] += fq[q];
@@ -449,7 +473,7 @@ __global__ void __launch_bounds__(128) grad_jk_kernel(GradArgs a, int chunk_q)
                                 // skip a pass whose components all belong to a failing side
                                 const bool needA = sideA && c0 < 3, needB = sideB && c0 + GC::NCP > 3;
                                 if (!needA && !needB) continue;
-                                grad_eval_pass<LA, LB, LC, LD, 0, GS>(sm, a, pb, pk, Ab, AB, C, CD, fac, c0, gl, gmask);
+                                grad_eval_pass<LA, LB, LC, LD, 0, GS>(sm, a, pb, pk, Ab, AB, C, CD, fac, c0, gl, gmask, sub, nsub);
                                 const double *G = sm + S::G;
                                 for (int s = 0; s < a.n_dm; s++) {
                                         const double *Ds = a.Ds + s * nn;
@@ -591,16 +615,18 @@ __global__ void __launch_bounds__(128) grad_thread_kernel(GradArgs a)
         constexpr int NG = K::NG, NR = GC::NR, SE = GC::SE;
         const int lane = threadIdx.x & 31;
         const int nseg = a.bra.n * B2_NBUCKET;
-        const long long total = a.chunk_off[nseg];
-        const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+        ChunkLoop loop(a.next, a.chunk_off[0], a.chunk_off[nseg]);
+        if (!loop.block_has_work()) return;
         const size_t n = (size_t)a.naoc, nn = n * n;
         const double *table = a.table + rys_padded_offset(NR);
         unsigned long long nq = 0, npq = 0;
-        for (long long chunk = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; chunk < total;
-             chunk += nwarps) {
+        long long chunk;
+        while (loop.get(chunk)) {
                 const int sgi = find_bra(a.chunk_off, nseg, chunk);
                 const int ij = sgi / B2_NBUCKET;
-                const int pos = (int)(chunk - a.chunk_off[sgi]) * 32 + lane;
+                // 2^lg lanes share a quartet's primitive quartets
+                const int lg = grad_segment_split(a, sgi), nsub = 1 << lg, sub = lane & (nsub - 1);
+                const int pos = (int)(chunk - a.chunk_off[sgi]) * (32 >> lg) + (lane >> lg);
                 const int kl = a.ket.boff[sgi % B2_NBUCKET] + a.kst[sgi] + pos;
                 const int4 sb = a.bra.sh[ij];
                 const int2 pb = a.bra.pr[ij];
@@ -627,16 +653,19 @@ __global__ void __launch_bounds__(128) grad_thread_kernel(GradArgs a)
                         const double A0[3] = {0.0, 0.0, 0.0};
                         const double C[3] = {Ak.x - Ab.x, Ak.y - Ab.y, Ak.z - Ab.z};
                         const double CD[3] = {CDk.x, CDk.y, CDk.z};
-                        nq += (unsigned long long)sideA + (unsigned long long)sideB;
-                        npq += (unsigned long long)pb.y * pk.y;
-                        for (int ip = 0; ip < pb.y; ip++) {
+                        if (sub == 0) {
+                                nq += (unsigned long long)sideA + (unsigned long long)sideB;
+                                npq += (unsigned long long)pb.y * pk.y;
+                        }
+                        for (int ip = 0, kp = sub; ip < pb.y; ip++, kp -= pk.y) {
+                                if (kp >= pk.y) continue;
                                 const double4 P = a.PP[pb.x + ip];
                                 const double2 KP = a.PK[pb.x + ip];
                                 const double2 EP = a.PE[pb.x + ip];
                                 const double Kab = KP.x * fac;
                                 const double Pv[3] = {P.x - Ab.x, P.y - Ab.y, P.z - Ab.z};
                                 const double ta = 2.0 * EP.x, tb = 2.0 * EP.y;
-                                for (int kp = 0; kp < pk.y; kp++) {
+                                for (; kp < pk.y; kp += nsub) {
                                         const double4 Q = a.PP[pk.x + kp];
                                         const double2 KQ = a.PK[pk.x + kp];
                                         const double Qv[3] = {Q.x - Ab.x, Q.y - Ab.y, Q.z - Ab.z};
@@ -692,6 +721,12 @@ __global__ void __launch_bounds__(128) grad_thread_kernel(GradArgs a)
                         grad_force_flush(a, sb, fs, lane);
                         continue;
                 }
+                // whole blocks into the first lane of the quartet, which contracts
+                // them (a share each would multiply the atomics)
+                for (int o = 1; o < nsub; o <<= 1)
+#pragma unroll
+                        for (int t = 0; t < 6 * NG; t++) G[t] += __shfl_xor_sync(0xffffffffu, G[t], o);
+                if (sub != 0) sideA = sideB = false;
                 for (int s = 0; s < a.n_dm; s++) {
                         const double *Ds = a.Ds + s * nn;
                         const double *X = a.Dc + s * nn;
@@ -838,7 +873,7 @@ __global__ void __launch_bounds__(32) grad_q0_kernel(GradQArgs q)
         double mA = 0.0, mB = 0.0;
         for (int pass = 0; pass < GC::NPASS; pass++) {
                 const int c0 = pass * GC::NCP;
-                grad_eval_pass<LA, LB, LA, LB, 1, 32>(sm, a, pr, pr, Av, AB, C0, AB, 1.0, c0, lane, 0xffffffffu);
+                grad_eval_pass<LA, LB, LA, LB, 1, 32>(sm, a, pr, pr, Av, AB, C0, AB, 1.0, c0, lane, 0xffffffffu, 0, 1);
                 const double *G = sm + S::G;
                 for (int cc = 0; cc < GC::NCP; cc++) {
                         const int side = (c0 + cc) / 3;
@@ -1015,16 +1050,18 @@ __global__ void __launch_bounds__(128) grad_force_kernel(GradArgs a)
         constexpr int NG = K::NG, NR = GC::NR, SE = GC::SE;
         const int lane = threadIdx.x & 31;
         const int nseg = a.bra.n * B2_NBUCKET;
-        const long long total = a.chunk_off[nseg];
-        const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+        ChunkLoop loop(a.next, a.chunk_off[0], a.chunk_off[nseg]);
+        if (!loop.block_has_work()) return;
         const size_t n = (size_t)a.naoc;
         const double *table = a.table + rys_padded_offset(NR);
         unsigned long long nq = 0, npq = 0;
-        for (long long chunk = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; chunk < total;
-             chunk += nwarps) {
+        long long chunk;
+        while (loop.get(chunk)) {
                 const int sgi = find_bra(a.chunk_off, nseg, chunk);
                 const int ij = sgi / B2_NBUCKET;
-                const int pos = (int)(chunk - a.chunk_off[sgi]) * 32 + lane;
+                // 2^lg lanes share a quartet's primitive quartets
+                const int lg = grad_segment_split(a, sgi), nsub = 1 << lg, sub = lane & (nsub - 1);
+                const int pos = (int)(chunk - a.chunk_off[sgi]) * (32 >> lg) + (lane >> lg);
                 const int kl = a.ket.boff[sgi % B2_NBUCKET] + a.kst[sgi] + pos;
                 const int4 sb = a.bra.sh[ij];
                 const int2 pb = a.bra.pr[ij];
@@ -1061,16 +1098,19 @@ __global__ void __launch_bounds__(128) grad_force_kernel(GradArgs a)
                         const double A0[3] = {0.0, 0.0, 0.0};
                         const double C[3] = {Ak.x - Ab.x, Ak.y - Ab.y, Ak.z - Ab.z};
                         const double CD[3] = {CDk.x, CDk.y, CDk.z};
-                        nq += (unsigned long long)sideA + (unsigned long long)sideB;
-                        npq += (unsigned long long)pb.y * pk.y;
-                        for (int ip = 0; ip < pb.y; ip++) {
+                        if (sub == 0) {
+                                nq += (unsigned long long)sideA + (unsigned long long)sideB;
+                                npq += (unsigned long long)pb.y * pk.y;
+                        }
+                        for (int ip = 0, kp = sub; ip < pb.y; ip++, kp -= pk.y) {
+                                if (kp >= pk.y) continue;
                                 const double4 P = a.PP[pb.x + ip];
                                 const double2 KP = a.PK[pb.x + ip];
                                 const double2 EP = a.PE[pb.x + ip];
                                 const double Kab = KP.x * fac;
                                 const double Pv[3] = {P.x - Ab.x, P.y - Ab.y, P.z - Ab.z};
                                 const double ta = 2.0 * EP.x, tb = 2.0 * EP.y;
-                                for (int kp = 0; kp < pk.y; kp++) {
+                                for (; kp < pk.y; kp += nsub) {
                                         const double4 Q = a.PP[pk.x + kp];
                                         const double2 KQ = a.PK[pk.x + kp];
                                         const double Qv[3] = {Q.x - Ab.x, Q.y - Ab.y, Q.z - Ab.z};

@@ -107,3 +107,25 @@ def test_threads(b2):
     for t in ts:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize('nprims,l_of,nctr', [
+    ((1, 2, 4, 9), (0, 0, 0, 0), 1),
+    ((1, 3, 5, 9), (1, 0, 1, 0), 1),
+    ((2, 4, 1, 9), (2, 1, 0, 0), 1),
+    ((4, 17, 1), (1, 0, 2), 2),
+])
+def test_long_contractions_gradient(b2, nprims, l_of, nctr):
+    """The gradient J/K and the fused force of long contractions, whose
+    primitive quartets are shared by lanes or lane groups."""
+    atm, bas, env = contracted_molecule(nprims, l_of, nctr=nctr)
+    plan = b2.Plan(atm, bas, env, direct_scf_tol=1e-13)
+    d = densities(plan.nao, 1)[0]
+    d = d + d.T
+    rj, rk = oracle.grad_jk(d, atm, bas, env)[:2]
+    vj, vk = plan.grad_jk(d)
+    assert abs(vj - rj).max() < TOL
+    assert abs(vk - rk).max() < TOL
+    from pyscf_b200 import grad
+    want = grad.grad_2e(rj, rk, d, grad.aoslice_by_atom(atm, bas))
+    assert abs(plan.grad_contract(d) - want).max() < plan.nao * TOL
