@@ -457,11 +457,14 @@ struct b200jk_plan {
         DevArr<int> fill_nkl, fill_kst;
         DevArr<long long> fill_nchunk, fill_chunk_off;
         DevArr<unsigned char> fill_cub;
+        DevArr<CountDesc> fill_cdesc;
+        DevArr<unsigned long long> fill_next;
         void release_fill()
         {
                 for (auto &c : fill_pc) c.release();
                 fill_one.release(); fill_nkl.release(); fill_kst.release();
                 fill_nchunk.release(); fill_chunk_off.release(); fill_cub.release();
+                fill_cdesc.release(); fill_next.release();
                 fill_ready = false;
         }
         std::vector<double> h_qcond;
@@ -2961,7 +2964,7 @@ static int ensure_fill(b200jk_plan *P)
         const int nbas = P->nbas;
         double qmax = 0;
         for (double v : P->h_qcond) qmax = std::max(qmax, v);
-        size_t maxn = 1;
+        size_t nseg = 1;   // segments of all classes: X is the bra of the classes Y <= X
         int rc;
         for (int X = 0; X < NPAIRCLASS; X++) {
                 std::vector<PairLite> hv;
@@ -2984,10 +2987,10 @@ static int ensure_fill(b200jk_plan *P)
                 for (size_t t = 0; t < idx.size(); t++) { h2[t] = hv[idx[t]]; q2[t] = q[idx[t]]; }
                 P->fill_pc[X].release();
                 if ((rc = upload_pairs(P, P->fill_pc[X], X, h2, q2))) return rc;
-                maxn = std::max(maxn, h2.size());
+                nseg += h2.size() * B2_NBUCKET * (X + 1);
         }
-        const size_t nseg = maxn * B2_NBUCKET;
-        if ((rc = dev_upload(P->fill_one, std::vector<double>(1, 1.0))) || (rc = dev_alloc(P->fill_nkl, nseg)) ||
+        if (nseg + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one fill");
+        if ((rc = dev_alloc(P->fill_cdesc, 64)) || (rc = dev_alloc(P->fill_next, 64)) || (rc = dev_upload(P->fill_one, std::vector<double>(1, 1.0))) || (rc = dev_alloc(P->fill_nkl, nseg)) ||
             (rc = dev_alloc(P->fill_kst, nseg)) || (rc = dev_alloc(P->fill_nchunk, nseg + 1)) ||
             (rc = dev_alloc(P->fill_chunk_off, nseg + 1)))
                 return rc;
@@ -3018,38 +3021,83 @@ int b200jk_int2e_s8(b200jk_plan *P, double *eri, long long len, int dev_ptr, voi
                 if ((rc = dev_alloc(tmp, (size_t)need))) return rc;
                 out = tmp.p;
         }
-        auto run = [&]() -> int {
-                CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * need, s));
+        // the classes with work, their segments and chunk bounds
+        struct Pass {
+                size_t t;
+                CountDesc d;
+                long long max_chunk;
+        };
+        std::vector<Pass> passes;
+        long long nseg = 0;
+        {
                 auto qcs = quartet_classes();
                 for (size_t t = 0; t < qcs.size(); t++) {
                         const PairClassDev &bra = P->fill_pc[qcs[t].X], &ket = P->fill_pc[qcs[t].Y];
                         if (bra.n == 0 || ket.n == 0) continue;
-                        const int la = bra.la, lb = bra.lb, lc = ket.la, ld = ket.lb;
-                        const int same = qcs[t].X == qcs[t].Y;
-                        const int nseg = bra.n * B2_NBUCKET;
-                        const int chunk = fill_chunk(la, lb, lc, ld);
-                        count_kernel<<<grid_for(nseg, 256), 256, 0, s>>>(
-                                bra.view(), ket.view(), same, B2_FILL_CUTOFF, P->fill_one.p, chunk, 0.0, 0, 0, 1,
-                                P->fill_nkl.p, P->fill_kst.p, P->fill_nchunk.p);
-                        CUDA_TRY(cudaGetLastError());
+                        Pass p;
+                        p.t = t;
+                        CountDesc &d = p.d;
+                        memset(&d, 0, sizeof(d));
+                        d.bra = bra.view();
+                        d.ket = ket.view();
+                        d.same = qcs[t].X == qcs[t].Y;
+                        d.chunk = fill_chunk(bra.la, bra.lb, ket.la, ket.lb);
+                        d.split = split_level(bra, ket, d.same, false, P->nsm);
+                        d.most = d.chunk == 32 ? 5 : (d.chunk == 16 ? 4 : 3);
+                        d.seg0 = d.scan0 = nseg;
+                        p.max_chunk = 0;
+                        for (int b = 0; b < B2_NBUCKET; b++) {
+                                const int len = d.chunk >> std::min(d.most, split_log2(d.split, B2_NBUCKET - 1, b));
+                                p.max_chunk += (long long)((ket.boff[b + 1] - ket.boff[b] + len - 1) / len) * bra.n;
+                        }
+                        nseg += (long long)bra.n * B2_NBUCKET;
+                        passes.push_back(p);
+                }
+        }
+        auto run = [&]() -> int {
+                CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * need, s));
+                auto qcs = quartet_classes();
+                FanLease lease(P->device);
+                int rc;
+                if ((rc = lease.pool.take(lease.fan))) return rc;
+                StreamFan &lanes = *lease.fan;
+                if (!passes.empty()) {
+                        std::vector<CountDesc> h;
+                        for (const Pass &p : passes) h.push_back(p.d);
+                        // pageable memory: staged before the call returns
+                        CUDA_TRY(cudaMemcpyAsync(P->fill_cdesc.p, h.data(), sizeof(CountDesc) * h.size(),
+                                                 cudaMemcpyHostToDevice, s));
                         CUDA_TRY(cudaMemsetAsync(P->fill_nchunk.p + nseg, 0, sizeof(long long), s));
+                        CUDA_TRY(cudaMemsetAsync(P->fill_next.p, 0, sizeof(unsigned long long) * 64, s));
+                        count_all_kernel<<<grid_for(nseg, 256), 256, 0, s>>>(
+                                P->fill_cdesc.p, (int)passes.size(), nseg, B2_FILL_CUTOFF, P->fill_one.p, 0, 1,
+                                P->fill_nkl.p, P->fill_kst.p, (unsigned long long *)P->fill_nchunk.p);
+                        CUDA_TRY(cudaGetLastError());
                         size_t tb = P->fill_cub.n;
                         CUDA_TRY(cub::DeviceScan::ExclusiveSum(P->fill_cub.p, tb, P->fill_nchunk.p, P->fill_chunk_off.p,
-                                                               nseg + 1, s));
+                                                               (int)(nseg + 1), s));
+                }
+                if ((rc = lanes.fork(s))) return rc;
+                for (const Pass &p : passes) {
+                        const size_t t = p.t;
+                        const PairClassDev &bra = P->fill_pc[qcs[t].X], &ket = P->fill_pc[qcs[t].Y];
                         FillArgs f = FillArgs();
                         JKArgs &a = f.jk;
                         a.tiled = 0;
                         a.bra = bra.view();
                         a.ket = ket.view();
                         a.PP = P->PP.p; a.PK = P->PK.p;
-                        a.chunk_off = P->fill_chunk_off.p;
-                        a.nkl = P->fill_nkl.p;
-                        a.kst = P->fill_kst.p;
+                        a.chunk_off = P->fill_chunk_off.p + p.d.scan0;
+                        a.nkl = P->fill_nkl.p + p.d.seg0;
+                        a.kst = P->fill_kst.p + p.d.seg0;
+                        a.next = P->fill_next.p + t;
+                        a.split = p.d.split;
+                        a.max_chunk = p.max_chunk;
                         a.table = table_ptr();
                         a.table_f = table_f_ptr();
                         a.goff = P->goff_all.p + P->goff_at[t];
                         a.tol = B2_FILL_CUTOFF;
-                        a.nbas = P->nbas; a.naoc = P->naoc; a.same = same;
+                        a.nbas = P->nbas; a.naoc = P->naoc; a.same = p.d.same;
                         a.omega2 = P->omega2;
                         f.cart_seg = P->cart_seg.p;
                         f.seg_info = P->seg_info.p;
@@ -3057,8 +3105,14 @@ int b200jk_int2e_s8(b200jk_plan *P, double *eri, long long len, int dev_ptr, voi
                         f.cart = P->cart;
                         f.eri = out;
                         std::string err;
-                        if (g_fill_launch[qcs[t].X](lc, ld, f, s, P->nsm, err)) return fail(B200JK_ECUDA, err);
+                        cudaStream_t cs = s;
+                        if ((rc = lanes.take(s, cs))) { lanes.join(s); return rc; }
+                        if (g_fill_launch[qcs[t].X](ket.la, ket.lb, f, cs, P->nsm, err)) {
+                                lanes.join(s);
+                                return fail(B200JK_ECUDA, err);
+                        }
                 }
+                if ((rc = lanes.join(s))) return rc;
                 if (!dev_ptr) CUDA_TRY(cudaMemcpyAsync(eri, out, sizeof(double) * need, cudaMemcpyDeviceToHost, s));
                 CUDA_TRY(cudaStreamSynchronize(s));
                 return B200JK_OK;

@@ -24,6 +24,13 @@ struct FillCfg {
 
 constexpr size_t SMEM_MAX = 227 * 1024;
 
+// blocks of a launch: no more than its chunks can occupy
+inline int grid_of(int grid, int block, long long max_chunk)
+{
+        const long long need = (max_chunk + block / 32 - 1) / (block / 32);
+        return max_chunk > 0 && need < grid ? (int)(need > 0 ? need : 1) : grid;
+}
+
 template <int LA, int LB, int LC, int LD>
 int launch_fill_one(const FillArgs &f, cudaStream_t s, int nsm, std::string &err)
 {
@@ -55,7 +62,7 @@ int launch_fill_one(const FillArgs &f, cudaStream_t s, int nsm, std::string &err
                 err = std::string("integral fill kernel configuration: ") + cudaGetErrorString(cfg.status);
                 return 1;
         }
-        fill_kernel<LA, LB, LC, LD><<<cfg.grid, cfg.block, cfg.smem, s>>>(f, 8 * (32 / GS));
+        fill_kernel<LA, LB, LC, LD><<<grid_of(cfg.grid, cfg.block, f.jk.max_chunk), cfg.block, cfg.smem, s>>>(f, 8 * (32 / GS));
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
                 err = std::string("integral fill kernel launch: ") + cudaGetErrorString(e);

@@ -1073,22 +1073,24 @@ __device__ __forceinline__ void group_load_goff(const int *goff, int gl, int *go
 template <int LA, int LB, int LC, int LD, int GS, typename R>
 __device__ __forceinline__ void group_eval_block(double *sm, const JKArgs &a, int2 pb, int2 pk, const double4 O,
                                                  const R A[3], const R AB[3], const R C[3], const R CD[3],
-                                                 R fac, int gl, unsigned gmask, const int *goff_r)
+                                                 R fac, int gl, unsigned gmask, const int *goff_r, int sub = 0,
+                                                 int nsub = 1)
 {
         using K = Class4<LA, LB, LC, LD>;
         using S = WarpSmem<LA, LB, LC, LD, R>;
         R *G = reinterpret_cast<R *>(sm) + S::G;
         R *H = reinterpret_cast<R *>(sm) + S::H;
         const R *table = table_of<R>(a) + RysLayout<R>::offset(K::NR);
-        // the first primitive quartet stores the block, later ones add to it
-        // (every pair has at least one primitive pair)
+        // the first primitive quartet stores the block, later ones add to it;
+        // primitive quartets sub, sub + nsub, ... of the bra-major list
         bool first = true;
-        for (int ip = 0; ip < pb.y; ip++) {
+        for (int ip = 0, kp = sub; ip < pb.y; ip++, kp -= pk.y) {
+                if (kp >= pk.y) continue;
                 const double4 P = a.PP[pb.x + ip];
                 const double2 KP = a.PK[pb.x + ip];
                 const R Kab = (R)KP.x * fac;
                 const R Pv[3] = {(R)(P.x - O.x), (R)(P.y - O.y), (R)(P.z - O.z)};
-                for (int kp = 0; kp < pk.y; kp++) {
+                for (; kp < pk.y; kp += nsub) {
                         const double4 Q = a.PP[pk.x + kp];
                         const double2 KQ = a.PK[pk.x + kp];
                         const R Qv[3] = {(R)(Q.x - O.x), (R)(Q.y - O.y), (R)(Q.z - O.z)};
@@ -1148,6 +1150,9 @@ __device__ __forceinline__ void group_eval_block(double *sm, const JKArgs &a, in
                         first = false;
                 }
         }
+        // fewer primitive quartets than nsub: an empty share
+        if (first)
+                for (int t = gl; t < K::NG; t += GS) G[t] = (R)0;
         __syncwarp(gmask);
 }
 

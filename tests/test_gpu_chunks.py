@@ -129,3 +129,28 @@ def test_long_contractions_gradient(b2, nprims, l_of, nctr):
     from pyscf_b200 import grad
     want = grad.grad_2e(rj, rk, d, grad.aoslice_by_atom(atm, bas))
     assert abs(plan.grad_contract(d) - want).max() < plan.nao * TOL
+
+
+@pytest.mark.parametrize('nprims,l_of,nctr', [
+    ((1, 2, 4, 9), (0, 0, 0, 0), 1),
+    ((1, 3, 5, 9), (1, 0, 1, 0), 1),
+    ((4, 17, 1), (1, 0, 2), 2),
+])
+def test_long_contractions_fill(b2, nprims, l_of, nctr):
+    """The s8 tensor of long contractions (groups of a warp share a quartet's
+    primitive quartets): J and K contracted from it on the host against the
+    oracle's direct J and K."""
+    atm, bas, env = contracted_molecule(nprims, l_of, nctr=nctr)
+    plan = b2.Plan(atm, bas, env, direct_scf_tol=0.0)
+    n = plan.nao
+    eri = plan.int2e_s8(device=False)
+    a = numpy.arange(n)
+    hi, lo = numpy.maximum(a[:, None], a), numpy.minimum(a[:, None], a)
+    tri = (hi * (hi + 1) // 2 + lo).ravel()
+    p, q = numpy.maximum(tri[:, None], tri), numpy.minimum(tri[:, None], tri)
+    full = eri[p * (p + 1) // 2 + q].reshape(n, n, n, n)
+    d = densities(n, 1)[0]
+    d = d + d.T
+    rj, rk, _ = oracle.get_jk(d, atm, bas, env, hermi=1, screen=False)
+    assert abs(numpy.einsum('ijkl,ji->kl', full, d) - rj).max() < TOL
+    assert abs(numpy.einsum('ijkl,jk->il', full, d) - rk).max() < TOL
