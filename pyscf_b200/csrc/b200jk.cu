@@ -3127,7 +3127,7 @@ struct IncoreWS {
         std::mutex mu;
         DevArr<double> A1, A2, Jp, t, Dt, eri, dms, vj, vk;
         DevArr<int4> items;
-        std::vector<int4> h_items;     // the fast kernel's four item lists, then the general ones
+        std::vector<int4> h_items;     // the kernel's four item lists
         int nf[4] = {0, 0, 0, 0};
         int items_nao = -1, items_s8 = -1;
 };
@@ -3186,14 +3186,13 @@ int b200jk_incore_jk(const double *eri, long long eri_len, int nao, const double
         }
         const int B = incore_block(nao);
         if (W.items_nao != nao || W.items_s8 != s8) {
-                std::vector<int4> fast[4], general;
-                incore_items(nao, s8, B, 2048, fast, general);
+                std::vector<int4> items[4];
+                incore_items(nao, s8, B, items);
                 W.h_items.clear();
                 for (int v = 0; v < 4; v++) {
-                        W.nf[v] = (int)fast[v].size();
-                        W.h_items.insert(W.h_items.end(), fast[v].begin(), fast[v].end());
+                        W.nf[v] = (int)items[v].size();
+                        W.h_items.insert(W.h_items.end(), items[v].begin(), items[v].end());
                 }
-                W.h_items.insert(W.h_items.end(), general.begin(), general.end());
                 if ((rc = dev_upload(W.items, W.h_items))) return rc;
                 W.items_nao = nao;
                 W.items_s8 = s8;
@@ -3213,7 +3212,6 @@ int b200jk_incore_jk(const double *eri, long long eri_len, int nao, const double
                         a.nf[v] = W.nf[v];
                         off += W.nf[v];
                 }
-                a.items = W.items.p + off; a.nitems = (int)W.h_items.size() - off;
                 // one read of the tensor gives J and the K images (a J-only
                 // call drops the images: the pass is bound by the read)
                 if (launch_incore_pass(a, s, err)) return fail(B200JK_ECUDA, err);

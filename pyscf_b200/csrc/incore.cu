@@ -18,22 +18,19 @@
 // images are then, for s8, A(D^T)^T (so K = A(D) + A(D)^T for symmetric D),
 // and for s4 the swapped entries are stored themselves (K = A(D)).
 //
-// Work decomposition: a thread block owns the packed rows ij of one pair of
-// AO blocks (i in block I, j in block J, I >= J, B AOs a block) and a window
+// Work decomposition.  A thread block owns the packed rows ij of one pair of
+// AO blocks (i in block I, j in block J, I >= J, 8 AOs a block) and a window
 // of packed columns kl.  Each thread takes one column kl of a 256-column
 // chunk and walks the block's rows, so every row's chunk is one coalesced
-// 2 KB read and each entry is read from HBM once.  Two kernels share the
-// windows: incore_fast_kernel takes every full block, in one launch of four
-// variants -- the interior of the packed matrix (blocks I > J, columns
-// before the block's rows: no per-entry test or weight), the windows of such
-// blocks that reach their rows (EDGE: q <= p tested per entry), and the same
-// two for the diagonal blocks I == J (DIAG: rows j > i skipped, the K images
-// of j == i halved) -- and incore_pass_kernel the blocks of the partial last
-// block row with every test.  The fast kernel sends the K images and J row
-// sums of a lane's register sums straight to the accumulators with float64
-// reductions (after a warp reduction where all lanes share k); the general
-// one stages them in shared-memory slabs.  J row sums are reduce-scattered
-// across the warp.  The bound is HBM: 8 bytes per stored entry.
+// 2 KB read and each entry is read from HBM once.  One launch of four
+// variants: the interior of the packed matrix (blocks I > J, columns before
+// the block's rows: no per-entry test or weight), the windows of such blocks
+// that reach their rows (EDGE: q <= p tested per entry), and the same two for
+// the diagonal blocks I == J (DIAG: rows j > i skipped, the K images of
+// j == i halved).  The K images and J row sums of a lane's register sums go
+// straight to the (L2-resident) accumulators with float64 reductions, after a
+// warp reduction where all lanes share k.  The floor is HBM: 8 bytes per
+// stored entry.
 #include <vector>
 #include "incore_launch.h"
 
@@ -79,124 +76,22 @@ __device__ __forceinline__ double reduce_scatter(double (&v)[N], int lane, int &
         return s;
 }
 
-__device__ __forceinline__ double warp_sum_d(double v)
-{
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        return v;
-}
+// stages of the kernel's ring of entries
+constexpr int STAGES = 4;
 
-template <int B, bool S8>
-__global__ void __launch_bounds__(NT, 2) incore_pass_kernel(IncoreArgs a)
+// 8 bytes global -> shared without a register; zeros where !ok (nothing is read)
+__device__ __forceinline__ void cp_async8z(double *smem, const double *g, bool ok)
 {
-        extern __shared__ __align__(16) double sm[];
-        const int nao = a.nao;
-        double *DI = sm, *DJ = DI + B * nao, *SI = DJ + B * nao, *SJ = SI + B * nao, *RJ = SJ + B * nao;
-        const int4 it = a.items[blockIdx.x];
-        const int i0 = it.x * B, j0 = it.y * B;
-        const int ni = min(B, nao - i0), nj = min(B, nao - j0);
-        const int tid = threadIdx.x, lane = tid & 31;
-        for (int e = tid; e < B * nao; e += NT) {
-                const int r = e / nao, x = e % nao;
-                DI[e] = r < ni ? a.D[(size_t)(i0 + r) * nao + x] : 0.0;
-                DJ[e] = r < nj ? a.D[(size_t)(j0 + r) * nao + x] : 0.0;
-                SI[e] = 0.0;
-                SJ[e] = 0.0;
-        }
-        for (int e = tid; e < B * B; e += NT) RJ[e] = 0.0;
-        __syncthreads();
-        const long long c0 = it.z, c1 = it.w;
-        for (long long qb = c0; qb < c1; qb += NT) {
-                const long long q = qb + tid;
-                const bool active = q < c1;
-                int k = 0, l = 0;
-                if (active) pair_of(q, k, l);
-                const double tq = active ? a.t[q] : 0.0;
-                const double wkl = k == l ? 0.5 : 1.0;
-                // whether all lanes of the warp share k (images into column k)
-                const int k0 = __shfl_sync(0xffffffffu, k, 0);
-                const bool kuni = __all_sync(0xffffffffu, !active || k == k0);
-                double acc2[B], acc4[B];
-#pragma unroll
-                for (int jj = 0; jj < B; jj++) {
-                        acc2[jj] = 0.0;
-                        acc4[jj] = 0.0;
-                }
-                double colj = 0.0;
-                for (int ii = 0; ii < ni; ii++) {
-                        const int i = i0 + ii;
-                        const long long pbase = (long long)i * (i + 1) / 2;
-                        // s8: rows before the chunk hold none of its columns
-                        if (S8 && pbase + min(i, j0 + nj - 1) < qb) continue;
-                        const double dik = DI[ii * nao + k], dil = DI[ii * nao + l];
-                        double v[B];
-#pragma unroll
-                        for (int jj = 0; jj < B; jj++) {
-                                const int j = j0 + jj;
-                                const long long p = pbase + j;
-                                const bool ok = active && jj < nj && j <= i && (!S8 || q <= p);
-                                v[jj] = ok ? __ldg(a.eri + (S8 ? p * (p + 1) / 2 + q : p * a.npair + q)) : 0.0;
-                        }
-                        double acc1 = 0.0, acc3 = 0.0, rp[B];
-#pragma unroll
-                        for (int jj = 0; jj < B; jj++) rp[jj] = 0.0;
-#pragma unroll
-                        for (int jj = 0; jj < B; jj++) {
-                                const int j = j0 + jj;
-                                const long long p = pbase + j;
-                                const double wpq = (S8 && p == q) ? 0.5 : 1.0;
-                                const double vj = v[jj] * wpq;
-                                const double vw = vj * (i == j ? 0.5 : 1.0) * wkl;
-                                acc1 += vw * DJ[jj * nao + k];
-                                acc3 += vw * DJ[jj * nao + l];
-                                acc2[jj] += vw * dik;
-                                acc4[jj] += vw * dil;
-                                if (a.Jp) {
-                                        const bool rowok = jj < nj && j <= i;
-                                        colj += vj * (rowok ? __ldg(a.t + p) : 0.0);
-                                        rp[jj] = vj * tq;
-                                }
-                        }
-                        if (active) atomicAdd(SI + ii * nao + l, acc1);
-                        if (kuni) {
-                                acc3 = warp_sum_d(acc3);
-                                if (lane == 0) atomicAdd(SI + ii * nao + k0, acc3);
-                        } else if (active) {
-                                atomicAdd(SI + ii * nao + k, acc3);
-                        }
-                        if (S8 && a.Jp) {
-                                int row;
-                                const double s = reduce_scatter<B>(rp, lane, row);
-                                if ((lane & (32 / B - 1)) == 0 && s != 0.0) atomicAdd(RJ + ii * B + row, s);
-                        }
-                }
-#pragma unroll
-                for (int jj = 0; jj < B; jj++)
-                        if (active && acc2[jj] != 0.0) atomicAdd(SJ + jj * nao + l, acc2[jj]);
-                if (kuni) {
-                        int row;
-                        const double s = reduce_scatter<B>(acc4, lane, row);
-                        if ((lane & (32 / B - 1)) == 0 && s != 0.0) atomicAdd(SJ + row * nao + k0, s);
-                } else if (active) {
-#pragma unroll
-                        for (int jj = 0; jj < B; jj++)
-                                if (acc4[jj] != 0.0) atomicAdd(SJ + jj * nao + k, acc4[jj]);
-                }
-                if (a.Jp && active && colj != 0.0) atomicAdd(a.Jp + q, colj);
-        }
-        __syncthreads();
-        for (int e = tid; e < B * nao; e += NT) {
-                const int r = e / nao, x = e % nao;
-                if (r < ni && SI[e] != 0.0) atomicAdd(a.A + (size_t)(i0 + r) * nao + x, SI[e]);
-                if (r < nj && SJ[e] != 0.0) atomicAdd(a.A + (size_t)(j0 + r) * nao + x, SJ[e]);
-        }
-        if (S8 && a.Jp)
-                for (int e = tid; e < B * B; e += NT) {
-                        const int ii = e / B, jj = e % B;
-                        const int i = i0 + ii, j = j0 + jj;
-                        if (ii < ni && jj < nj && j <= i && RJ[e] != 0.0)
-                                atomicAdd(a.Jp + (long long)i * (i + 1) / 2 + j, RJ[e]);
-                }
+        const unsigned dst = (unsigned)__cvta_generic_to_shared(smem);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(g), "r"(ok ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit()
+{
+        asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N> __device__ __forceinline__ void cp_async_wait_group()
+{
+        asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // The interior of the packed matrix: full AO blocks I > J (so i > j for
@@ -211,22 +106,69 @@ __global__ void __launch_bounds__(NT, 2) incore_pass_kernel(IncoreArgs a)
 // stored only for q <= p and counts half on the packed diagonal q == p.
 // DIAG: a diagonal block I == J, whose rows are the pairs j <= i (the others
 // are skipped, uniformly over the block) and count half for j == i.
+// A partial last block row only has fewer rows i.
+//
+// What bounds it is the shared-memory and shuffle pipe, so a lane keeps the
+// density rows of its column's k and l in registers for all rows of the block
+// (2 x 8 doubles), reads the row weights T as 16-byte vectors and reduces its
+// sums over l four rows at a time (12 shuffles instead of 40).
+// Measured per call (s8, one symmetric density, HBM floor in brackets): nao
+// 192 609 -> 541 us (207), nao 129 341 -> 197 us (42), nao 64 107 -> 73 us;
+// s4, nao 117, two general densities 819 -> 352 us (115): bases whose size is
+// no multiple of 8 spent their time in a general kernel for the last block row.
 template <int B, bool S8, bool EDGE, bool DIAG>
 __device__ __forceinline__ void incore_fast_body(const IncoreArgs &a, const int4 it)
 {
         extern __shared__ __align__(16) double sm[];
         const int nao = a.nao;
-        double *DI = sm, *DJ = DI + B * nao;
+        double *T = sm, *ring = T + B * B, *DI = ring + STAGES * B * NT, *DJ = DI + B * nao;
         const int i0 = it.x * B, j0 = it.y * B;
+        const int nrow = min(B, nao - i0);
         const int tid = threadIdx.x, lane = tid & 31;
+        const long long c0 = it.z, c1 = it.w;
+        // the stages: row group fi of the chunk of columns at fq, slot fs
+        int fi = 0, fs = 0;
+        long long fq = c0;
+        auto fetch = [&]() {
+                if (fq < c1) {
+                        const int i = i0 + fi;
+                        const long long q = fq + tid;
+                        const long long p0 = (long long)i * (i + 1) / 2 + j0;
+                        // edge windows: rows before the chunk hold none of its columns
+                        if (!EDGE || p0 + B - 1 >= fq) {
+                                const double *row = a.eri + (S8 ? p0 * (p0 + 1) / 2 : p0 * a.npair) + q;
+                                double *dst = ring + fs * (B * NT) + tid;
+#pragma unroll
+                                for (int jj = 0; jj < B; jj++) {
+                                        // DIAG rows j > i do not exist; what is not stored reads as zero
+                                        const bool ok = q < c1 && (!DIAG || jj <= fi) && (!EDGE || q <= p0 + jj);
+                                        cp_async8z(dst + jj * NT, ok ? row : a.eri, ok);
+                                        row += S8 ? p0 + jj + 1 : a.npair;   // next row: p + 1 entries on (s8)
+                                }
+                        }
+                        fs = (fs + 1) % STAGES;
+                        if (++fi == nrow) {
+                                fi = 0;
+                                fq += NT;
+                        }
+                }
+                cp_async_commit();
+        };
+#pragma unroll
+        for (int st = 0; st < STAGES - 1; st++) fetch();
         for (int e = tid; e < B * nao; e += NT) {
                 const int r = e / nao, x = e % nao;
-                DI[e] = a.D[(size_t)(i0 + r) * nao + x];
-                DJ[e] = a.D[(size_t)(j0 + r) * nao + x];
+                DI[e] = i0 + r < nao ? a.D[(size_t)(i0 + r) * nao + x] : 0.0;
+                DJ[e] = j0 + r < nao ? a.D[(size_t)(j0 + r) * nao + x] : 0.0;
+        }
+        for (int e = tid; e < B * B; e += NT) {
+                // (diagonal blocks: rows j > i do not exist)
+                const int i = i0 + e / B, j = j0 + e % B;
+                T[e] = j <= i && i < nao ? a.t[(long long)i * (i + 1) / 2 + j] : 0.0;
         }
         __syncthreads();
         double *AI = a.A + (size_t)i0 * nao, *AJ = a.A + (size_t)j0 * nao;
-        const long long c0 = it.z, c1 = it.w;
+        int slot = 0;
         for (long long qb = c0; qb < c1; qb += NT) {
                 const long long q = qb + tid;
                 const bool active = q < c1;
@@ -236,72 +178,81 @@ __device__ __forceinline__ void incore_fast_body(const IncoreArgs &a, const int4
                 const double wkl = k == l ? 0.5 : 1.0;
                 const int k0 = __shfl_sync(0xffffffffu, k, 0);
                 const bool kuni = __all_sync(0xffffffffu, !active || k == k0);
-                double acc2[B], acc4[B];
+                double acc2[B], acc4[B], djk[B], djl[B];
 #pragma unroll
                 for (int jj = 0; jj < B; jj++) {
                         acc2[jj] = 0.0;
                         acc4[jj] = 0.0;
+                        djk[jj] = DJ[jj * nao + k];
+                        djl[jj] = DJ[jj * nao + l];
                 }
                 double colj = 0.0;
-                for (int ii = 0; ii < B; ii++) {
-                        const int i = i0 + ii;
-                        const long long p0 = (long long)i * (i + 1) / 2 + j0;
-                        // edge windows: rows before the chunk hold none of its columns
-                        if (EDGE && p0 + B - 1 < qb) continue;
-                        const double *row = a.eri + (S8 ? p0 * (p0 + 1) / 2 : p0 * a.npair) + q;
-                        double v[B];
+                for (int ib = 0; ib < nrow; ib += 4) {
+                        double a3[4];
 #pragma unroll
-                        for (int jj = 0; jj < B; jj++) {
-                                // DIAG rows j > i do not exist
-                                const bool rowok = !DIAG || jj <= ii;
-                                if (EDGE) {
-                                        const long long p = p0 + jj;
-                                        v[jj] = rowok && active && q <= p ? __ldg(row) * (q == p ? 0.5 : 1.0) : 0.0;
-                                } else {
-                                        v[jj] = rowok && active ? __ldg(row) : 0.0;
+                        for (int u = 0; u < 4; u++) {
+                                const int ii = ib + u;
+                                a3[u] = 0.0;
+                                if (ii >= nrow) continue;
+                                fetch();
+                                cp_async_wait_group<STAGES - 1>();
+                                const double *src = ring + slot * (B * NT) + tid;
+                                slot = (slot + 1) % STAGES;
+                                const int i = i0 + ii;
+                                const long long p0 = (long long)i * (i + 1) / 2 + j0;
+                                if (EDGE && p0 + B - 1 < qb) continue;
+                                const double dik = DI[ii * nao + k], dil = DI[ii * nao + l];
+                                double acc1 = 0.0, acc3 = 0.0, rp[B];
+#pragma unroll
+                                for (int jj = 0; jj < B; jj += 2) {
+                                        const double2 tw = *reinterpret_cast<const double2 *>(T + ii * B + jj);
+#pragma unroll
+                                        for (int h = 0; h < 2; h++) {
+                                                const int j = jj + h;
+                                                double v = src[j * NT];
+                                                if (EDGE && q == p0 + j) v *= 0.5;   // the packed diagonal counts half
+                                                // the K images of a row j == i count half (DIAG)
+                                                const double vk = DIAG && j == ii ? 0.5 * v : v;
+                                                acc1 += vk * djk[j];
+                                                acc3 += vk * djl[j];
+                                                acc2[j] += vk * dik;
+                                                acc4[j] += vk * dil;
+                                                colj += v * (h ? tw.y : tw.x);
+                                                rp[j] = v * tq;
+                                        }
                                 }
-                                row += S8 ? p0 + jj + 1 : a.npair;   // next row: p + 1 entries on (s8)
+                                a3[u] = wkl * acc3;
+                                if (active && acc1 != 0.0) atomicAdd(AI + (size_t)ii * nao + l, wkl * acc1);
+                                if (!kuni && active && acc3 != 0.0) atomicAdd(AI + (size_t)ii * nao + k, a3[u]);
+                                if (S8 && a.Jp) {
+                                        int rrow;
+                                        const double s = reduce_scatter<B>(rp, lane, rrow);
+                                        if ((lane & (32 / B - 1)) == 0 && (!DIAG || rrow <= ii) && s != 0.0)
+                                                atomicAdd(a.Jp + p0 + rrow, s);
+                                }
                         }
-                        const double dik = DI[ii * nao + k], dil = DI[ii * nao + l];
-                        double acc1 = 0.0, acc3 = 0.0, rp[B];
-#pragma unroll
-                        for (int jj = 0; jj < B; jj++) {
-                                // the K images of a row j == i count half (DIAG)
-                                const double vk = DIAG && jj == ii ? 0.5 * v[jj] : v[jj];
-                                acc1 += vk * DJ[jj * nao + k];
-                                acc3 += vk * DJ[jj * nao + l];
-                                acc2[jj] += vk * dik;
-                                acc4[jj] += vk * dil;
-                                colj += v[jj] * __ldg(a.t + p0 + jj);
-                                rp[jj] = v[jj] * tq;
-                        }
-                        if (active && acc1 != 0.0) atomicAdd(AI + (size_t)ii * nao + l, wkl * acc1);
                         if (kuni) {
-                                acc3 = warp_sum_d(wkl * acc3);
-                                if (lane == 0 && acc3 != 0.0) atomicAdd(AI + (size_t)ii * nao + k0, acc3);
-                        } else if (active && acc3 != 0.0) {
-                                atomicAdd(AI + (size_t)ii * nao + k, wkl * acc3);
-                        }
-                        if (S8 && a.Jp) {
                                 int rrow;
-                                const double s = reduce_scatter<B>(rp, lane, rrow);
-                                if ((lane & (32 / B - 1)) == 0 && s != 0.0) atomicAdd(a.Jp + p0 + rrow, s);
+                                const double s = reduce_scatter<4>(a3, lane, rrow);
+                                if ((lane & 7) == 0 && ib + rrow < nrow && s != 0.0)
+                                        atomicAdd(AI + (size_t)(ib + rrow) * nao + k0, s);
                         }
                 }
 #pragma unroll
                 for (int jj = 0; jj < B; jj++) {
                         acc2[jj] *= wkl;
                         acc4[jj] *= wkl;
-                        if (active && acc2[jj] != 0.0) atomicAdd(AJ + (size_t)jj * nao + l, acc2[jj]);
+                        if (active && (!DIAG || jj < nrow) && acc2[jj] != 0.0) atomicAdd(AJ + (size_t)jj * nao + l, acc2[jj]);
                 }
                 if (kuni) {
                         int rrow;
                         const double s = reduce_scatter<B>(acc4, lane, rrow);
-                        if ((lane & (32 / B - 1)) == 0 && s != 0.0) atomicAdd(AJ + (size_t)rrow * nao + k0, s);
+                        if ((lane & (32 / B - 1)) == 0 && (!DIAG || rrow < nrow) && s != 0.0)
+                                atomicAdd(AJ + (size_t)rrow * nao + k0, s);
                 } else if (active) {
 #pragma unroll
                         for (int jj = 0; jj < B; jj++)
-                                if (acc4[jj] != 0.0) atomicAdd(AJ + (size_t)jj * nao + k, acc4[jj]);
+                                if ((!DIAG || jj < nrow) && acc4[jj] != 0.0) atomicAdd(AJ + (size_t)jj * nao + k, acc4[jj]);
                 }
                 if (a.Jp && active && colj != 0.0) atomicAdd(a.Jp + q, colj);
         }
@@ -397,24 +348,16 @@ int check(const char *what, std::string &err)
 template <int B, bool S8>
 int launch_pass(const IncoreArgs &a, cudaStream_t s, std::string &err)
 {
-        const size_t smem = sizeof(double) * (4 * (size_t)B * a.nao + B * B);
-        cudaError_t e = cudaFuncSetAttribute(incore_pass_kernel<B, S8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        const size_t smem = sizeof(double) * (2 * (size_t)B * a.nao + B * B + (size_t)STAGES * B * NT);
+        cudaError_t e = cudaFuncSetAttribute(incore_fast_kernel<B, S8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
-        const size_t smem_fast = sizeof(double) * 2 * (size_t)B * a.nao;
-        if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(incore_fast_kernel<B, S8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem_fast);
         if (e != cudaSuccess) {
                 err = std::string("in-core kernel configuration: ") + cudaGetErrorString(e);
                 return 1;
         }
-        const int nfast = a.nf[0] + a.nf[1] + a.nf[2] + a.nf[3];
-        if (nfast > 0) {
-                incore_fast_kernel<B, S8><<<nfast, NT, smem_fast, s>>>(a);
-                if (check("in-core kernel launch", err)) return 1;
-        }
-        if (a.nitems > 0) {
-                incore_pass_kernel<B, S8><<<a.nitems, NT, smem, s>>>(a);
+        const int n = a.nf[0] + a.nf[1] + a.nf[2] + a.nf[3];
+        if (n > 0) {
+                incore_fast_kernel<B, S8><<<n, NT, smem, s>>>(a);
                 if (check("in-core kernel launch", err)) return 1;
         }
         return 0;
@@ -422,24 +365,30 @@ int launch_pass(const IncoreArgs &a, cudaStream_t s, std::string &err)
 
 } // namespace
 
-// 8 AO rows per block: a lane keeps 4 x B doubles in registers (the J-row
-// image sums, one row of entries and its row-J parts), which B = 8 keeps
-// under the 128 registers of two resident blocks; the shared memory of a block is 4 slabs of B x nao
-// doubles (+ B^2), so nao up to 880
+// 8 AO rows per block: a lane keeps 4 x B doubles in registers (its J-row
+// image sums and density rows), which B = 8 keeps under the 128 registers of
+// two resident blocks.  nao up to 906 (two density slabs of B x nao doubles
+// beside the 64 KB ring of entries).
 int incore_block(int nao)
 {
-        const size_t limit = 227 * 1024;
-        if (sizeof(double) * (4 * 8 * (size_t)nao + 64) <= limit) return 8;
-        return 0;
+        return nao <= 906 ? 8 : 0;
 }
 
-void incore_items(int nao, int s8, int B, long long window, std::vector<int4> (&fast)[4],
-                  std::vector<int4> &general)
+void incore_items(int nao, int s8, int B, std::vector<int4> (&items)[4])
 {
-        for (auto &v : fast) v.clear();
-        general.clear();
+        for (auto &v : items) v.clear();
         const long long npair = (long long)nao * (nao + 1) / 2;
         const int nb = (nao + B - 1) / B;
+        // columns of a window: 2048, less where that leaves fewer than four
+        // blocks per SM (nao 64: 107 us with 50 blocks)
+        long long total = 0;   // columns of all block pairs
+        for (int I = 0; I < nb; I++)
+                for (int J = 0; J <= I; J++) {
+                        const long long i1 = std::min(nao, (I + 1) * B) - 1;
+                        total += s8 ? i1 * (i1 + 1) / 2 + 1 : npair;
+                }
+        const long long want = total / (4 * 148 * NT) * NT;
+        const long long window = std::min<long long>(2048, std::max<long long>(NT, want));
         auto split = [&](std::vector<int4> &v, int I, int J, long long c0, long long c1) {
                 for (long long c = c0; c < c1; c += window)
                         v.push_back(make_int4(I, J, (int)c, (int)std::min(c1, c + window)));
@@ -449,21 +398,17 @@ void incore_items(int nao, int s8, int B, long long window, std::vector<int4> (&
                         const int imax = std::min(nao, (I + 1) * B) - 1;
                         const int jmax = std::min(std::min(nao, (J + 1) * B) - 1, imax);
                         const long long pmax = (long long)imax * (imax + 1) / 2 + jmax;
-                        const long long ncol = s8 ? pmax + 1 : npair;
-                        const bool full = (I + 1) * B <= nao;
                         const int diag = I == J ? 2 : 0;
-                        if (!full) {
-                                split(general, I, J, 0, ncol);
-                        } else if (!s8) {
-                                split(fast[diag], I, J, 0, ncol);
+                        if (!s8) {
+                                split(items[diag], I, J, 0, npair);
                         } else {
                                 // the block's first row (i0, j0): columns
                                 // before it are below the packed diagonal for
                                 // every row of the block
                                 const long long i0 = (long long)I * B;
                                 const long long pmin = i0 * (i0 + 1) / 2 + (long long)J * B;
-                                split(fast[diag], I, J, 0, pmin);
-                                split(fast[diag + 1], I, J, pmin, ncol);
+                                split(items[diag], I, J, 0, pmin);
+                                split(items[diag + 1], I, J, pmin, pmax + 1);
                         }
                 }
 }

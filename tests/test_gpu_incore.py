@@ -167,3 +167,33 @@ def test_int2e_s8_cartesian_and_range_separated(tag):
     _close(vk, g['%s_vk' % tag])
     del eri
     torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize('nao', [1, 7, 8, 9, 15, 16, 23, 65])
+@pytest.mark.parametrize('sym', ['s8', 's4'])
+@pytest.mark.parametrize('hermi', [0, 1, 2])
+def test_incore_block_edges(nao, sym, hermi):
+    """Bases on both sides of the 8-function blocks (partial last block rows,
+    a single block, several column windows) against the full contraction in
+    float64.  1e-12 relative to the largest element: sums of nao^2 products."""
+    from pyscf_b200 import incore, lib
+    if lib.device_count() == 0:
+        pytest.skip('no GPU')
+    rng = numpy.random.default_rng(nao)
+    npair = nao * (nao + 1) // 2
+    m = rng.standard_normal((npair, npair))
+    m = m + m.T
+    eri = m[numpy.tril_indices(npair)] if sym == 's8' else m
+    d = rng.standard_normal((2, nao, nao))
+    if hermi:
+        d = d + (1 if hermi == 1 else -1) * d.transpose(0, 2, 1)
+    a = numpy.arange(nao)
+    hi, lo = numpy.maximum(a[:, None], a), numpy.minimum(a[:, None], a)
+    tri = hi * (hi + 1) // 2 + lo
+    full = m[tri][:, :, tri]
+    rj = numpy.einsum('ijkl,sji->skl', full, d)
+    rk = numpy.einsum('ijkl,sjk->sil', full, d)
+    vj, vk = incore.incore(eri, d, hermi=hermi)
+    scale = abs(rk).max()
+    assert abs(vj - rj).max() <= 1e-12 * max(scale, abs(rj).max())
+    assert abs(vk - rk).max() <= 1e-12 * scale
