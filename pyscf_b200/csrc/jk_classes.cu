@@ -46,7 +46,7 @@ int launch_one(const JKArgs &a, const JKArgs *margs, const long long *mchunk, in
                         int nb = 0;
                         if constexpr (thread) {
                                 cfg.block = 128;
-                                cfg.smem = stage_table<R>(K::NR) ? sizeof(R) * rys_slice_elems<R>(K::NR) : 0;
+                                cfg.smem = stage_table<R>(K::NR) ? sizeof(R) * RysStaged<K::NR, R>::ELEMS : 0;
                                 cfg.status = cudaFuncSetAttribute(jk_thread_kernel<LA, LB, LC, LD, (NP > 0 ? NP : 1), R, MULTI, KR>,
                                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem);
                                 if (cfg.status == cudaSuccess)
@@ -99,7 +99,7 @@ int launch_run(const JKArgs &a, cudaStream_t s, int nsm, std::string &err)
                 if (!cfg.ready) {
                         int nb = 0;
                         cfg.block = 128;
-                        cfg.smem = stage_table<double>(K::NR) ? sizeof(double) * rys_slice_elems<double>(K::NR) : 0;
+                        cfg.smem = stage_table<double>(K::NR) ? sizeof(double) * RysStaged<K::NR, double>::ELEMS : 0;
                         cfg.status = cudaFuncSetAttribute(jk_thread_run_kernel<LA, LB, LC, LD, BR>,
                                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem);
                         if (cfg.status == cudaSuccess)

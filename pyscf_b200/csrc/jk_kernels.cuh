@@ -403,6 +403,20 @@ template <typename R> __host__ __device__ constexpr bool stage_table(int nr)
 {
         return sizeof(R) == 4 || nr <= 4;
 }
+// copies the order-NR slice into shared memory (RysStaged layout), all
+// threads of the block
+template <int NR, typename R> __device__ __forceinline__ void stage_rys(R *dst, const R *src)
+{
+        using S = RysStaged<NR, R>;
+        constexpr int V = 16 / (int)sizeof(R), NV = S::ROW / V;   // 16-byte vectors of a row
+        constexpr int ROWS = RysLayout<R>::t_asym(NR) * 2 * NR;
+        for (int e = threadIdx.x; e < ROWS * NV; e += blockDim.x) {
+                const int row = e / NV, k = e - row * NV, p = row / (2 * NR), f = row - p * (2 * NR);
+                *reinterpret_cast<RysVec16<R> *>(dst + p * S::PIECE + f * S::ROW + k * V) =
+                        *reinterpret_cast<const RysVec16<R> *>(src + row * RysLayout<R>::ROW + k * V);
+        }
+        __syncthreads();
+}
 template <> __device__ __forceinline__ const double *table_of<double>(const JKArgs &a) { return a.table; }
 template <> __device__ __forceinline__ const float *table_of<float>(const JKArgs &a) { return a.table_f; }
 
@@ -456,11 +470,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk
         if (!loop.block_has_work()) return;
         const R *tab = table_of<R>(a0) + RysLayout<R>::offset(K::NR);
         if constexpr (stage_table<R>(K::NR)) {
-                constexpr int NS = rys_slice_elems<R>(K::NR);
-                const RysVec4<R> *src = reinterpret_cast<const RysVec4<R> *>(tab);
-                RysVec4<R> *dst = reinterpret_cast<RysVec4<R> *>(smem_dyn);
-                for (int t = threadIdx.x; t < NS / 4; t += blockDim.x) dst[t] = src[t];
-                __syncthreads();
+                stage_rys<K::NR, R>(reinterpret_cast<R *>(smem_dyn), tab);
                 tab = reinterpret_cast<const R *>(smem_dyn);
         }
         unsigned long long nq = 0, npq = 0;
@@ -559,7 +569,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk
                                                 PrimQ<R> sq;
                                                 prim_setup<R>(sq, (R)P.w, (R)KP.y, Pv, (R)Q.w, (R)KQ.y, Qv, A, C,
                                                               Kab * (R)KQ.x, (R)a.omega2);
-                                                add_prim_quartet_part<LA, LB, LC, LD, PART * NGP, NGP, R>(Gp, tab, sq, AB, CD);
+                                                add_prim_quartet_part<LA, LB, LC, LD, PART * NGP, NGP, R, stage_table<R>(K::NR)>(Gp, tab, sq, AB, CD);
                                         }
                                         while (kp >= pk.y) { kp -= pk.y; ip++; }
                                 }
@@ -749,12 +759,8 @@ __global__ void __launch_bounds__(128, B2_THREAD_MINB) jk_thread_run_kernel(JKAr
         if (!loop.block_has_work()) return;
         const double *tab = a.table + RysLayout<double>::offset(K::NR);
         if constexpr (stage_table<double>(K::NR)) {
-                constexpr int NS = rys_slice_elems<double>(K::NR);
-                const RysVec4<double> *src = reinterpret_cast<const RysVec4<double> *>(tab);
-                RysVec4<double> *dst = reinterpret_cast<RysVec4<double> *>(smem_dyn);
-                for (int t = threadIdx.x; t < NS / 4; t += blockDim.x) dst[t] = src[t];
-                __syncthreads();
-                tab = reinterpret_cast<const double *>(smem_dyn);
+                stage_rys<K::NR, double>(smem_dyn, tab);
+                tab = smem_dyn;
         }
         const size_t n = (size_t)a.naoc;
         const int nrun = a.tile_b / BR;   // runs per tile
@@ -839,7 +845,7 @@ __global__ void __launch_bounds__(128, B2_THREAD_MINB) jk_thread_run_kernel(JKAr
                                                 const double Qv[3] = {Q.x - Ab.x, Q.y - Ab.y, Q.z - Ab.z};
                                                 PrimQ<double> sq;
                                                 prim_setup<double>(sq, P.w, KP.y, Pv, Q.w, KQ.y, Qv, A0, C, Kab * KQ.x, a.omega2);
-                                                add_prim_quartet_part<LA, LB, LC, LD, 0, NG, double>(G, tab, sq, AB, CD);
+                                                add_prim_quartet_part<LA, LB, LC, LD, 0, NG, double, stage_table<double>(K::NR)>(G, tab, sq, AB, CD);
                                         }
                                 }
                                 nq++;

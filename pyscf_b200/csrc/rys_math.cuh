@@ -159,6 +159,22 @@ template <> struct RysLayout<float> {
         static B2_HDC int offset(int n) { return rys_f_offset(n); }
 };
 
+// The order-NR slice as kernels keep it in shared memory: rows without their
+// padding, pieces 16 bytes longer than their rows.  Lanes read the same row
+// offset of different pieces at once; with the global layout's 128-byte rows
+// every piece starts on the same bank (up to 8 wavefronts per 8 lanes of a
+// 16-byte load), here eight consecutive pieces start on different ones.
+template <int NR, typename R>
+struct RysStaged {
+        static constexpr int ROW = sizeof(R) == 8 ? RYS_DEG + 1 : RYS_F_ROW;
+        static constexpr int PIECE = 2 * NR * ROW + 16 / (int)sizeof(R);
+        static constexpr int ELEMS = RysLayout<R>::t_asym(NR) * PIECE;
+};
+template <typename R>
+struct alignas(16) RysVec16 {
+        R v[16 / sizeof(R)];
+};
+
 // elements of the order-n slice of the table of type R
 template <typename R>
 B2_HDC int rys_slice_elems(int n) { return RysLayout<R>::t_asym(n) * 2 * n * RysLayout<R>::ROW; }
@@ -216,6 +232,47 @@ B2_HD void rys_roots_slice(R T, const R *__restrict__ tab, R *u, R *w)
         for (int f = 0; f < NR; f++) {
                 u[f] = rys_poly<R>(c + f * L::ROW, x);
                 w[f] = rys_poly<R>(c + (NR + f) * L::ROW, x);
+        }
+}
+
+// Horner evaluation of a staged row (16-byte aligned)
+template <typename R>
+B2_HD R rys_poly_staged(const R *__restrict__ row, R x)
+{
+        constexpr int V = 16 / (int)sizeof(R), N = (sizeof(R) == 8 ? RYS_DEG + 1 : RYS_F_ROW);
+        static_assert(N % V == 0, "whole 16-byte vectors");
+        RysVec16<R> q[N / V];
+#pragma unroll
+        for (int k = 0; k < N / V; k++) q[k] = reinterpret_cast<const RysVec16<R> *>(row)[k];
+        R r = q[N / V - 1].v[V - 1];
+#pragma unroll
+        for (int k = N - 2; k >= 0; k--) r = b2fma(r, x, q[k / V].v[k % V]);
+        return r;
+}
+
+// rys_roots_slice from a staged slice (the same arithmetic)
+template <int NR, typename R>
+B2_HD void rys_roots_staged(R T, const R *__restrict__ tab, R *u, R *w)
+{
+        using L = RysLayout<R>;
+        using S = RysStaged<NR, R>;
+        if (!(T < (R)L::t_asym(NR))) {
+                const R it = (R)1 / T;
+                const R st = b2sqrt(it);
+#pragma unroll
+                for (int i = 0; i < NR; i++) {
+                        u[i] = (R)rys_herm_x2(NR * (NR - 1) / 2 + i) * it;
+                        w[i] = (R)rys_herm_w(NR * (NR - 1) / 2 + i) * st;
+                }
+                return;
+        }
+        const int p = (int)T;
+        const R x = (R)2 * (T - (R)p) - (R)1;
+        const R *c = tab + p * S::PIECE;
+#pragma unroll
+        for (int f = 0; f < NR; f++) {
+                u[f] = rys_poly_staged<R>(c + f * S::ROW, x);
+                w[f] = rys_poly_staged<R>(c + (NR + f) * S::ROW, x);
         }
 }
 
@@ -417,13 +474,15 @@ B2_HD void assemble_part(R *Gp, const R *hx, const R *hy, const R *hz, std::inte
 }
 
 // One primitive quartet into components [BASE, BASE + N) of the block.
-// `tab` is the order-NR slice of the padded table of type R.
-template <int LA, int LB, int LC, int LD, int BASE, int N, typename R>
+// `tab` is the order-NR slice of the padded table of type R, or (STAGED) its
+// shared-memory form.
+template <int LA, int LB, int LC, int LD, int BASE, int N, typename R, bool STAGED = false>
 B2_HD void add_prim_quartet_part(R *Gp, const R *tab, const PrimQ<R> &s, const R AB[3], const R CD[3])
 {
         using K = Class4<LA, LB, LC, LD>;
         R u[K::NR], w[K::NR];
-        rys_roots_slice<K::NR, R>(s.T, tab, u, w);
+        if constexpr (STAGED) rys_roots_staged<K::NR, R>(s.T, tab, u, w);
+        else rys_roots_slice<K::NR, R>(s.T, tab, u, w);
 #pragma unroll
         for (int r = 0; r < K::NR; r++) {
                 RysCoef<R> rc;
