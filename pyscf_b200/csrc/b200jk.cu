@@ -2447,16 +2447,24 @@ struct b200jk_batch {
         cudaStream_t stream = nullptr;
         cudaEvent_t ev0 = nullptr, ev1 = nullptr;
         DevArr<JKArgs> args;
-        DevArr<int> segoff, nkl, kst;
+        // per entry (a molecule in a class and pass): first segment and class;
+        // per class and pass: what its entries share
+        DevArr<long long> seg0;
+        DevArr<int> cls, nkl, kst;
+        DevArr<BatchClass> bc;
         DevArr<long long> nchunk, chunk_off, mchunk;
         DevArr<unsigned char> cub_tmp;
         DevArr<unsigned long long> stats;
-        JKArgs *h_args = nullptr;       // pinned staging of the per-class argument arrays
-        int *h_segoff = nullptr;
-        size_t h_cap_args = 0, h_cap_seg = 0;
-        // staging of the asynchronous entry (read by captured graphs at replay)
-        JKArgs *h_args_async = nullptr;
-        int *h_segoff_async = nullptr;
+        StreamFan fan;                  // the batch's own: captured graphs hold forks to it
+        // pinned staging of the synchronous [0] and the asynchronous [1] entry
+        // (read by captured graphs at replay)
+        struct Staging {
+                JKArgs *args = nullptr;
+                long long *seg0 = nullptr;
+                int *cls = nullptr;
+                BatchClass *bc = nullptr;
+        } staging[2];
+        size_t h_cap = 0;               // entries the staging holds
         // workspace generation of every plan when the last synchronous build
         // sized the buffers; the asynchronous entry refuses to run when a
         // plan's workspace has moved since (its captured graphs would use the
@@ -2466,14 +2474,23 @@ struct b200jk_batch {
         const float *tbl_f = nullptr;
         int64_t quartets = 0, prim_quartets = 0, fp32_quartets = 0, launches = 0;
         double last_ms = 0;
+        void free_staging()
+        {
+                for (Staging &h : staging) {
+                        if (h.args) cudaFreeHost(h.args);
+                        if (h.seg0) cudaFreeHost(h.seg0);
+                        if (h.cls) cudaFreeHost(h.cls);
+                        if (h.bc) cudaFreeHost(h.bc);
+                        h = Staging();
+                }
+                h_cap = 0;
+        }
         ~b200jk_batch()
         {
-                args.release(); segoff.release(); nkl.release(); kst.release(); nchunk.release();
-                chunk_off.release(); mchunk.release(); cub_tmp.release(); stats.release();
-                if (h_args) cudaFreeHost(h_args);
-                if (h_segoff) cudaFreeHost(h_segoff);
-                if (h_args_async) cudaFreeHost(h_args_async);
-                if (h_segoff_async) cudaFreeHost(h_segoff_async);
+                args.release(); seg0.release(); cls.release(); bc.release(); nkl.release(); kst.release();
+                nchunk.release(); chunk_off.release(); mchunk.release(); cub_tmp.release(); stats.release();
+                fan.release();
+                free_staging();
                 if (ev0) cudaEventDestroy(ev0);
                 if (ev1) cudaEventDestroy(ev1);
                 if (stream) cudaStreamDestroy(stream);
@@ -2555,60 +2572,57 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
         }
         auto qcs = quartet_classes();
         const int nclass = (int)qcs.size();
-        // argument arrays of every (class, pass): only molecules with work in the class
-        std::vector<size_t> at(2 * nclass + 1, 0), sat(2 * nclass + 1, 0);
-        std::vector<int> ncnt(2 * nclass, 0);
-        size_t tot_args = 0, tot_seg = 0;
-        int max_segs = 1;
+        // the entries, class-major: the molecules with work in each class, for
+        // the float64 pass and (mixed) the float32 pass.  Buffers are sized for
+        // both passes whatever this call's precision
+        std::vector<size_t> at(2 * nclass, 0);
+        std::vector<int> ncnt(nclass, 0);
+        size_t cap = 0, nent = 0;
+        long long cap_segs = 0, nseg = 0;
         for (int t = 0; t < nclass; t++) {
-                int cnt = 0, segs = 0;
+                long long segs = 0;
                 for (int m = 0; m < nmol; m++) {
                         const PairClassDev &bra = B->plans[m]->pc[qcs[t].X], &ket = B->plans[m]->pc[qcs[t].Y];
                         if (bra.n == 0 || ket.n == 0) continue;
-                        cnt++;
-                        segs += bra.n * B2_NBUCKET;
+                        ncnt[t]++;
+                        segs += (long long)bra.n * B2_NBUCKET;
                 }
-                max_segs = std::max(max_segs, segs);
-                for (int pass = 0; pass < 2; pass++) {
-                        at[2 * t + pass] = tot_args;
-                        sat[2 * t + pass] = tot_seg;
-                        ncnt[2 * t + pass] = cnt;
-                        tot_args += cnt;
-                        tot_seg += cnt + 1;
+                cap += 2 * (size_t)ncnt[t];
+                cap_segs += 2 * segs;
+                const int np = mixed && class_tau(B->plans[0], t) > 0 ? 2 : 1;
+                for (int pass = 0; pass < np; pass++) {
+                        at[2 * t + pass] = nent;
+                        nent += ncnt[t];
+                        nseg += segs;
                 }
         }
+        if (cap_segs + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one batch");
         if (async) {
-                if (tot_args > B->h_cap_args || tot_seg > B->h_cap_seg || !B->h_args_async || B->args.n < tot_args)
+                if (cap > B->h_cap || !B->staging[1].args || B->args.n < cap || B->nkl.n < (size_t)cap_segs)
                         return fail(B200JK_EINVAL, "b200jk_batch_get_jk_async needs one b200jk_batch_get_jk call first");
         } else {
-                if (tot_args > B->h_cap_args || !B->h_args_async) {
-                        if (B->h_args) cudaFreeHost(B->h_args);
-                        if (B->h_args_async) cudaFreeHost(B->h_args_async);
-                        B->h_args = B->h_args_async = nullptr;
-                        CUDA_TRY(cudaMallocHost(&B->h_args, sizeof(JKArgs) * tot_args));
-                        CUDA_TRY(cudaMallocHost(&B->h_args_async, sizeof(JKArgs) * tot_args));
-                        B->h_cap_args = tot_args;
+                if (cap > B->h_cap || !B->staging[1].args) {
+                        B->free_staging();
+                        for (auto &h : B->staging) {
+                                CUDA_TRY(cudaMallocHost(&h.args, sizeof(JKArgs) * std::max<size_t>(1, cap)));
+                                CUDA_TRY(cudaMallocHost(&h.seg0, sizeof(long long) * (cap + 1)));
+                                CUDA_TRY(cudaMallocHost(&h.cls, sizeof(int) * std::max<size_t>(1, cap)));
+                                CUDA_TRY(cudaMallocHost(&h.bc, sizeof(BatchClass) * 2 * nclass));
+                        }
+                        B->h_cap = cap;
                 }
-                if (tot_seg > B->h_cap_seg || !B->h_segoff_async) {
-                        if (B->h_segoff) cudaFreeHost(B->h_segoff);
-                        if (B->h_segoff_async) cudaFreeHost(B->h_segoff_async);
-                        B->h_segoff = B->h_segoff_async = nullptr;
-                        CUDA_TRY(cudaMallocHost(&B->h_segoff, sizeof(int) * tot_seg));
-                        CUDA_TRY(cudaMallocHost(&B->h_segoff_async, sizeof(int) * tot_seg));
-                        B->h_cap_seg = tot_seg;
-                }
-                if ((rc = dev_alloc(B->args, std::max<size_t>(1, tot_args))) ||
-                    (rc = dev_alloc(B->segoff, std::max<size_t>(1, tot_seg))) || (rc = dev_alloc(B->nkl, max_segs)) ||
-                    (rc = dev_alloc(B->kst, max_segs)) || (rc = dev_alloc(B->nchunk, max_segs + 1)) ||
-                    (rc = dev_alloc(B->chunk_off, max_segs + 1)) || (rc = dev_alloc(B->mchunk, nmol + 1)) ||
-                    (rc = dev_alloc(B->stats, 6 * 64)))
+                const size_t ns = (size_t)std::max(1ll, cap_segs);
+                if ((rc = dev_alloc(B->args, std::max<size_t>(1, cap))) || (rc = dev_alloc(B->seg0, cap + 1)) ||
+                    (rc = dev_alloc(B->cls, std::max<size_t>(1, cap))) || (rc = dev_alloc(B->bc, 2 * nclass)) ||
+                    (rc = dev_alloc(B->nkl, ns)) || (rc = dev_alloc(B->kst, ns)) || (rc = dev_alloc(B->nchunk, ns + 1)) ||
+                    (rc = dev_alloc(B->chunk_off, ns + 1)) || (rc = dev_alloc(B->mchunk, cap + 1)) ||
+                    (rc = dev_alloc(B->stats, 6 * 64)) || (rc = B->fan.create()))
                         return rc;
                 size_t cub_bytes = 0;
-                cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, B->nchunk.p, B->chunk_off.p, max_segs + 1);
+                cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, B->nchunk.p, B->chunk_off.p, (int)(cap_segs + 1));
                 if ((rc = dev_alloc(B->cub_tmp, cub_bytes + 16))) return rc;
         }
-        JKArgs *h_args = async ? B->h_args_async : B->h_args;
-        int *h_segoff = async ? B->h_segoff_async : B->h_segoff;
+        const b200jk_batch::Staging &h = B->staging[async ? 1 : 0];
 
         if (!async) CUDA_TRY(cudaEventRecord(B->ev0, s));
         int64_t launches = 0;
@@ -2642,81 +2656,102 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
         CUDA_TRY(cudaMemsetAsync(B->stats.p, 0, 6 * 64 * sizeof(unsigned long long), s));
         const double *tbl = B->tbl;
         const float *tbl_f = B->tbl_f;
-        // argument arrays (pointers only depend on the workspaces): fill and upload once
-        for (int t = 0; t < nclass; t++) {
-                for (int pass = 0; pass < 2; pass++) {
-                        JKArgs *ha = h_args + at[2 * t + pass];
-                        int *hs = h_segoff + sat[2 * t + pass];
-                        int k = 0, seg = 0;
-                        for (int m = 0; m < nmol; m++) {
-                                b200jk_plan *P = B->plans[m];
-                                const PairClassDev &bra = P->pc[qcs[t].X], &ket = P->pc[qcs[t].Y];
-                                if (bra.n == 0 || ket.n == 0) continue;
-                                JKArgs a{};
-                                a.bra = bra.view();
-                                a.ket = ket.view();
-                                a.PP = P->PP.p; a.PK = P->PK.p;
-                                a.chunk_off = B->chunk_off.p + seg;
-                                a.nkl = B->nkl.p + seg;
-                                a.kst = B->kst.p + seg;
-                                a.dm_cond = P->dm_cond.p;
-                                a.table = tbl;
-                                a.table_f = tbl_f;
-                                a.goff = P->goff_all.p + P->goff_at[t];
-                                a.Jacc = P->Jacc.p; a.Kacc = P->Kacc.p;
-                                a.Ds = P->Ds.p; a.Dk = P->Dc.p;
-                                a.Dpk = P->Dpk.p + P->pk_off[qcs[t].Y];
-                                a.Jpk = P->Jpk.p + P->pk_off[qcs[t].Y];
-                                a.pk_stride = P->pk_total;
-                                a.stats = B->stats.p + 2 * (64 * pass + t);
-                                a.dmax4 = (const double *)P->dmax.p;
-                                a.tol = P->tol > 0 ? P->tol : -1.0;
-                                a.nbas = P->nbas; a.naoc = P->naoc; a.n_dm = 1; a.nk = nk;
-                                a.with_j = with_j; a.with_k = with_k; a.same = qcs[t].X == qcs[t].Y;
-                                a.screen = P->screen;
-                                a.omega2 = P->omega2;
-                                a.split = 1;
-                                ha[k] = a;
-                                hs[k] = seg;
-                                k++;
-                                seg += bra.n * B2_NBUCKET;
+        // the entries (pointers only depend on the workspaces): fill and upload
+        {
+                long long seg = 0;
+                for (int t = 0; t < nclass; t++) {
+                        int la, lb, lc, ld;
+                        class_l(qcs[t].X, la, lb);
+                        class_l(qcs[t].Y, lc, ld);
+                        const double tau = mixed ? class_tau(B->plans[0], t) : 0.0;
+                        for (int pass = 0; pass < (tau > 0 ? 2 : 1); pass++) {
+                                // bra runs (variant 2) need the tiled pass of one plan: a batch
+                                // runs those classes as variant 0
+                                int variant = class_variant(B->plans[0], t, pass);
+                                if (variant == 2) variant = 0;
+                                BatchClass &c = h.bc[2 * t + pass];
+                                c.chunk = family_chunk(la, lb, lc, ld, variant);
+                                c.most = family_is_thread(la, lb, lc, ld) ? (variant == 0 ? 5 : 0) : 3;
+                                c.pass = pass;
+                                c.pad = 0;
+                                c.tau = tau;
+                                size_t e = at[2 * t + pass];
+                                for (int m = 0; m < nmol; m++) {
+                                        b200jk_plan *P = B->plans[m];
+                                        const PairClassDev &bra = P->pc[qcs[t].X], &ket = P->pc[qcs[t].Y];
+                                        if (bra.n == 0 || ket.n == 0) continue;
+                                        JKArgs a{};
+                                        a.bra = bra.view();
+                                        a.ket = ket.view();
+                                        a.PP = P->PP.p; a.PK = P->PK.p;
+                                        a.chunk_off = B->chunk_off.p + seg;
+                                        a.nkl = B->nkl.p + seg;
+                                        a.kst = B->kst.p + seg;
+                                        a.dm_cond = P->dm_cond.p;
+                                        a.table = tbl;
+                                        a.table_f = tbl_f;
+                                        a.goff = P->goff_all.p + P->goff_at[t];
+                                        a.Jacc = P->Jacc.p; a.Kacc = P->Kacc.p;
+                                        a.Ds = P->Ds.p; a.Dk = P->Dc.p;
+                                        a.Dpk = P->Dpk.p + P->pk_off[qcs[t].Y];
+                                        a.Jpk = P->Jpk.p + P->pk_off[qcs[t].Y];
+                                        a.pk_stride = P->pk_total;
+                                        a.stats = B->stats.p + 2 * (64 * pass + t);
+                                        a.next = B->stats.p + 4 * 64 + 64 * pass + t;
+                                        a.dmax4 = (const double *)P->dmax.p;
+                                        a.tol = P->tol > 0 ? P->tol : -1.0;
+                                        a.nbas = P->nbas; a.naoc = P->naoc; a.n_dm = 1; a.nk = nk;
+                                        a.with_j = with_j; a.with_k = with_k; a.same = qcs[t].X == qcs[t].Y;
+                                        a.screen = P->screen;
+                                        a.omega2 = P->omega2;
+                                        a.split = 1;
+                                        h.args[e] = a;
+                                        h.seg0[e] = seg;
+                                        h.cls[e] = 2 * t + pass;
+                                        e++;
+                                        seg += (long long)bra.n * B2_NBUCKET;
+                                }
                         }
-                        hs[k] = seg;
                 }
+                h.seg0[nent] = seg;
         }
-        CUDA_TRY(cudaMemcpyAsync(B->args.p, h_args, sizeof(JKArgs) * tot_args, cudaMemcpyHostToDevice, s));
-        CUDA_TRY(cudaMemcpyAsync(B->segoff.p, h_segoff, sizeof(int) * tot_seg, cudaMemcpyHostToDevice, s));
-        for (int t = 0; t < nclass; t++) {
-                int la, lb, lc, ld;
-                class_l(qcs[t].X, la, lb);
-                class_l(qcs[t].Y, lc, ld);
-                const double tau = mixed ? class_tau(B->plans[0], t) : 0.0;
-                for (int pass = 0; pass < (tau > 0 ? 2 : 1); pass++) {
-                        const int nm = ncnt[2 * t + pass];
-                        if (nm == 0) continue;
-                        // bra runs (variant 2) need the tiled pass of one plan: a batch
-                        // runs those classes as variant 0
-                        int variant = class_variant(B->plans[0], t, pass);
-                        if (variant == 2) variant = 0;
-                        const int chunk = family_chunk(la, lb, lc, ld, variant);
-                        const JKArgs *dargs = B->args.p + at[2 * t + pass];
-                        const int *dseg = B->segoff.p + sat[2 * t + pass];
-                        const int segs = h_segoff[sat[2 * t + pass] + nm];
-                        const int most = family_is_thread(la, lb, lc, ld) ? (variant == 0 ? 5 : 0) : 3;
-                        count_kernel_multi<<<grid_for(segs, 256), 256, 0, s>>>(dargs, dseg, nm, chunk, most, tau,
-                                                                              pass, B->nkl.p, B->kst.p, B->nchunk.p);
-                        CUDA_TRY(cudaGetLastError());
-                        CUDA_TRY(cudaMemsetAsync(B->nchunk.p + segs, 0, sizeof(long long), s));
-                        size_t tmp = B->cub_tmp.n;
-                        CUDA_TRY(cub::DeviceScan::ExclusiveSum(B->cub_tmp.p, tmp, B->nchunk.p, B->chunk_off.p, segs + 1, s));
-                        batch_chunk_starts<<<grid_for(nm + 1, 128), 128, 0, s>>>(B->chunk_off.p, dseg, nm, B->mchunk.p);
-                        CUDA_TRY(cudaGetLastError());
-                        JKArgs a0 = h_args[at[2 * t + pass]];
-                        a0.next = B->stats.p + 4 * 64 + 64 * pass + t;
-                        if ((rc = dispatch_jk(B->plans[0], la, lb, lc, ld, a0, pass, s, dargs, B->mchunk.p, nm, variant)))
-                                return rc;
-                        launches += 3;
+        if (nent > 0) {
+                CUDA_TRY(cudaMemcpyAsync(B->args.p, h.args, sizeof(JKArgs) * nent, cudaMemcpyHostToDevice, s));
+                CUDA_TRY(cudaMemcpyAsync(B->seg0.p, h.seg0, sizeof(long long) * (nent + 1), cudaMemcpyHostToDevice, s));
+                CUDA_TRY(cudaMemcpyAsync(B->cls.p, h.cls, sizeof(int) * nent, cudaMemcpyHostToDevice, s));
+                CUDA_TRY(cudaMemcpyAsync(B->bc.p, h.bc, sizeof(BatchClass) * 2 * nclass, cudaMemcpyHostToDevice, s));
+                count_kernel_multi<<<grid_for(nseg, 256), 256, 0, s>>>(B->args.p, B->seg0.p, B->cls.p, B->bc.p, (int)nent,
+                                                                      B->nkl.p, B->kst.p, B->nchunk.p);
+                CUDA_TRY(cudaGetLastError());
+                CUDA_TRY(cudaMemsetAsync(B->nchunk.p + nseg, 0, sizeof(long long), s));
+                size_t tmp = B->cub_tmp.n;
+                CUDA_TRY(cub::DeviceScan::ExclusiveSum(B->cub_tmp.p, tmp, B->nchunk.p, B->chunk_off.p, (int)(nseg + 1), s));
+                batch_chunk_starts<<<grid_for((long long)nent + 1, 128), 128, 0, s>>>(B->chunk_off.p, B->seg0.p, (int)nent,
+                                                                                    B->mchunk.p);
+                CUDA_TRY(cudaGetLastError());
+                launches += 2;
+                if ((rc = B->fan.fork(s))) return rc;
+                for (int t = 0; t < nclass; t++) {
+                        if (ncnt[t] == 0) continue;
+                        int la, lb, lc, ld;
+                        class_l(qcs[t].X, la, lb);
+                        class_l(qcs[t].Y, lc, ld);
+                        const double tau = mixed ? class_tau(B->plans[0], t) : 0.0;
+                        for (int pass = 0; pass < (tau > 0 ? 2 : 1); pass++) {
+                                int variant = class_variant(B->plans[0], t, pass);
+                                if (variant == 2) variant = 0;
+                                const size_t e = at[2 * t + pass];
+                                cudaStream_t cs = s;
+                                if ((rc = B->fan.take(s, cs)) ||
+                                    (rc = dispatch_jk(B->plans[0], la, lb, lc, ld, h.args[e], pass, cs, B->args.p + e,
+                                                      B->mchunk.p + e, ncnt[t], variant))) {
+                                        B->fan.join(s);
+                                        return rc;
+                                }
+                                launches++;
+                        }
                 }
+                if ((rc = B->fan.join(s))) return rc;
         }
         // back to the output basis, per molecule
         for (int m = 0; m < nmol; m++) {

@@ -319,32 +319,41 @@ static __global__ void count_kernel(PairView bra, PairView ket, int same, double
         count_segment(bra, ket, same, tol, *dmax4, chunk, tau32, pass, shard, nshard, t, nkl[t], kst[t], nchunk[t]);
 }
 
-// Count kernel of a batch of molecules: one thread per segment of the batch;
-// molecule m owns segments [segoff[m], segoff[m+1]) of the concatenated
-// nkl/kst/nchunk arrays.
-static __global__ void count_kernel_multi(const JKArgs *__restrict__ margs, const int *__restrict__ segoff, int nmol,
-                                          int chunk, int most, double tau32, int pass, int *nkl, int *kst,
-                                          long long *nchunk)
+// What one class and pass of a batch shares: chunk length, cut limit of its
+// segments, precision pass, float32 threshold.
+struct BatchClass {
+        int chunk, most, pass, pad;
+        double tau;
+};
+
+// Count kernel of a batch of molecules, all classes and passes in one launch:
+// entry e (a molecule in a class and pass) owns segments [seg0[e],
+// seg0[e + 1]) of the concatenated nkl/kst/nchunk arrays.
+static __global__ void count_kernel_multi(const JKArgs *__restrict__ margs, const long long *__restrict__ seg0,
+                                          const int *__restrict__ cls, const BatchClass *__restrict__ bc, int nent,
+                                          int *nkl, int *kst, long long *nchunk)
 {
-        const int t = blockIdx.x * blockDim.x + threadIdx.x;
-        if (t >= segoff[nmol]) return;
-        int lo = 0, hi = nmol;   // segoff[lo] <= t < segoff[hi]
+        const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+        if (t >= seg0[nent]) return;
+        int lo = 0, hi = nent;   // seg0[lo] <= t < seg0[hi]
         while (hi - lo > 1) {
                 const int mid = (lo + hi) >> 1;
-                if (segoff[mid] <= t) lo = mid;
+                if (seg0[mid] <= t) lo = mid;
                 else hi = mid;
         }
         const JKArgs &a = margs[lo];
-        const int sgi = t - segoff[lo];
-        count_segment(a.bra, a.ket, a.same, a.tol > 0 ? a.tol : 0.0, *a.dmax4, chunk >> segment_split(a, sgi, most),
-                      tau32, pass, 0, 1, sgi, nkl[t], kst[t], nchunk[t]);
+        const BatchClass c = bc[cls[lo]];
+        const int sgi = (int)(t - seg0[lo]);
+        count_segment(a.bra, a.ket, a.same, a.tol > 0 ? a.tol : 0.0, *a.dmax4,
+                      c.chunk >> segment_split(a, sgi, c.most), c.tau, c.pass, 0, 1, sgi, nkl[t], kst[t], nchunk[t]);
 }
 
-// first chunk of every molecule of a batch: mchunk[m] = chunk_off[segoff[m]]
-static __global__ void batch_chunk_starts(const long long *chunk_off, const int *segoff, int nmol, long long *mchunk)
+// first chunk of every entry: mchunk[e] = chunk_off[seg0[e]]; a class's last
+// entry ends where the next class's first one starts
+static __global__ void batch_chunk_starts(const long long *chunk_off, const long long *seg0, int nent, long long *mchunk)
 {
         const int m = blockIdx.x * blockDim.x + threadIdx.x;
-        if (m <= nmol) mchunk[m] = chunk_off[segoff[m]];
+        if (m <= nent) mchunk[m] = chunk_off[seg0[m]];
 }
 
 // All quartet classes (and precision passes) of one build counted in one
@@ -465,7 +474,7 @@ __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk
         // small (float64 up to four roots, <= 59 KB; float32 always, <= 27 KB),
         // read from global memory otherwise
         extern __shared__ __align__(32) double smem_dyn[];
-        ChunkLoop loop(a0.next, MULTI ? 0 : a0.chunk_off[0],
+        ChunkLoop loop(a0.next, MULTI ? mchunk[0] : a0.chunk_off[0],
                        MULTI ? mchunk[nmol] : a0.chunk_off[a0.tiled ? a0.ntile : a0.bra.n * B2_NBUCKET]);
         if (!loop.block_has_work()) return;
         const R *tab = table_of<R>(a0) + RysLayout<R>::offset(K::NR);
@@ -1209,7 +1218,7 @@ __global__ void __launch_bounds__(128, (warp_min_blocks<LA, LB, LC, LD, R, GS_>(
         const unsigned gmask = GS == 32 ? 0xffffffffu : (((1u << GS) - 1u) << (grp * GS));
         const int wib = threadIdx.x >> 5;
         double *sm = smem_dyn + (size_t)(wib * NGRP + grp) * S::SIZE;
-        ChunkLoop loop(a0.next, MULTI ? 0 : a0.chunk_off[0],
+        ChunkLoop loop(a0.next, MULTI ? mchunk[0] : a0.chunk_off[0],
                        MULTI ? mchunk[nmol] : a0.chunk_off[a0.tiled ? a0.ntile : a0.bra.n * B2_NBUCKET]);
         if (!loop.block_has_work()) return;
         unsigned long long nq = 0, npq = 0;
