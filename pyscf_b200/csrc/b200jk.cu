@@ -347,18 +347,54 @@ struct FanLease {
 struct PairClassDev {
         int la = 0, lb = 0, n = 0;
         int boff[B2_NBUCKET + 1] = {0, 0, 0, 0, 0};
-        DevArr<int4> sh;
-        DevArr<int2> pr;
-        DevArr<double> q, qs;
-        DevArr<double4> A, AB;
+        // the class's arrays, in one allocation that later uploads reuse (six
+        // allocations and copies a class made up most of a small plan's set-up)
+        DevArr<unsigned char> mem;
+        int4 *sh = nullptr;
+        int2 *pr = nullptr;
+        double *q = nullptr, *qs = nullptr;
+        double4 *A = nullptr, *AB = nullptr;
         PairView view() const
         {
                 PairView v;
-                v.sh = sh.p; v.pr = pr.p; v.q = q.p; v.qs = qs.p; v.A = A.p; v.AB = AB.p; v.n = n;
+                v.sh = sh; v.pr = pr; v.q = q; v.qs = qs; v.A = A; v.AB = AB; v.n = n;
                 for (int b = 0; b <= B2_NBUCKET; b++) v.boff[b] = boff[b];
                 return v;
         }
-        void release() { sh.release(); pr.release(); q.release(); qs.release(); A.release(); AB.release(); n = 0; }
+        int upload(const std::vector<int4> &hsh, const std::vector<int2> &hpr, const std::vector<double> &hq,
+                   const std::vector<double> &hqs, const std::vector<double4> &hA, const std::vector<double4> &hAB)
+        {
+                const size_t m = hsh.size();
+                sh = nullptr; pr = nullptr; q = qs = nullptr; A = AB = nullptr;
+                if (m == 0) return B200JK_OK;
+                size_t off = 0;
+                auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
+                const size_t osh = take(sizeof(int4) * m), opr = take(sizeof(int2) * m), oq = take(sizeof(double) * m),
+                             oqs = take(sizeof(double) * m), oA = take(sizeof(double4) * m), oAB = take(sizeof(double4) * m);
+                std::vector<unsigned char> h(off);
+                memcpy(&h[osh], hsh.data(), sizeof(int4) * m);
+                memcpy(&h[opr], hpr.data(), sizeof(int2) * m);
+                memcpy(&h[oq], hq.data(), sizeof(double) * m);
+                memcpy(&h[oqs], hqs.data(), sizeof(double) * m);
+                memcpy(&h[oA], hA.data(), sizeof(double4) * m);
+                memcpy(&h[oAB], hAB.data(), sizeof(double4) * m);
+                int rc;
+                if ((rc = dev_alloc(mem, off))) return rc;
+                CUDA_TRY(cudaMemcpy(mem.p, h.data(), off, cudaMemcpyHostToDevice));
+                sh = (int4 *)(mem.p + osh);
+                pr = (int2 *)(mem.p + opr);
+                q = (double *)(mem.p + oq);
+                qs = (double *)(mem.p + oqs);
+                A = (double4 *)(mem.p + oA);
+                AB = (double4 *)(mem.p + oAB);
+                return B200JK_OK;
+        }
+        void release()
+        {
+                mem.release();
+                sh = nullptr; pr = nullptr; q = qs = nullptr; A = AB = nullptr;
+                n = 0;
+        }
 };
 
 // what the gradient set-up keeps of the planner's segments and pairs
@@ -379,8 +415,6 @@ struct GradPlan {
         double tol = 0;
         PairClassDev bra[NPAIRCLASS], ket[NPAIRCLASS];
         DevArr<double> q0;
-        DevArr<int2> goff;
-        std::vector<size_t> goff_at;   // [X * NPAIRCLASS + Y], then NPAIRCLASS^2 + X for q0
         std::vector<double> h_q0;
         DevArr<double> D, Dc, Ds, V, out, dmc, fac, de;
         DevArr<int> shell_atom;
@@ -399,7 +433,7 @@ struct GradPlan {
                 cls_ev.clear();
                 for (auto &c : bra) c.release();
                 for (auto &c : ket) c.release();
-                q0.release(); goff.release(); D.release(); Dc.release(); Ds.release(); V.release(); out.release();
+                q0.release(); D.release(); Dc.release(); Ds.release(); V.release(); out.release();
                 de.release(); shell_atom.release();
                 dmc.release(); fac.release(); dmax.release(); stats.release(); nkl.release(); kst.release();
                 nchunk.release(); chunk_off.release(); cub_tmp.release(); cdesc.release();
@@ -476,8 +510,6 @@ struct b200jk_plan {
         std::vector<PairLite> all_pairs[NPAIRCLASS];   // before screening
         GradPlan grad;
         DevArr<double> c2s, qcond, dm_cond;
-        DevArr<int> goff_all;
-        std::vector<size_t> goff_at;   // per quartet class
         DevArr<int4> seg_info;
         DevArr<int> out_seg, out_comp, cart_seg, cart_comp, ao_loc_d;
         // workspace; ws_gen counts the times its buffers moved
@@ -505,7 +537,7 @@ struct b200jk_plan {
                 for (auto &c : pc) c.release();
                 PP.release(); PK.release(); PE.release(); grad.release(); c2s.release();
                 pk_src.release(); Dpk.release(); Jpk.release(); qcond.release(); dm_cond.release();
-                goff_all.release(); seg_info.release(); out_seg.release(); out_comp.release();
+                seg_info.release(); out_seg.release(); out_comp.release();
                 cart_seg.release(); cart_comp.release(); ao_loc_d.release();
                 D.release(); Dc.release(); Ds.release(); Jacc.release(); Kacc.release(); outJ.release(); outK.release();
                 i1_pair.release(); i1_off.release(); i1_seg.release(); i1_atoms.release(); i1_seg_cart.release();
@@ -770,6 +802,117 @@ __global__ void fp64_fma_kernel(double *sink, int iters, double m)
         sink[(size_t)blockIdx.x * blockDim.x + threadIdx.x] = a0 + a1 + a2 + a3 + a4 + a5 + a6 + a7;
 }
 
+// Offset tables of every quartet class (packed 2D-integral offsets per
+// Cartesian component): the same for every plan, so they live beside the Rys
+// tables, filled once per device.  Built and uploaded per plan they took 1-2
+// ms of each plan_create, and the gradient's 14 ms of each geometry's first
+// gradient.
+static constexpr int pair_components(int X)
+{
+        constexpr int n[] = {1, 3, 9, 6, 18, 36, 10, 30, 60, 100};   // NA NB of 00, 10, 11, 20, ...
+        return n[X];
+}
+static constexpr int jk_goff_size()
+{
+        int s = 0;
+        for (int X = 0; X < NPAIRCLASS; X++)
+                for (int Y = 0; Y <= X; Y++) s += pair_components(X) * pair_components(Y);
+        return s;
+}
+static constexpr int grad_goff_size()
+{
+        int s = 0;
+        for (int X = 0; X < NPAIRCLASS; X++) {
+                for (int Y = 0; Y < NPAIRCLASS; Y++) s += pair_components(X) * pair_components(Y);
+                s += pair_components(X) * pair_components(X);
+        }
+        return s;
+}
+static __device__ int d_goff[jk_goff_size()];
+static __device__ int2 d_grad_goff[grad_goff_size()];
+
+// start of quartet class t (J/K), of (bra class, ket class) or, at
+// NPAIRCLASS^2 + X, of the derivative bound of class X (gradient)
+static const std::vector<size_t> &jk_goff_at()
+{
+        static const std::vector<size_t> at = [] {
+                std::vector<size_t> v;
+                size_t o = 0;
+                for (const QClass &c : quartet_classes()) {
+                        v.push_back(o);
+                        o += (size_t)pair_components(c.X) * pair_components(c.Y);
+                }
+                return v;
+        }();
+        return at;
+}
+static const std::vector<size_t> &grad_goff_at()
+{
+        static const std::vector<size_t> at = [] {
+                std::vector<size_t> v;
+                size_t o = 0;
+                for (int X = 0; X < NPAIRCLASS; X++)
+                        for (int Y = 0; Y < NPAIRCLASS; Y++) {
+                                v.push_back(o);
+                                o += (size_t)pair_components(X) * pair_components(Y);
+                        }
+                for (int X = 0; X < NPAIRCLASS; X++) {
+                        v.push_back(o);
+                        o += (size_t)pair_components(X) * pair_components(X);
+                }
+                return v;
+        }();
+        return at;
+}
+
+static void grad_goff(int la, int lb, int lc, int ld, int mode, std::vector<int2> &out);
+
+static std::mutex g_goff_mu;
+static bool g_goff_ready[64], g_grad_goff_ready[64];
+
+// (a failed upload is tried again by the next call)
+static int ensure_goff(int device, bool gradient)
+{
+        std::lock_guard<std::mutex> lk(g_goff_mu);
+        if (!gradient && !g_goff_ready[device]) {
+                std::vector<int> all;
+                for (const QClass &c : quartet_classes()) {
+                        int la, lb, lc, ld;
+                        class_l(c.X, la, lb);
+                        class_l(c.Y, lc, ld);
+                        class_goff(la, lb, lc, ld, all);
+                }
+                CUDA_TRY(cudaMemcpyToSymbol(d_goff, all.data(), sizeof(int) * all.size()));
+                g_goff_ready[device] = true;
+        }
+        if (gradient && !g_grad_goff_ready[device]) {
+                std::vector<int2> all;
+                for (int mode = 0; mode < 2; mode++)
+                        for (int X = 0; X < NPAIRCLASS; X++)
+                                for (int Y = mode ? X : 0; Y < (mode ? X + 1 : NPAIRCLASS); Y++) {
+                                        int la, lb, lc, ld;
+                                        class_l(X, la, lb);
+                                        class_l(Y, lc, ld);
+                                        grad_goff(la, lb, lc, ld, mode, all);
+                                }
+                CUDA_TRY(cudaMemcpyToSymbol(d_grad_goff, all.data(), sizeof(int2) * all.size()));
+                g_grad_goff_ready[device] = true;
+        }
+        return B200JK_OK;
+}
+static const int *goff_ptr(size_t t)
+{
+        void *p = nullptr;
+        cudaGetSymbolAddress(&p, d_goff);
+        return (const int *)p + jk_goff_at()[t];
+}
+static const int2 *grad_goff_ptr(size_t t)
+{
+        void *p = nullptr;
+        cudaGetSymbolAddress(&p, d_grad_goff);
+        return (const int2 *)p + grad_goff_at()[t];
+}
+
 static const double *table_ptr()
 {
         void *p = nullptr;
@@ -927,10 +1070,9 @@ int b200jk_plan_create(const int32_t *atm, int natm, const int32_t *bas, int nba
         }
         if (device < 0 || device >= ndev) return bail(fail(B200JK_EINVAL, "device index out of range"));
         if (cudaSetDevice(device) != cudaSuccess) return bail(fail(B200JK_ECUDA, "cudaSetDevice failed"));
-        if ((rc = ensure_tables(device))) return bail(rc);
-        cudaDeviceProp prop;
-        if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return bail(fail(B200JK_ECUDA, "cudaGetDeviceProperties failed"));
-        P->nsm = prop.multiProcessorCount;
+        if ((rc = ensure_tables(device)) || (rc = ensure_goff(device, false))) return bail(rc);
+        if (cudaDeviceGetAttribute(&P->nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+                return bail(fail(B200JK_ECUDA, "cudaDeviceGetAttribute failed"));
         if (cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreate(&P->ev0) != cudaSuccess || cudaEventCreate(&P->ev1) != cudaSuccess)
                 return bail(fail(B200JK_ECUDA, "stream/event creation failed"));
@@ -1005,21 +1147,6 @@ int b200jk_plan_create(const int32_t *atm, int natm, const int32_t *bas, int nba
                 for (const HostPair &h : pairs[X]) P->all_pairs[X].push_back({h.i, h.j, h.prim0, h.nprim});
         }
 
-        // Cartesian offset tables of all quartet classes (also used by q_cond)
-        {
-                std::vector<int> all;
-                auto qcs = quartet_classes();
-                P->goff_at.assign(qcs.size(), 0);
-                for (size_t t = 0; t < qcs.size(); t++) {
-                        int la, lb, lc, ld;
-                        class_l(qcs[t].X, la, lb);
-                        class_l(qcs[t].Y, lc, ld);
-                        P->goff_at[t] = all.size();
-                        class_goff(la, lb, lc, ld, all);
-                }
-                if ((rc = dev_upload(P->goff_all, all))) return bail(rc);
-        }
-
         // upload unsorted pairs, compute q_cond on the GPU
         auto upload_class = [&](int X, const std::vector<HostPair> &hv) -> int {
                 PairClassDev &c = P->pc[X];
@@ -1041,11 +1168,7 @@ int b200jk_plan_create(const int32_t *atm, int natm, const int32_t *bas, int nba
                         Av[t] = make_double4(A.R[0], A.R[1], A.R[2], hv[t].i == hv[t].j ? 1.0 : 0.0);
                         ABv[t] = make_double4(A.R[0] - B.R[0], A.R[1] - B.R[1], A.R[2] - B.R[2], 0.0);
                 }
-                int r;
-                if ((r = dev_upload(c.sh, sh)) || (r = dev_upload(c.pr, pr)) || (r = dev_upload(c.q, q)) ||
-                    (r = dev_upload(c.qs, qs)) || (r = dev_upload(c.A, Av)) || (r = dev_upload(c.AB, ABv)))
-                        return r;
-                return B200JK_OK;
+                return c.upload(sh, pr, q, qs, Av, ABv);
         };
         for (int X = 0; X < NPAIRCLASS; X++)
                 if ((rc = upload_class(X, pairs[X]))) return bail(rc);
@@ -1062,7 +1185,7 @@ int b200jk_plan_create(const int32_t *atm, int natm, const int32_t *bas, int nba
                         qa.table = table_ptr();
                         size_t gi = 0;
                         for (size_t t = 0; t < qcs.size(); t++) if (qcs[t].X == X && qcs[t].Y == X) gi = t;
-                        qa.goff = P->goff_all.p + P->goff_at[gi];
+                        qa.goff = goff_ptr(gi);
                         qa.c2s = P->c2s.p;
                         qa.qcond = (unsigned long long *)P->qcond.p;
                         qa.nbas = nbas;
@@ -1174,11 +1297,15 @@ int b200jk_plan_update_coords(b200jk_plan *P, const double *env, int env_len)
         std::swap(P->pk_off, T->pk_off);
         std::swap(P->pk_total, T->pk_total);
         std::swap(P->pk_src, T->pk_src);
-        std::swap(P->grad, T->grad);   // derivative bounds belong to the old geometry
+        P->grad.q0_ready = false;      // derivative bounds belong to the old geometry
+        P->grad.lists_ready = false;   // (the gradient's workspace stays)
+        P->grad.quartets = P->grad.prim_quartets = P->grad.launches = 0;
+        P->grad.last_ms = 0;
+        P->grad.cls.clear();
         std::swap(P->h_atoms, T->h_atoms);
         P->nuc_model_ok = T->nuc_model_ok;
         P->i1_npair = -1;              // the one-electron pair list is planned again on next use
-        P->release_fill();             // so are the integral fill's pair lists
+        P->fill_ready = false;         // so are the integral fill's pair lists
         P->shell_pairs = T->shell_pairs;
         P->prim_pairs = T->prim_pairs;
         P->st = T->st;
@@ -1587,7 +1714,7 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
                 a.dm_cond = P->dm_cond.p;
                 a.table = tbl;
                 a.table_f = tbl_f;
-                a.goff = P->goff_all.p + P->goff_at[t];
+                a.goff = goff_ptr(t);
                 a.Jacc = P->Jacc.p; a.Kacc = P->Kacc.p;
                 a.Ds = P->Ds.p; a.Dk = P->Dc.p;
                 a.Dpk = P->Dpk.p + P->pk_off[qcs[t].Y];
@@ -2063,11 +2190,7 @@ static int upload_pairs(const b200jk_plan *P, PairClassDev &c, int X, const std:
                 Av[t] = make_double4(A.R[0], A.R[1], A.R[2], hv[t].i == hv[t].j ? 1.0 : 0.0);
                 ABv[t] = make_double4(A.R[0] - B.R[0], A.R[1] - B.R[1], A.R[2] - B.R[2], 0.0);
         }
-        int r;
-        if ((r = dev_upload(c.sh, sh)) || (r = dev_upload(c.pr, pr)) || (r = dev_upload(c.q, q)) ||
-            (r = dev_upload(c.qs, q)) || (r = dev_upload(c.A, Av)) || (r = dev_upload(c.AB, ABv)))
-                return r;
-        return B200JK_OK;
+        return c.upload(sh, pr, q, q, Av, ABv);
 }
 
 // q0 (once per plan) and the gradient pair lists (per screening tolerance)
@@ -2078,46 +2201,29 @@ static int ensure_grad(b200jk_plan *P, double tol)
         const size_t n2 = (size_t)nbas * nbas;
         int rc;
         if (!g.q0_ready) {
-                std::vector<int2> all;
-                g.goff_at.assign(NPAIRCLASS * NPAIRCLASS + NPAIRCLASS, 0);
-                for (int X = 0; X < NPAIRCLASS; X++) {
-                        int la, lb;
-                        class_l(X, la, lb);
-                        for (int Y = 0; Y < NPAIRCLASS; Y++) {
-                                int lc, ld;
-                                class_l(Y, lc, ld);
-                                g.goff_at[X * NPAIRCLASS + Y] = all.size();
-                                grad_goff(la, lb, lc, ld, 0, all);
-                        }
-                }
-                for (int X = 0; X < NPAIRCLASS; X++) {
-                        int la, lb;
-                        class_l(X, la, lb);
-                        g.goff_at[NPAIRCLASS * NPAIRCLASS + X] = all.size();
-                        grad_goff(la, lb, la, lb, 1, all);
-                }
-                if ((rc = dev_upload(g.goff, all))) return rc;
+                if ((rc = ensure_goff(P->device, true))) return rc;
                 std::vector<double> init(n2, 1e-100);
                 if ((rc = dev_upload(g.q0, init))) return rc;
+                // (the pair lists of the bounds go where the ket lists go later)
                 for (int X = 0; X < NPAIRCLASS; X++) {
                         const std::vector<PairLite> &hv = P->all_pairs[X];
                         if (hv.empty()) continue;
-                        PairClassDev tmp;
-                        if ((rc = upload_pairs(P, tmp, X, hv, std::vector<double>(hv.size(), 0.0)))) return rc;
+                        if ((rc = upload_pairs(P, g.ket[X], X, hv, std::vector<double>(hv.size(), 0.0)))) return rc;
                         GradQArgs q;
                         q.omega2 = P->omega2;
-                        q.pairs = tmp.view();
+                        q.pairs = g.ket[X].view();
                         q.PP = P->PP.p; q.PK = P->PK.p; q.PE = P->PE.p;
                         q.table = table_ptr();
-                        q.goff = g.goff.p + g.goff_at[NPAIRCLASS * NPAIRCLASS + X];
+                        q.goff = grad_goff_ptr(NPAIRCLASS * NPAIRCLASS + X);
                         q.c2s = P->c2s.p;
                         q.q0 = (unsigned long long *)g.q0.p;
                         q.nbas = nbas;
                         q.cart = P->cart;
                         std::string err;
-                        if (g_gq0_launch[X](q, P->stream, err)) { tmp.release(); return fail(B200JK_ECUDA, err); }
+                        if (g_gq0_launch[X](q, P->stream, err)) return fail(B200JK_ECUDA, err);
+                }
+                {
                         const cudaError_t e = cudaStreamSynchronize(P->stream);
-                        tmp.release();
                         if (e != cudaSuccess) return fail(B200JK_ECUDA, std::string("gradient q_cond: ") + cudaGetErrorString(e));
                 }
                 g.h_q0.resize(n2);
@@ -2156,8 +2262,6 @@ static int ensure_grad(b200jk_plan *P, double tol)
                 };
                 order(hb, qb);
                 order(hk, qk);
-                g.bra[X].release();
-                g.ket[X].release();
                 if ((rc = upload_pairs(P, g.bra[X], X, hb, qb)) || (rc = upload_pairs(P, g.ket[X], X, hk, qk))) return rc;
         }
         g.tol = tol;
@@ -2309,7 +2413,7 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
                 a.q1 = P->qcond.p;
                 a.dmc = g.dmc.p;
                 a.table = table_ptr();
-                a.goff = g.goff.p + g.goff_at[t];
+                a.goff = grad_goff_ptr(t);
                 a.Vj = Vj; a.Vk = Vk;
                 a.Ds = g.Ds.p; a.Dc = g.Dc.p;
                 a.stats = g.stats.p + 2 * t;
@@ -2690,7 +2794,7 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                                         a.dm_cond = P->dm_cond.p;
                                         a.table = tbl;
                                         a.table_f = tbl_f;
-                                        a.goff = P->goff_all.p + P->goff_at[t];
+                                        a.goff = goff_ptr(t);
                                         a.Jacc = P->Jacc.p; a.Kacc = P->Kacc.p;
                                         a.Ds = P->Ds.p; a.Dk = P->Dc.p;
                                         a.Dpk = P->Dpk.p + P->pk_off[qcs[t].Y];
@@ -2959,7 +3063,7 @@ extern "C" int b200jk_get_jk_noalloc(b200jk_plan *P, const double *dms, int n_dm
                 a.kst = kst;
                 a.dm_cond = dmc;
                 a.table = tbl;
-                a.goff = P->goff_all.p + P->goff_at[t];
+                a.goff = goff_ptr(t);
                 a.Jacc = Jacc; a.Kacc = Kacc;
                 a.Ds = Ds; a.Dk = Dc;
                 a.stats = stats + 2 * t;
@@ -3030,7 +3134,6 @@ static int ensure_fill(b200jk_plan *P)
                 std::vector<PairLite> h2(hv.size());
                 std::vector<double> q2(hv.size());
                 for (size_t t = 0; t < idx.size(); t++) { h2[t] = hv[idx[t]]; q2[t] = q[idx[t]]; }
-                P->fill_pc[X].release();
                 if ((rc = upload_pairs(P, P->fill_pc[X], X, h2, q2))) return rc;
                 nseg += h2.size() * B2_NBUCKET * (X + 1);
         }
@@ -3140,7 +3243,7 @@ int b200jk_int2e_s8(b200jk_plan *P, double *eri, long long len, int dev_ptr, voi
                         a.max_chunk = p.max_chunk;
                         a.table = table_ptr();
                         a.table_f = table_f_ptr();
-                        a.goff = P->goff_all.p + P->goff_at[t];
+                        a.goff = goff_ptr(t);
                         a.tol = B2_FILL_CUTOFF;
                         a.nbas = P->nbas; a.naoc = P->naoc; a.same = p.d.same;
                         a.omega2 = P->omega2;
