@@ -22,7 +22,7 @@ CSRC = os.path.join(HERE, 'csrc')
 OBJ = os.path.join(HERE, '_build')
 LIB = os.path.join(HERE, 'libb200jk.so')
 HEADERS = ['rys_math.cuh', 'jk_kernels.cuh', 'jk_launch.h', 'rys_table.inc', 'rys_table_f.inc',
-           'grad_kernels.cuh', 'grad_launch.h', 'int1e_kernels.cuh', 'fill_kernels.cuh', 'fill_launch.h',
+           'jk_rows.cuh', 'grad_kernels.cuh', 'grad_launch.h', 'int1e_kernels.cuh', 'fill_kernels.cuh', 'fill_launch.h',
            'incore_launch.h']
 ARCH = ['-gencode', 'arch=compute_100a,code=sm_100a']
 PAIR_CLASSES = [(la, lb) for la in range(4) for lb in range(la + 1)]
@@ -56,12 +56,13 @@ def up_to_date(target=LIB):
 # headers each translation unit includes (directly or through another header)
 _RYS = ['rys_math.cuh', 'rys_table.inc', 'rys_table_f.inc']
 _JK = _RYS + ['jk_kernels.cuh', 'jk_launch.h']
+_JKC = _JK + ['jk_rows.cuh']
 _GRAD = _JK + ['grad_kernels.cuh', 'grad_launch.h']
 _FILL = _JK + ['fill_kernels.cuh', 'fill_launch.h']
 UNIT_DEPS = {
     'b200jk.cu': _GRAD + _FILL + ['int1e_kernels.cuh', 'incore_launch.h', '../../include/b200jk.h'],
     'jk_qcond.cu': _JK,
-    'jk_classes.cu': _JK,
+    'jk_classes.cu': _JKC,
     'grad_classes.cu': _GRAD,
     'fill_classes.cu': _FILL,
     'incore.cu': ['incore_launch.h'],

@@ -3,6 +3,7 @@
 // 55 classes of l <= 3 build in parallel.
 #include <mutex>
 #include "jk_launch.h"
+#include "jk_rows.cuh"
 
 #ifndef B2_KET_LD
 #error "compile with -DB2_BRA_LA -DB2_BRA_LB -DB2_KET_LC -DB2_KET_LD"
@@ -86,6 +87,44 @@ int launch_one(const JKArgs &a, const JKArgs *margs, const long long *mchunk, in
         return 0;
 }
 
+// row family (jk_rows.cuh)
+template <int LA, int LB, int LC, int LD, int CS, typename R, bool MULTI>
+int launch_row(const JKArgs &a, const JKArgs *margs, const long long *mchunk, int nmol, cudaStream_t s, int nsm,
+               std::string &err)
+{
+        static LaunchCfg cfg;
+        static std::mutex mu;
+        {
+                std::lock_guard<std::mutex> lk(mu);
+                if (!cfg.ready) {
+                        using S = RowSmem<LA, LB, LC, LD, CS, R>;
+                        int nb = 0;
+                        cfg.block = 32 * S::WPB;
+                        cfg.smem = sizeof(double) * (S::TABLE + (size_t)S::WPB * S::WARP);
+                        cfg.status = cudaFuncSetAttribute(jk_row_kernel<LA, LB, LC, LD, CS, R, MULTI>,
+                                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.smem);
+                        if (cfg.status == cudaSuccess)
+                                cfg.status = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                                        &nb, jk_row_kernel<LA, LB, LC, LD, CS, R, MULTI>, cfg.block, cfg.smem);
+                        cfg.grid = (nb > 0 ? nb : 1) * nsm;
+                        cfg.ready = true;
+                }
+        }
+        if (cfg.status != cudaSuccess) {
+                err = std::string("kernel configuration: ") + cudaGetErrorString(cfg.status);
+                return 1;
+        }
+        // (the kernel's blocks start one per chunk, not per block of warps)
+        jk_row_kernel<LA, LB, LC, LD, CS, R, MULTI><<<grid_of(cfg.grid, 32, a.max_chunk), cfg.block, cfg.smem, s>>>(
+                a, family_chunk(LA, LB, LC, LD), margs, mchunk, nmol);
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) {
+                err = std::string("kernel launch: ") + cudaGetErrorString(e);
+                return 1;
+        }
+        return 0;
+}
+
 // variant 2 of the register family: bra runs of BR pairs (float64 pass,
 // tiled chunk order, one symmetric density; the host checks these)
 template <int LA, int LB, int LC, int LD, int BR>
@@ -129,6 +168,14 @@ int B2_FN_NAME(const JKArgs &a, cudaStream_t s, int nsm, int fp32, int variant, 
                const long long *mchunk, int nmol, std::string &err)
 {
         constexpr int NP = thread_parts<B2_BRA_LA, B2_BRA_LB, B2_KET_LC, B2_KET_LD>();
+        // the row family has one width: variants 0 and 1 are the same launch
+        constexpr int CS = NP > 0 ? 0 : row_split<B2_BRA_LA, B2_BRA_LB, B2_KET_LC, B2_KET_LD>();
+        if constexpr (CS > 0) {
+#define B2_LR(R, M) launch_row<B2_BRA_LA, B2_BRA_LB, B2_KET_LC, B2_KET_LD, CS, R, M>(a, margs, mchunk, nmol, s, nsm, err)
+                if (nmol > 0) return fp32 ? B2_LR(float, true) : B2_LR(double, true);
+                return fp32 ? B2_LR(float, false) : B2_LR(double, false);
+#undef B2_LR
+        } else {
         constexpr int KRUN = NP > 0 ? ket_run<B2_BRA_LA, B2_BRA_LB, B2_KET_LC, B2_KET_LD, NP>() : 1;
         // the shared-memory family's variant 1: half as many lanes per quartet
         // (only where one warp's groups still fit the 200 KB a block may use here)
@@ -163,6 +210,7 @@ int B2_FN_NAME(const JKArgs &a, cudaStream_t s, int nsm, int fp32, int variant, 
         if (nmol > 0) return fp32 ? B2_L(float, true, 1) : B2_L(double, true, 1);
         return fp32 ? B2_L(float, false, 1) : B2_L(double, false, 1);
 #undef B2_L
+        }
 }
 
 // B2_NP_NAME is launch_jk_<la><lb><lc><ld>_np: the parts of the register

@@ -6,6 +6,10 @@
 #include <string>
 #include "jk_kernels.cuh"
 
+// accumulators a lane of the row family may keep (jk_rows.cuh): 72 doubles, 144
+// of the 255 registers a thread has there
+#define B2_ROW_ACC 72
+
 namespace b200jk {
 
 // parts of the register family of class (la lb | lc ld) as its translation
@@ -69,12 +73,24 @@ inline bool family_has_variant_n(int la, int lb, int lc, int ld, int v)
         if (v == 2) return family_bra_run(la, lb, lc, ld) > 1;
         return false;
 }
+// lane groups per warp of the row family (host twin of row_split<> and
+// RowSmem<>::NGRP in jk_rows.cuh); 0 where the class has no row kernel
+inline int family_row_groups(int la, int lb, int lc, int ld)
+{
+        if (family_thread_parts(la, lb, lc, ld) > 0) return 0;
+        const int na = ncart(la), nb = ncart(lb), nc = ncart(lc), nd = ncart(ld);
+        for (int cs = 1; cs <= nc; cs++)
+                if (nc % cs == 0 && na * cs <= 32 && nb * (nc / cs) * nd <= B2_ROW_ACC) return 32 / (na * cs);
+        return 0;
+}
 // quartets per chunk: 32 x kets per lane in the register family (variant 0:
 // one ket per lane, 1: family_ket_run), 8 per group of the warp otherwise
 inline int family_chunk(int la, int lb, int lc, int ld, int variant = 0)
 {
         if (family_thread_parts(la, lb, lc, ld) > 0)
                 return 32 * (variant == 1 ? family_ket_run(la, lb, lc, ld) : 1);   // bra runs: 32 kets too
+        // row family: a multiple of its 3, 5 or 10 groups that one warp screens at once
+        if (const int ng = family_row_groups(la, lb, lc, ld)) return ng >= 3 ? 30 : 8 * ng;
         const int gs = family_group(la, lb, lc, ld);
         return 8 * (32 / (variant == 1 && family_half_groups(la, lb, lc, ld) ? gs / 2 : gs));   // 8 quartets per group
 }

@@ -302,6 +302,29 @@ B2_HD void rys_root_one(R T, const R *__restrict__ tab, int r, R &u, R &w)
         w = rys_poly<R>(c + (NR + r) * L::ROW, x);
 }
 
+// rys_root_one from a staged slice
+template <int NR, typename R>
+B2_HD void rys_root_one_staged(R T, const R *__restrict__ tab, int r, R &u, R &w)
+{
+        using L = RysLayout<R>;
+        using S = RysStaged<NR, R>;
+        if (!(T < (R)L::t_asym(NR))) {
+                const R it = (R)1 / T;
+                double x2 = rys_herm_x2(NR * (NR - 1) / 2), wh = rys_herm_w(NR * (NR - 1) / 2);
+#pragma unroll
+                for (int i = 1; i < NR; i++)
+                        if (r == i) { x2 = rys_herm_x2(NR * (NR - 1) / 2 + i); wh = rys_herm_w(NR * (NR - 1) / 2 + i); }
+                u = (R)x2 * it;
+                w = (R)wh * b2sqrt(it);
+                return;
+        }
+        const int p = (int)T;
+        const R x = (R)2 * (T - (R)p) - (R)1;
+        const R *c = tab + p * S::PIECE;
+        u = rys_poly_staged<R>(c + r * S::ROW, x);
+        w = rys_poly_staged<R>(c + (NR + r) * S::ROW, x);
+}
+
 // 2D vertical recurrence: g[e*NF + f], e < NE, f < NF.
 template <int NE, int NF, typename R>
 B2_HD void vrr2d(R *g, R g00, R c00, R c00p, R b10, R b01, R b00)

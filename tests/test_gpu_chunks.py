@@ -154,3 +154,38 @@ def test_long_contractions_fill(b2, nprims, l_of, nctr):
     rj, rk, _ = oracle.get_jk(d, atm, bas, env, hermi=1, screen=False)
     assert abs(numpy.einsum('ijkl,ji->kl', full, d) - rj).max() < TOL
     assert abs(numpy.einsum('ijkl,jk->il', full, d) - rk).max() < TOL
+
+
+@pytest.mark.parametrize('nprims,l_of,ncopy', [
+    ((1, 2, 3), (2, 1, 0), 5),      # (21|20), (21|11), (22|10): 5 groups of 6 lanes, 10 of 3
+    ((1, 2), (3, 1), 4),            # (31|11), (31|31): 3 groups of 10 lanes
+    ((1, 1, 2), (3, 2, 1), 2),      # (32|21), (32|11), (33|10): shares of the third index
+])
+@pytest.mark.parametrize('omega', [0.0, 0.4])
+def test_row_family(b2, nprims, l_of, ncopy, omega):
+    """The row family's classes on a chain whose distant kets fail the screen
+    (survivors are compacted, the last round of groups is partly empty): one
+    symmetric density, two general ones, J or K alone, the long-range operator,
+    and every quartet in float32 (2e-5 of the largest element: the bound the
+    float32 kernels are held to elsewhere)."""
+    atm, bas, env = contracted_molecule(nprims, l_of, ncopy=ncopy)
+    env[8] = omega
+    for a in atm:
+        env[a[1]] *= 3.0
+        env[a[1] + 1] *= 2.5
+    plan = b2.Plan(atm, bas, env, direct_scf_tol=1e-13)
+    d = densities(plan.nao, 2)
+    ds = d[0] + d[0].T
+    rj, rk, _ = oracle.get_jk(ds, atm, bas, env, hermi=1)
+    tol = TOL * max(1.0, abs(rj).max(), abs(rk).max())
+    vj, vk = plan.get_jk(ds, hermi=1)
+    assert abs(vj - rj).max() < tol and abs(vk - rk).max() < tol
+    assert abs(plan.get_jk(ds, hermi=1, with_k=False)[0] - rj).max() < tol
+    assert abs(plan.get_jk(ds, hermi=1, with_j=False)[1] - rk).max() < tol
+    plan.set_mixed_threshold(1e30)
+    fj, fk = plan.get_jk(ds, hermi=1, precision=b2.PREC_MIXED)
+    assert abs(fj - rj).max() < 2e-5 * abs(rj).max() and abs(fk - rk).max() < 2e-5 * abs(rk).max()
+    vj, vk = plan.get_jk(d, hermi=0)
+    for s in range(2):
+        rj, rk, _ = oracle.get_jk(d[s], atm, bas, env, hermi=0)
+        assert abs(vj[s] - rj).max() < tol and abs(vk[s] - rk).max() < tol
