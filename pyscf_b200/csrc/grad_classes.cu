@@ -139,7 +139,7 @@ int launch_gq0_one(const GradQArgs &q, cudaStream_t s, std::string &err)
         {
                 std::lock_guard<std::mutex> lk(mu);
                 if (!cfg.ready) {
-                        cfg.smem = sizeof(double) * S::SIZE;
+                        cfg.smem = sizeof(double) * S::SIZE * grad_q0_warps<LA, LB>();
                         cfg.status = cfg.smem > SMEM_MAX ? cudaErrorInvalidConfiguration
                                                          : cudaFuncSetAttribute(grad_q0_kernel<LA, LB>,
                                                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -152,7 +152,8 @@ int launch_gq0_one(const GradQArgs &q, cudaStream_t s, std::string &err)
                 return 1;
         }
         if (q.pairs.n == 0) return 0;
-        grad_q0_kernel<LA, LB><<<q.pairs.n, 32, cfg.smem, s>>>(q);
+        constexpr int W = grad_q0_warps<LA, LB>();
+        grad_q0_kernel<LA, LB><<<(q.pairs.n + W - 1) / W, 32 * W, cfg.smem, s>>>(q);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
                 err = std::string("gradient q_cond launch: ") + cudaGetErrorString(e);

@@ -845,17 +845,24 @@ struct GradQArgs {
         int nbas, cart;
 };
 
+// warps of a block, as qcond_warps
 template <int LA, int LB>
-__global__ void __launch_bounds__(32) grad_q0_kernel(GradQArgs q)
+__host__ __device__ constexpr int grad_q0_warps()
+{
+        constexpr int fit = 100 * 1024 / (8 * GradSmem<LA, LB, LA, LB, 1>::SIZE);
+        return fit < 1 ? 1 : (fit > 8 ? 8 : fit);
+}
+
+template <int LA, int LB>
+__global__ void __launch_bounds__((32 * grad_q0_warps<LA, LB>())) grad_q0_kernel(GradQArgs q)
 {
         using K = Class4<LA, LB, LA, LB>;
         using GC = GClass<LA, LB, LA, LB, 1>;
         using S = GradSmem<LA, LB, LA, LB, 1>;
+        constexpr int W = grad_q0_warps<LA, LB>();
         extern __shared__ __align__(32) double smem_dyn[];
-        double *sm = smem_dyn;
-        const int lane = threadIdx.x & 31;
-        const int ij = blockIdx.x;
-        if (ij >= q.pairs.n) return;
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        double *sm = smem_dyn + w * S::SIZE;
         GradArgs a;
         a.PP = q.PP;
         a.PK = q.PK;
@@ -863,17 +870,17 @@ __global__ void __launch_bounds__(32) grad_q0_kernel(GradQArgs q)
         a.table = q.table;
         a.goff = q.goff;
         a.omega2 = q.omega2;
-        const int4 sh = q.pairs.sh[ij];
-        const int2 pr = q.pairs.pr[ij];
-        const double4 Av = q.pairs.A[ij];
-        const double4 ABv = q.pairs.AB[ij];
-        const double AB[3] = {ABv.x, ABv.y, ABv.z}, C0[3] = {0.0, 0.0, 0.0};
         const int nsa = q.cart ? K::NA : 2 * LA + 1, nsb = q.cart ? K::NB : 2 * LB + 1;
         const double *ca = q.c2s + LA * 100, *cb = q.c2s + LB * 100;
-        double mA = 0.0, mB = 0.0;
-        for (int pass = 0; pass < GC::NPASS; pass++) {
-                const int c0 = pass * GC::NCP;
-                grad_eval_pass<LA, LB, LA, LB, 1, 32>(sm, a, pr, pr, Av, AB, C0, AB, 1.0, c0, lane, 0xffffffffu, 0, 1);
+        // share sub of nsub of the derivative components from c0 of pair ij
+        auto evaluate = [&](int ij, int2 pr, int c0, int sub, int nsub) {
+                const double4 Av = q.pairs.A[ij];
+                const double4 ABv = q.pairs.AB[ij];
+                const double AB[3] = {ABv.x, ABv.y, ABv.z}, C0[3] = {0.0, 0.0, 0.0};
+                grad_eval_pass<LA, LB, LA, LB, 1, 32>(sm, a, pr, pr, Av, AB, C0, AB, 1.0, c0, lane, 0xffffffffu, sub, nsub);
+        };
+        // one warp: the largest diagonal element per side of its components
+        auto fold = [&](int c0, double &mA, double &mB) {
                 const double *G = sm + S::G;
                 for (int cc = 0; cc < GC::NCP; cc++) {
                         const int side = (c0 + cc) / 3;
@@ -905,17 +912,52 @@ __global__ void __launch_bounds__(32) grad_q0_kernel(GradQArgs q)
                         else mB = fmax(mB, m);
                 }
                 __syncwarp();
-        }
+        };
+        auto finish = [&](int ij, double mA, double mB) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-                mA = fmax(mA, __shfl_xor_sync(0xffffffffu, mA, o));
-                mB = fmax(mB, __shfl_xor_sync(0xffffffffu, mB, o));
+                for (int o = 16; o > 0; o >>= 1) {
+                        mA = fmax(mA, __shfl_xor_sync(0xffffffffu, mA, o));
+                        mB = fmax(mB, __shfl_xor_sync(0xffffffffu, mB, o));
+                }
+                if (lane == 0) {
+                        const int4 sh = q.pairs.sh[ij];
+                        const unsigned long long bA = (unsigned long long)__double_as_longlong(sqrt(fmax(mA, 1e-100)));
+                        const unsigned long long bB = (unsigned long long)__double_as_longlong(sqrt(fmax(mB, 1e-100)));
+                        atomicMax(q.q0 + (size_t)sh.z * q.nbas + sh.w, bA);
+                        atomicMax(q.q0 + (size_t)sh.w * q.nbas + sh.z, bB);
+                }
+        };
+        // a pair per warp, then the pairs of long contractions shared by all
+        const int ij0 = blockIdx.x * W;
+        auto shared_pair = [&](int2 pr) { return W > 1 && pr.y * pr.y > 64; };
+        if (ij0 + w < q.pairs.n) {
+                const int2 pr = q.pairs.pr[ij0 + w];
+                if (!shared_pair(pr)) {
+                        double mA = 0.0, mB = 0.0;
+                        for (int c0 = 0; c0 < 6; c0 += GC::NCP) {
+                                evaluate(ij0 + w, pr, c0, 0, 1);
+                                fold(c0, mA, mB);
+                        }
+                        finish(ij0 + w, mA, mB);
+                }
         }
-        if (lane == 0) {
-                const unsigned long long bA = (unsigned long long)__double_as_longlong(sqrt(fmax(mA, 1e-100)));
-                const unsigned long long bB = (unsigned long long)__double_as_longlong(sqrt(fmax(mB, 1e-100)));
-                atomicMax(q.q0 + (size_t)sh.z * q.nbas + sh.w, bA);
-                atomicMax(q.q0 + (size_t)sh.w * q.nbas + sh.z, bB);
+        for (int i = 0; i < W && ij0 + i < q.pairs.n; i++) {   // (uniform over the block)
+                const int2 pr = q.pairs.pr[ij0 + i];
+                if (!shared_pair(pr)) continue;
+                double mA = 0.0, mB = 0.0;
+                for (int c0 = 0; c0 < 6; c0 += GC::NCP) {
+                        __syncthreads();
+                        evaluate(ij0 + i, pr, c0, w, W);
+                        __syncthreads();
+                        for (int t = threadIdx.x; t < GC::NCP * GC::NG; t += blockDim.x) {
+                                double v = 0.0;
+                                for (int k = 0; k < W; k++) v += smem_dyn[k * S::SIZE + S::G + t];
+                                smem_dyn[S::G + t] = v;
+                        }
+                        __syncthreads();
+                        if (w == 0) fold(c0, mA, mB);
+                }
+                if (w == 0) finish(ij0 + i, mA, mB);
         }
 }
 

@@ -1387,6 +1387,9 @@ __global__ void __launch_bounds__(128, (warp_min_blocks<LA, LB, LC, LD, R, GS_>(
 // Schwarz conditioner: one warp per shell pair evaluates (ij|ij), transforms
 // the diagonal to the output basis and folds sqrt(max |(ab|ab)|) into the
 // parent-shell entry (CVHFnr_int2e_q_cond, pyscf/lib/vhf/optimizer.c:408-454).
+// The warps of a block take a pair each; pairs of long contractions (an
+// 8-primitive shell with itself has 4096 primitive quartets, 1.5 ms on one
+// warp) are then shared by all of them.
 struct QArgs {
         double omega2;               // as JKArgs::omega2
         PairView pairs;
@@ -1399,63 +1402,100 @@ struct QArgs {
         int nbas, cart;
 };
 
+// warps of a block: 8 where 100 KB of shared memory admit them
 template <int LA, int LB>
-__global__ void __launch_bounds__(32) qcond_kernel(QArgs q)
+__host__ __device__ constexpr int qcond_warps()
+{
+        constexpr int fit = 100 * 1024 / (8 * WarpSmem<LA, LB, LA, LB, double>::SIZE);
+        return fit < 1 ? 1 : (fit > 8 ? 8 : fit);
+}
+
+template <int LA, int LB>
+__global__ void __launch_bounds__((32 * qcond_warps<LA, LB>())) qcond_kernel(QArgs q)
 {
         using K = Class4<LA, LB, LA, LB>;
         using S = WarpSmem<LA, LB, LA, LB, double>;
+        constexpr int W = qcond_warps<LA, LB>();
         extern __shared__ __align__(32) double smem_dyn[];
-        double *sm = smem_dyn;
-        const int lane = threadIdx.x & 31;
-        const int ij = blockIdx.x;
-        if (ij >= q.pairs.n) return;
+        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+        double *sm = smem_dyn + w * S::SIZE;
         JKArgs a;
         a.PP = q.PP;
         a.PK = q.PK;
         a.table = q.table;
         a.goff = q.goff;
         a.omega2 = q.omega2;
-        const int4 sh = q.pairs.sh[ij];
-        const int2 pr = q.pairs.pr[ij];
-        const double4 Av = q.pairs.A[ij];
-        const double4 ABv = q.pairs.AB[ij];
-        const double A[3] = {0.0, 0.0, 0.0}, AB[3] = {ABv.x, ABv.y, ABv.z};
         int goff_r[group_goff_regs<LA, LB, LA, LB, 32, double>()];
         group_load_goff<LA, LB, LA, LB, 32, double>(q.goff, lane, goff_r);
-        group_eval_block<LA, LB, LA, LB, 32, double>(sm, a, pr, pr, Av, A, AB, A, AB, 1.0, lane, 0xffffffffu, goff_r);
-        const double *G = sm + S::G;
         const int nsa = q.cart ? K::NA : 2 * LA + 1, nsb = q.cart ? K::NB : 2 * LB + 1;
         const double *ca = q.c2s + LA * 100, *cb = q.c2s + LB * 100;
-        double m = 0.0;
-        for (int t = lane; t < nsa * nsb; t += 32) {
-                const int mi = t / nsb, ni = t % nsb;
-                double v = 0.0;
-                for (int x = 0; x < K::NA; x++) {
-                        const double c1 = ca[mi * 10 + x];
-                        if (c1 == 0.0) continue;
-                        for (int y = 0; y < K::NB; y++) {
-                                const double c2 = cb[ni * 10 + y];
-                                if (c2 == 0.0) continue;
-                                for (int x2 = 0; x2 < K::NA; x2++) {
-                                        const double c3 = ca[mi * 10 + x2];
-                                        if (c3 == 0.0) continue;
-                                        for (int y2 = 0; y2 < K::NB; y2++) {
-                                                const double c4 = cb[ni * 10 + y2];
-                                                if (c4 == 0.0) continue;
-                                                v += c1 * c2 * c3 * c4 * G[((x * K::NB + y) * K::NA + x2) * K::NB + y2];
+        // share w of nsub of the block of pair ij
+        auto evaluate = [&](int ij, int2 pr, int sub, int nsub) {
+                const double4 Av = q.pairs.A[ij];
+                const double4 ABv = q.pairs.AB[ij];
+                const double A[3] = {0.0, 0.0, 0.0}, AB[3] = {ABv.x, ABv.y, ABv.z};
+                group_eval_block<LA, LB, LA, LB, 32, double>(sm, a, pr, pr, Av, A, AB, A, AB, 1.0, lane, 0xffffffffu, goff_r,
+                                                             sub, nsub);
+        };
+        // one warp: the bound from its block
+        auto finish = [&](int ij) {
+                const int4 sh = q.pairs.sh[ij];
+                const double *G = sm + S::G;
+                double m = 0.0;
+                for (int t = lane; t < nsa * nsb; t += 32) {
+                        const int mi = t / nsb, ni = t % nsb;
+                        double v = 0.0;
+                        for (int x = 0; x < K::NA; x++) {
+                                const double c1 = ca[mi * 10 + x];
+                                if (c1 == 0.0) continue;
+                                for (int y = 0; y < K::NB; y++) {
+                                        const double c2 = cb[ni * 10 + y];
+                                        if (c2 == 0.0) continue;
+                                        for (int x2 = 0; x2 < K::NA; x2++) {
+                                                const double c3 = ca[mi * 10 + x2];
+                                                if (c3 == 0.0) continue;
+                                                for (int y2 = 0; y2 < K::NB; y2++) {
+                                                        const double c4 = cb[ni * 10 + y2];
+                                                        if (c4 == 0.0) continue;
+                                                        v += c1 * c2 * c3 * c4 * G[((x * K::NB + y) * K::NA + x2) * K::NB + y2];
+                                                }
                                         }
                                 }
                         }
+                        m = fmax(m, fabs(v));
                 }
-                m = fmax(m, fabs(v));
-        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (lane == 0) {
-                const double qv = sqrt(fmax(m, 1e-100));
-                const unsigned long long bits = (unsigned long long)__double_as_longlong(qv);
-                atomicMax(q.qcond + (size_t)sh.z * q.nbas + sh.w, bits);
-                atomicMax(q.qcond + (size_t)sh.w * q.nbas + sh.z, bits);
+                for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+                if (lane == 0) {
+                        const double qv = sqrt(fmax(m, 1e-100));
+                        const unsigned long long bits = (unsigned long long)__double_as_longlong(qv);
+                        atomicMax(q.qcond + (size_t)sh.z * q.nbas + sh.w, bits);
+                        atomicMax(q.qcond + (size_t)sh.w * q.nbas + sh.z, bits);
+                }
+                __syncwarp();
+        };
+        const int ij0 = blockIdx.x * W;
+        auto shared_pair = [&](int2 pr) { return W > 1 && pr.y * pr.y > 64; };
+        if (ij0 + w < q.pairs.n) {
+                const int2 pr = q.pairs.pr[ij0 + w];
+                if (!shared_pair(pr)) {
+                        evaluate(ij0 + w, pr, 0, 1);
+                        finish(ij0 + w);
+                }
+        }
+        for (int i = 0; i < W && ij0 + i < q.pairs.n; i++) {   // (uniform over the block)
+                const int2 pr = q.pairs.pr[ij0 + i];
+                if (!shared_pair(pr)) continue;
+                __syncthreads();
+                evaluate(ij0 + i, pr, w, W);
+                __syncthreads();
+                for (int t = threadIdx.x; t < K::NG; t += blockDim.x) {
+                        double v = 0.0;
+                        for (int k = 0; k < W; k++) v += smem_dyn[k * S::SIZE + S::G + t];
+                        smem_dyn[S::G + t] = v;
+                }
+                __syncthreads();
+                if (w == 0) finish(ij0 + i);
         }
 }
 

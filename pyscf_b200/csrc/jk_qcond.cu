@@ -6,10 +6,11 @@ namespace b200jk {
 template <int LA, int LB>
 static int launch_q(const QArgs &q, cudaStream_t s, std::string &err)
 {
-        const size_t smem = sizeof(double) * WarpSmem<LA, LB, LA, LB>::SIZE;
+        constexpr int W = qcond_warps<LA, LB>();
+        const size_t smem = sizeof(double) * WarpSmem<LA, LB, LA, LB>::SIZE * W;
         cudaError_t e = cudaFuncSetAttribute(qcond_kernel<LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess && q.pairs.n > 0) {
-                qcond_kernel<LA, LB><<<q.pairs.n, 32, smem, s>>>(q);
+                qcond_kernel<LA, LB><<<(q.pairs.n + W - 1) / W, 32 * W, smem, s>>>(q);
                 e = cudaGetLastError();
         }
         if (e != cudaSuccess) {
