@@ -371,6 +371,117 @@ __device__ __forceinline__ void grad_eval_force(double *sm, const GradArgs &a, i
         __syncwarp(gmask);
 }
 
+// All six derivative blocks of one quartet into G, for the classes that hold
+// them at once (GC::NCP == 6).  Each lane assembles the six derivatives of its
+// components together: they share the undifferentiated 2D integrals and the
+// offsets, which grad_eval_pass, a derivative component at a time with
+// run-time direction and side, reloads for each (and addresses through local
+// memory).  Where a lane's share fits registers (at most 48 sums) the blocks
+// are written once, else the first primitive quartet stores and later ones
+// add.
+template <int LA, int LB, int LC, int LD, int GS>
+__device__ __forceinline__ void grad_eval_all(double *sm, const GradArgs &a, int2 pb, int2 pk, const double4 O,
+                                              const double AB[3], const double C[3], const double CD[3], double fac,
+                                              int gl, unsigned gmask, int sub, int nsub)
+{
+        using GC = GClass<LA, LB, LC, LD, 0>;
+        using S = GradSmem<LA, LB, LC, LD, 0>;
+        constexpr int NR = GC::NR, SE = GC::SE, NG = GC::NG;
+        constexpr int SA = GC::STEP_A, SB = GC::STEP_B;
+        constexpr int NT = (NG + GS - 1) / GS;
+        constexpr bool REGS = 6 * NT <= 48;
+        double *G = sm + S::G;
+        double *E = sm + S::E;
+        const double *table = a.table + rys_padded_offset(NR);
+        const double A[3] = {0.0, 0.0, 0.0};
+        double acc[REGS ? 6 * NT : 1];
+        if constexpr (REGS) {
+#pragma unroll
+                for (int t = 0; t < 6 * NT; t++) acc[t] = 0.0;
+        }
+        bool first = true;
+        for (int ip = 0, kp = sub; ip < pb.y; ip++, kp -= pk.y) {
+                if (kp >= pk.y) continue;
+                const double4 P = a.PP[pb.x + ip];
+                const double2 KP = a.PK[pb.x + ip];
+                const double2 EP = a.PE[pb.x + ip];
+                const double Kab = KP.x * fac;
+                const double Pv[3] = {P.x - O.x, P.y - O.y, P.z - O.z};
+                const double ta = 2.0 * EP.x, tb = 2.0 * EP.y;
+                for (; kp < pk.y; kp += nsub) {
+                        const double4 Q = a.PP[pk.x + kp];
+                        const double2 KQ = a.PK[pk.x + kp];
+                        const double Qv[3] = {Q.x - O.x, Q.y - O.y, Q.z - O.z};
+                        __syncwarp(gmask);
+                        for (int task = gl; task < 3 * NR; task += GS) {
+                                const int r = task / 3, dir = task - 3 * r;
+                                PrimQ<double> sq;
+                                prim_setup<double>(sq, P.w, KP.y, Pv, Q.w, KQ.y, Qv, A, C, Kab * KQ.x, a.omega2);
+                                double ur, wr;
+                                rys_root_one<NR, double>(sq.T, table, r, ur, wr);
+                                RysCoef<double> rc;
+                                rys_coef<double>(rc, ur, sq);
+                                const double g00 = dir == 2 ? sq.pref * wr : 1.0;
+                                const double abx = dir == 0 ? AB[0] : (dir == 1 ? AB[1] : AB[2]);
+                                const double cdx = dir == 0 ? CD[0] : (dir == 1 ? CD[1] : CD[2]);
+                                grad_slice<LA, LB, LC, LD, 0>(E + (dir * NR + r) * SE, g00, rc, dir, abx, cdx);
+                        }
+                        __syncwarp(gmask);
+                        auto component = [&](int t, double f[6]) {
+                                const int2 o = __ldg(a.goff + t);
+                                const int ox = o.x & 1023, oy = (o.x >> 10) & 1023, oz = o.x >> 20;
+                                const int axn = gexp(o.y, 0, 0), ayn = gexp(o.y, 0, 1), azn = gexp(o.y, 0, 2);
+                                const int bxn = gexp(o.y, 1, 0), byn = gexp(o.y, 1, 1), bzn = gexp(o.y, 1, 2);
+#pragma unroll
+                                for (int r = 0; r < NR; r++) {
+                                        const double *Ex = E + r * SE, *Ey = E + (NR + r) * SE, *Ez = E + (2 * NR + r) * SE;
+                                        const double ex = Ex[ox], ey = Ey[oy], ez = Ez[oz];
+                                        double dax = ta * Ex[ox + SA], day = ta * Ey[oy + SA], daz = ta * Ez[oz + SA];
+                                        if (axn) dax -= axn * Ex[ox - SA];
+                                        if (ayn) day -= ayn * Ey[oy - SA];
+                                        if (azn) daz -= azn * Ez[oz - SA];
+                                        double dbx = tb * Ex[ox + SB], dby = tb * Ey[oy + SB], dbz = tb * Ez[oz + SB];
+                                        if (bxn) dbx -= bxn * Ex[ox - SB];
+                                        if (byn) dby -= byn * Ey[oy - SB];
+                                        if (bzn) dbz -= bzn * Ez[oz - SB];
+                                        const double eyz = ey * ez, exz = ex * ez, exy = ex * ey;
+                                        f[0] += dax * eyz;
+                                        f[1] += day * exz;
+                                        f[2] += daz * exy;
+                                        f[3] += dbx * eyz;
+                                        f[4] += dby * exz;
+                                        f[5] += dbz * exy;
+                                }
+                        };
+                        if constexpr (REGS) {
+#pragma unroll
+                                for (int i = 0; i < NT; i++)
+                                        if (NG % GS == 0 || gl + i * GS < NG) component(gl + i * GS, acc + 6 * i);
+                        } else {
+                                for (int t = gl; t < NG; t += GS) {
+                                        double f[6];
+#pragma unroll
+                                        for (int q = 0; q < 6; q++) f[q] = first ? 0.0 : G[q * NG + t];
+                                        component(t, f);
+#pragma unroll
+                                        for (int q = 0; q < 6; q++) G[q * NG + t] = f[q];
+                                }
+                        }
+                        first = false;
+                }
+        }
+        if constexpr (REGS) {
+#pragma unroll
+                for (int i = 0; i < NT; i++)
+                        if (NG % GS == 0 || gl + i * GS < NG)
+#pragma unroll
+                                for (int q = 0; q < 6; q++) G[q * NG + gl + i * GS] = acc[6 * i + q];
+        } else if (first) {   // fewer primitive quartets than nsub: an empty share
+                for (int t = gl; t < 6 * NG; t += GS) G[t] = 0.0;
+        }
+        __syncwarp(gmask);
+}
+
 template <int LA, int LB, int LC, int LD>
 __host__ __device__ constexpr int grad_group_size()
 {
@@ -473,7 +584,10 @@ __global__ void __launch_bounds__(128) grad_jk_kernel(GradArgs a, int chunk_q)
                                 // skip a pass whose components all belong to a failing side
                                 const bool needA = sideA && c0 < 3, needB = sideB && c0 + GC::NCP > 3;
                                 if (!needA && !needB) continue;
-                                grad_eval_pass<LA, LB, LC, LD, 0, GS>(sm, a, pb, pk, Ab, AB, C, CD, fac, c0, gl, gmask, sub, nsub);
+                                if constexpr (GC::NCP == 6)
+                                        grad_eval_all<LA, LB, LC, LD, GS>(sm, a, pb, pk, Ab, AB, C, CD, fac, gl, gmask, sub, nsub);
+                                else
+                                        grad_eval_pass<LA, LB, LC, LD, 0, GS>(sm, a, pb, pk, Ab, AB, C, CD, fac, c0, gl, gmask, sub, nsub);
                                 const double *G = sm + S::G;
                                 for (int s = 0; s < a.n_dm; s++) {
                                         const double *Ds = a.Ds + s * nn;
