@@ -2315,7 +2315,9 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
                         d.bra = bra.view();
                         d.ket = ket.view();
                         d.chunk = grad_chunk(bra.la, bra.lb, ket.la, ket.lb, fused);
-                        d.split = split_level(bra, ket, 0, grad_register_family(bra.la, bra.lb, ket.la, ket.lb, fused), P->nsm);
+                        const bool reg = grad_register_family(bra.la, bra.lb, ket.la, ket.lb, fused);
+                        d.split = split_level(bra, ket, 0, reg, P->nsm);
+                        if (!reg && d.split == 1) d.split = 3;
                         d.most = d.chunk == 32 ? 5 : (d.chunk == 16 ? 4 : 3);
                         d.seg0 = d.scan0 = nseg_all;
                         p.max_chunk = 0;
@@ -3191,6 +3193,7 @@ int b200jk_int2e_s8(b200jk_plan *P, double *eri, long long len, int dev_ptr, voi
                         d.same = qcs[t].X == qcs[t].Y;
                         d.chunk = fill_chunk(bra.la, bra.lb, ket.la, ket.lb);
                         d.split = split_level(bra, ket, d.same, false, P->nsm);
+                        if (d.split == 1) d.split = 3;
                         d.most = d.chunk == 32 ? 5 : (d.chunk == 16 ? 4 : 3);
                         d.seg0 = d.scan0 = nseg;
                         p.max_chunk = 0;

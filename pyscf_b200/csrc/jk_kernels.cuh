@@ -170,7 +170,10 @@ __device__ __forceinline__ bool quartet_passes(const JKArgs &a, int4 sb, double 
 // the expected primitive quartets of the two buckets: at level 1 only where a
 // lane would run hundreds of them (the contraction, done by one lane of the
 // 2^s, stays below a tenth of the work); at level 2, for classes with too few
-// quartets to occupy every lane, wherever there is more than one.
+// quartets to occupy every lane, wherever there is more than one.  Level 3 is level 1
+// of the gradient's and the fill's group families: a group takes 8 quartets of
+// a chunk one after the other, so the first three halvings only shorten its
+// row, and are made from a few dozen primitive quartets in the row on.
 __host__ __device__ inline int split_log2(int level, int bra_bucket, int ket_bucket)
 {
         if (level == 0) return 0;
@@ -178,6 +181,7 @@ __host__ __device__ inline int split_log2(int level, int bra_bucket, int ket_buc
         const int l2[B2_NBUCKET] = {0, 2, 3, 5};
         const int e = l2[bra_bucket] + l2[ket_bucket];
         if (level == 1) return e >= 10 ? 5 : (e >= 8 ? 3 : 0);
+        if (level == 3) return e >= 10 ? 5 : (e >= 8 ? 4 : (e >= 5 ? 3 : e / 2));
         return e >= 5 ? 5 : e;
 }
 
