@@ -371,16 +371,20 @@ struct PairClassDev {
                 auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
                 const size_t osh = take(sizeof(int4) * m), opr = take(sizeof(int2) * m), oq = take(sizeof(double) * m),
                              oqs = take(sizeof(double) * m), oA = take(sizeof(double4) * m), oAB = take(sizeof(double4) * m);
-                std::vector<unsigned char> h(off);
-                memcpy(&h[osh], hsh.data(), sizeof(int4) * m);
-                memcpy(&h[opr], hpr.data(), sizeof(int2) * m);
-                memcpy(&h[oq], hq.data(), sizeof(double) * m);
-                memcpy(&h[oqs], hqs.data(), sizeof(double) * m);
-                memcpy(&h[oA], hA.data(), sizeof(double4) * m);
-                memcpy(&h[oAB], hAB.data(), sizeof(double4) * m);
                 int rc;
                 if ((rc = dev_alloc(mem, off))) return rc;
-                CUDA_TRY(cudaMemcpy(mem.p, h.data(), off, cudaMemcpyHostToDevice));
+                const struct { size_t at, bytes; const void *src; } part[] = {
+                        {osh, sizeof(int4) * m, hsh.data()}, {opr, sizeof(int2) * m, hpr.data()},
+                        {oq, sizeof(double) * m, hq.data()}, {oqs, sizeof(double) * m, hqs.data()},
+                        {oA, sizeof(double4) * m, hA.data()}, {oAB, sizeof(double4) * m, hAB.data()}};
+                if (off <= 256 * 1024) {
+                        // small: gathered on the host, one copy
+                        std::vector<unsigned char> h(off);
+                        for (const auto &c : part) memcpy(&h[c.at], c.src, c.bytes);
+                        CUDA_TRY(cudaMemcpy(mem.p, h.data(), off, cudaMemcpyHostToDevice));
+                } else {
+                        for (const auto &c : part) CUDA_TRY(cudaMemcpy(mem.p + c.at, c.src, c.bytes, cudaMemcpyHostToDevice));
+                }
                 sh = (int4 *)(mem.p + osh);
                 pr = (int2 *)(mem.p + opr);
                 q = (double *)(mem.p + oq);
@@ -518,7 +522,8 @@ struct b200jk_plan {
         DevArr<double> D, Dc, Ds, Jacc, Kacc, outJ, outK;
         DevArr<unsigned long long> dmax, stats;
         // segments of all classes and passes of a build, counted in one launch
-        DevArr<int> nkl, kst;
+        // (nkl: their lengths, then their starts)
+        DevArr<int> nkl;
         DevArr<long long> nchunk, chunk_off;
         DevArr<unsigned char> cub_tmp;
         DevArr<CountDesc> cdesc;
@@ -544,7 +549,7 @@ struct b200jk_plan {
                 i1_seg_atom.release(); i1_de.release();
                 i1_S.release(); i1_H.release(); i1_zero.release(); i1_out.release();
                 release_fill();
-                dmax.release(); stats.release(); nkl.release(); kst.release(); nchunk.release(); chunk_off.release(); cub_tmp.release();
+                dmax.release(); stats.release(); nkl.release(); nchunk.release(); chunk_off.release(); cub_tmp.release();
                 cdesc.release();
                 if (counted) g_fans[device].plan_removed();
                 for (auto e : cls_ev) cudaEventDestroy(e);
@@ -579,7 +584,9 @@ typedef int (*jk_launcher_t)(const JKArgs &, cudaStream_t, int, int, int, const 
 // Launch variant of a float64 pass in a plan the autotuner has not timed:
 // the autotuner's choices on the FP64 build of (H2O)64/cc-pVTZ, where each
 // won by 15-25% per class -- bra runs (2) for eight register-family
-// classes of s and p kets, half-width groups (1) for (21|20) and (22|10).
+// classes of s and p kets, and 1 for (21|20) and (22|10), which chose half-width
+// groups before the row family took them (there 0 and 1 are the same launch).
+// Of (H2O)27/cc-pVTZ the defaults take 946 ms, variant 0 everywhere 975 ms.
 // Callers that never tune (a drop-in SCF, whose first builds would pay for
 // the timing) get them on plans of DEFAULT_VARIANT_MIN_NAO or more AOs.
 // Smaller plans keep variant 0: bra runs give a warp four bra pairs, too
@@ -1574,8 +1581,8 @@ static int ensure_count(b200jk_plan *P, const std::vector<ClassPass> &passes, lo
 {
         int rc;
         if (nscan + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one build");
-        if ((rc = dev_alloc(P->nkl, (size_t)std::max(1ll, nseg))) || (rc = dev_alloc(P->kst, (size_t)std::max(1ll, nseg))) ||
-            (rc = dev_alloc(P->nchunk, (size_t)nscan + 1)) || (rc = dev_alloc(P->chunk_off, (size_t)nscan + 1)))
+        // (lengths, then starts)
+        if ((rc = dev_alloc(P->nkl, 2 * (size_t)std::max(1ll, nseg))) || (rc = dev_alloc(P->nchunk, (size_t)nscan + 1)) || (rc = dev_alloc(P->chunk_off, (size_t)nscan + 1)))
                 return rc;
         size_t tmp = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, tmp, P->nchunk.p, P->chunk_off.p, (int)(nscan + 1));
@@ -1683,7 +1690,7 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
                 CUDA_TRY(cudaMemsetAsync(P->nchunk.p, 0, sizeof(long long) * (nscan + 1), s));
                 count_all_kernel<<<grid_for(nseg, 256), 256, 0, s>>>(
                         P->cdesc.p, (int)passes.size(), nseg, P->tol > 0 ? P->tol : 0.0, (const double *)P->dmax.p,
-                        P->shard, P->nshard, P->nkl.p, P->kst.p, (unsigned long long *)P->nchunk.p);
+                        P->shard, P->nshard, P->nkl.p, P->nkl.p + nseg, (unsigned long long *)P->nchunk.p);
                 CUDA_TRY(cudaGetLastError());
                 size_t tmp = P->cub_tmp.n;
                 CUDA_TRY(cub::DeviceScan::ExclusiveSum(P->cub_tmp.p, tmp, P->nchunk.p, P->chunk_off.p, (int)(nscan + 1), s));
@@ -1710,7 +1717,7 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
                 a.PP = P->PP.p; a.PK = P->PK.p;
                 a.chunk_off = P->chunk_off.p + c.d.scan0;
                 a.nkl = P->nkl.p + c.d.seg0;
-                a.kst = P->kst.p + c.d.seg0;
+                a.kst = P->nkl.p + nseg + c.d.seg0;
                 a.dm_cond = P->dm_cond.p;
                 a.table = tbl;
                 a.table_f = tbl_f;
