@@ -217,7 +217,8 @@ int b200jk_set_profiling(b200jk_plan *plan, int on);
 
 /* Autotuner: for every quartet class with more than one launch variant (the
  * register family with one or several kets per lane, or bra runs; the shared-memory
- * family with full- or half-width lane groups per quartet), time each variant
+ * family with full- or half-width lane groups per quartet; classes of the row
+ * family run the same launch as 0 and 1), time each variant
  * on FP64 J/K builds of the density dm (nao x nao, symmetric; host array, or
  * device array with dev_ptrs = 1), then the float32 pass's variants on mixed
  * builds at the plan's threshold, and keep the faster for later builds of
@@ -236,7 +237,8 @@ int b200jk_set_tile(b200jk_plan *plan, int tile_b);
  * of mixed builds (B200JK_PREC_MIXED).  Before any tuning: 0 everywhere on
  * plans of fewer than 1500 AOs; from 1500 AOs on, the float64 pass uses the
  * autotuner's measured choices on a large cc-pVTZ workload (bra runs for
- * eight classes of s and p kets, half-width groups for (21|20) and (22|10)). */
+ * eight classes of s and p kets; 1 for (21|20) and (22|10), row-family classes
+ * since, where it is the same launch as 0). */
 int b200jk_get_tuning(const b200jk_plan *plan, int precision, int *variants, int max, int *n);
 
 /* Set the variants directly (n = 55; 0 everywhere, 1 or 2 only where the

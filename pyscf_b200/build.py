@@ -112,9 +112,7 @@ THREAD_PARTS = {
 # blocks per SM of the shared-memory family's float64 kernels where the
 # build overrides warp_min_blocks<> (jk_kernels.cuh: 4 where the groups'
 # shared memory admits 4 blocks, else 0); B2_WARP_MINB="la lb lc ld:n,..."
-# in the environment replaces it.  Empty: without the cap of 4 (128
-# registers) the tuned half-width (21|20) and (22|10) kernels took 852 and
-# 359 ms instead of 720 and 327 ms on the FP64 build of (H2O)64/cc-pVTZ.
+# in the environment replaces it.
 WARP_MINB = {}
 
 
@@ -191,6 +189,13 @@ def _source_of(cmd):
     raise ValueError(cmd)
 
 
+def _weight(obj):
+    """Rough compile time of a unit: gradient, fill and class units by the
+    angular momenta in their names."""
+    l = sum(int(c) for c in obj if c.isdigit())
+    return {'grad': 1000, 'fill': 100, 'b200': 500}.get(obj[:4], 0) + l
+
+
 def build(force=False, verbose=False, extra=(), jobs=None):
     # every unit is checked against its own sources (an object compiled while
     # its source was being edited is older than the edit even when the library
@@ -199,7 +204,8 @@ def build(force=False, verbose=False, extra=(), jobs=None):
     units = _units()
     if extra:
         units = [(cmd[:-3] + list(extra) + cmd[-3:] if cmd[0] != 'g++' else cmd, o) for cmd, o in units]
-    # rebuild only the units whose sources, headers or flags changed
+    # rebuild only the units whose sources, headers or flags changed, the
+    # longest first (the f classes' gradient kernels take many minutes each)
     todo = []
     for cmd, o in units:
         flags_file = o + '.cmd'
@@ -207,6 +213,7 @@ def build(force=False, verbose=False, extra=(), jobs=None):
         same_flags = os.path.exists(flags_file) and open(flags_file).read() == line
         if force or not same_flags or _stale(o, _source_of(cmd), flags_file):
             todo.append((cmd, o))
+    todo.sort(key=lambda u: -_weight(os.path.basename(u[1])))
 
     def run(u):
         cmd, o = u

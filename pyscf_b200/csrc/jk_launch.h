@@ -45,7 +45,8 @@ inline int family_group_smem(int la, int lb, int lc, int ld)
         return (x + 3) & ~3;
 }
 // half-width groups (variant 1 of the shared-memory family: 32 -> 16 or
-// 16 -> 8 lanes) where one warp's groups fit the 200 KB a block may use
+// 16 -> 8 lanes) where one warp's groups fit the 200 KB a block may use; the
+// row family's classes keep the variant they had there, as the same launch
 inline bool family_half_groups(int la, int lb, int lc, int ld)
 {
         const int gs = family_group(la, lb, lc, ld);

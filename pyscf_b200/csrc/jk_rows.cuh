@@ -18,8 +18,7 @@
 //
 // Measured on the FP64 build of (H2O)16/cc-pVTZ against groups with the block
 // in shared memory: (21|20) 25.6 -> 13.2 ms, (21|11) 17.1 -> 7.9, (21|21) 13.4 ->
-// 5.8, (31|21) 10.7 -> 4.3, (22|21) 10.3 -> 5.7, (32|22) 4.5 -> 1.4, all classes
-// 344 -> 232 ms.  What bounds it now is latency at 8-12 warps per SM: the chain
+// 5.8, (31|21) 10.7 -> 4.3, (22|21) 10.3 -> 5.7, (32|22) 4.5 -> 1.4 ms.  What bounds it now is latency at 8-12 warps per SM: the chain
 // of one primitive quartet (division, root polynomial, recurrence, two passes
 // through shared memory) and the loads of its data.
 //
@@ -36,9 +35,6 @@ template <int LA, int LB, int LC, int LD>
 __host__ __device__ constexpr int row_split()
 {
         using K = Class4<LA, LB, LC, LD>;
-#if defined(B2_ROW_CS) && defined(B2_KET_LD)
-        if (LA == B2_BRA_LA && LB == B2_BRA_LB && LC == B2_KET_LC && LD == B2_KET_LD) return B2_ROW_CS;
-#endif
         for (int cs = 1; cs <= K::NC; cs++)
                 if (K::NC % cs == 0 && K::NA * cs <= 32 && K::NB * (K::NC / cs) * K::ND <= B2_ROW_ACC) return cs;
         return 0;
