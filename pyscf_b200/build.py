@@ -90,8 +90,17 @@ def _stale(obj, src, flags_file):
 # B2_THREAD_MINB=<n> (every class) or "la lb lc ld:n,..." in the environment
 # overrides it.
 THREAD_MINB = {
-    (1, 0, 0, 0): 4, (1, 1, 0, 0): 4, (2, 0, 0, 0): 4, (2, 1, 0, 0): 4,
+    (1, 0, 0, 0): 6, (1, 1, 0, 0): 4, (2, 0, 0, 0): 5, (2, 1, 0, 0): 4,
+    (2, 0, 1, 0): 4, (1, 1, 1, 0): 3, (3, 0, 0, 0): 5,
     (3, 0, 1, 0): 3, (2, 2, 0, 0): 3, (3, 1, 0, 0): 3,
+}
+# with the table staged free of bank conflicts latency is what is left, and
+# more warps pay in five classes ((H2O)16/cc-pVTZ: (10|00) 14.1 -> 12.6 ms at 6
+# blocks, (11|10) 8.8 -> 7.5 at 3, (20|10) 12.9 -> 12.2 at 4, (20|00) 8.5 -> 7.9
+# at 5, (30|00) 2.4 -> 2.3 at 5); their bra-run kernels keep the bounds they
+# were tuned with.
+RUN_MINB = {
+    (1, 0, 0, 0): 4, (2, 0, 0, 0): 4, (2, 0, 1, 0): 0, (1, 1, 1, 0): 0, (3, 0, 0, 0): 0,
 }
 
 
@@ -163,6 +172,8 @@ def _units():
                                 '-DB2_THREAD_MINB=%d' % _thread_minb((la, lb, lc, ld))] +
                      (['-DB2_THREAD_PARTS=%d' % _thread_parts((la, lb, lc, ld))]
                       if _thread_parts((la, lb, lc, ld)) else []) +
+                     (['-DB2_RUN_MINB=%d' % RUN_MINB[(la, lb, lc, ld)]]
+                      if (la, lb, lc, ld) in RUN_MINB else []) +
                      (['-DB2_WARP_MINB=%d' % _warp_minb((la, lb, lc, ld))]
                       if _warp_minb((la, lb, lc, ld)) is not None else []) +
                      [os.path.join(CSRC, 'jk_classes.cu'), '-o', o], o))

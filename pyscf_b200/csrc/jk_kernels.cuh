@@ -7,10 +7,11 @@
 //     q_ij q_kl max(4 D_ji, 4 D_lk, D_jk, D_jl, D_ik, D_il) > tol
 // (CVHFnrs8_prescreen, pyscf/lib/vhf/optimizer.c:90-117) form a prefix of the
 // sorted ket list, so the work of a class is  sum_ij nkl(ij)  quartets; it is
-// cut into chunks (32 quartets for the thread-per-quartet family, 8 for the
-// warp-per-quartet family) and a grid-stride loop of warps walks the chunks
-// (warp -> chunk -> bra pair by binary search of the chunk prefix sum).  The
-// exact per-quartet test is then applied with the parent-shell density bound.
+// cut into chunks (32 quartets for the thread-per-quartet family, about 30 for
+// the row family of jk_rows.cuh, 8 per lane group for the warp-per-quartet
+// family) which the warps draw from a queue (chunk -> bra pair by binary search
+// of the chunk prefix sum).  The exact per-quartet test is then applied with
+// the parent-shell density bound.
 //
 // Arithmetic.  Integrals are Cartesian; the density enters in the Cartesian
 // AO basis D_c = C^T D C and the results leave as C J_c C^T (C the block
@@ -464,6 +465,10 @@ __host__ __device__ constexpr int ket_run()
 #ifndef B2_THREAD_MINB
 #define B2_THREAD_MINB 0
 #endif
+// the same for the bra-run kernels
+#ifndef B2_RUN_MINB
+#define B2_RUN_MINB B2_THREAD_MINB
+#endif
 
 template <int LA, int LB, int LC, int LD, int NP, typename R, bool MULTI, int KR>
 __global__ void __launch_bounds__(128, (sizeof(R) == 8 ? B2_THREAD_MINB : 0)) jk_thread_kernel(JKArgs a0, const JKArgs *__restrict__ margs,
@@ -762,7 +767,7 @@ __host__ __device__ constexpr int bra_run()
 // those images.  K[b,c], K[b,d] still take one atomic per quartet and J[a,b]
 // one per bra pair and warp.
 template <int LA, int LB, int LC, int LD, int BR>
-__global__ void __launch_bounds__(128, B2_THREAD_MINB) jk_thread_run_kernel(JKArgs a)
+__global__ void __launch_bounds__(128, B2_RUN_MINB) jk_thread_run_kernel(JKArgs a)
 {
         using K = Class4<LA, LB, LC, LD>;
         constexpr int NG = K::NG;
