@@ -179,8 +179,14 @@ struct DevArr {
         void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
 };
 
+// Host arrays travel on the stream of the kernels that read them.  (A plain
+// cudaMemcpy from pageable memory may return before the data is on the device,
+// and it runs on the legacy stream, which the non-blocking streams of this
+// file do not wait for: a kernel launched next could read the allocation's
+// earlier contents.)  The source is staged before the call returns.  Tables
+// that other streams read later are followed by a wait in their set-up.
 template <typename T>
-static int dev_upload(DevArr<T> &d, const std::vector<T> &h)
+static int dev_upload(DevArr<T> &d, const std::vector<T> &h, cudaStream_t s)
 {
         d.release();
         d.n = h.size();
@@ -189,7 +195,7 @@ static int dev_upload(DevArr<T> &d, const std::vector<T> &h)
                 d.p = nullptr;
                 return fail(B200JK_ENOMEM, "cudaMalloc failed for a plan table");
         }
-        CUDA_TRY(cudaMemcpy(d.p, h.data(), sizeof(T) * d.n, cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpyAsync(d.p, h.data(), sizeof(T) * d.n, cudaMemcpyHostToDevice, s));
         return B200JK_OK;
 }
 
@@ -362,7 +368,8 @@ struct PairClassDev {
                 return v;
         }
         int upload(const std::vector<int4> &hsh, const std::vector<int2> &hpr, const std::vector<double> &hq,
-                   const std::vector<double> &hqs, const std::vector<double4> &hA, const std::vector<double4> &hAB)
+                   const std::vector<double> &hqs, const std::vector<double4> &hA, const std::vector<double4> &hAB,
+                   cudaStream_t s)
         {
                 const size_t m = hsh.size();
                 sh = nullptr; pr = nullptr; q = qs = nullptr; A = AB = nullptr;
@@ -381,9 +388,10 @@ struct PairClassDev {
                         // small: gathered on the host, one copy
                         std::vector<unsigned char> h(off);
                         for (const auto &c : part) memcpy(&h[c.at], c.src, c.bytes);
-                        CUDA_TRY(cudaMemcpy(mem.p, h.data(), off, cudaMemcpyHostToDevice));
+                        CUDA_TRY(cudaMemcpyAsync(mem.p, h.data(), off, cudaMemcpyHostToDevice, s));
                 } else {
-                        for (const auto &c : part) CUDA_TRY(cudaMemcpy(mem.p + c.at, c.src, c.bytes, cudaMemcpyHostToDevice));
+                        for (const auto &c : part)
+                                CUDA_TRY(cudaMemcpyAsync(mem.p + c.at, c.src, c.bytes, cudaMemcpyHostToDevice, s));
                 }
                 sh = (int4 *)(mem.p + osh);
                 pr = (int2 *)(mem.p + opr);
@@ -788,7 +796,8 @@ static int ensure_tables(int device)
                 rys_pad_table(rys_table_data, padded.data());
                 g_table_status[device] =
                         (cudaMemcpyToSymbol(d_rys_table, padded.data(), sizeof(double) * padded.size()) == cudaSuccess &&
-                         cudaMemcpyToSymbol(d_rys_table_f, rys_table_f_data, sizeof(float) * RYS_F_SIZE) == cudaSuccess)
+                         cudaMemcpyToSymbol(d_rys_table_f, rys_table_f_data, sizeof(float) * RYS_F_SIZE) == cudaSuccess &&
+                         cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess)
                                 ? 0 : 1;
         });
         if (g_table_status[device]) return fail(B200JK_ECUDA, "could not upload the Rys tables");
@@ -890,6 +899,7 @@ static int ensure_goff(int device, bool gradient)
                         class_goff(la, lb, lc, ld, all);
                 }
                 CUDA_TRY(cudaMemcpyToSymbol(d_goff, all.data(), sizeof(int) * all.size()));
+                CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
                 g_goff_ready[device] = true;
         }
         if (gradient && !g_grad_goff_ready[device]) {
@@ -903,6 +913,7 @@ static int ensure_goff(int device, bool gradient)
                                         grad_goff(la, lb, lc, ld, mode, all);
                                 }
                 CUDA_TRY(cudaMemcpyToSymbol(d_grad_goff, all.data(), sizeof(int2) * all.size()));
+                CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
                 g_grad_goff_ready[device] = true;
         }
         return B200JK_OK;
@@ -1096,10 +1107,12 @@ int b200jk_plan_create(const int32_t *atm, int natm, const int32_t *bas, int nba
                 for (int k = 0; k < nf; k++) { out_seg[g.out_off + k] = (int)s; out_comp[g.out_off + k] = k; }
                 for (int k = 0; k < ncart(g.l); k++) { cart_seg[g.cart_off + k] = (int)s; cart_comp[g.cart_off + k] = k; }
         }
-        if ((rc = dev_upload(P->seg_info, seg_info)) || (rc = dev_upload(P->out_seg, out_seg)) ||
-            (rc = dev_upload(P->out_comp, out_comp)) || (rc = dev_upload(P->cart_seg, cart_seg)) ||
-            (rc = dev_upload(P->cart_comp, cart_comp)) || (rc = dev_upload(P->ao_loc_d, P->ao_loc)) ||
-            (rc = dev_upload(P->c2s, build_c2s(P->cart))))
+        // (every table of the plan is uploaded on its stream, and waited for at the end)
+        cudaStream_t s = P->stream;
+        if ((rc = dev_upload(P->seg_info, seg_info, s)) || (rc = dev_upload(P->out_seg, out_seg, s)) ||
+            (rc = dev_upload(P->out_comp, out_comp, s)) || (rc = dev_upload(P->cart_seg, cart_seg, s)) ||
+            (rc = dev_upload(P->cart_comp, cart_comp, s)) || (rc = dev_upload(P->ao_loc_d, P->ao_loc, s)) ||
+            (rc = dev_upload(P->c2s, build_c2s(P->cart), s)))
                 return bail(rc);
 
         // shell pairs and primitive pairs
@@ -1139,7 +1152,7 @@ int b200jk_plan_create(const int32_t *atm, int natm, const int32_t *bas, int nba
                 }
         }
         P->prim_pairs = (int64_t)hPP.size();
-        if ((rc = dev_upload(P->PP, hPP)) || (rc = dev_upload(P->PK, hPK)) || (rc = dev_upload(P->PE, hPE)))
+        if ((rc = dev_upload(P->PP, hPP, s)) || (rc = dev_upload(P->PK, hPK, s)) || (rc = dev_upload(P->PE, hPE, s)))
                 return bail(rc);
         // the gradient set-up re-screens the unpruned pairs with its own bounds
         P->segl.resize(segs.size());
@@ -1175,13 +1188,13 @@ int b200jk_plan_create(const int32_t *atm, int natm, const int32_t *bas, int nba
                         Av[t] = make_double4(A.R[0], A.R[1], A.R[2], hv[t].i == hv[t].j ? 1.0 : 0.0);
                         ABv[t] = make_double4(A.R[0] - B.R[0], A.R[1] - B.R[1], A.R[2] - B.R[2], 0.0);
                 }
-                return c.upload(sh, pr, q, qs, Av, ABv);
+                return c.upload(sh, pr, q, qs, Av, ABv, s);
         };
         for (int X = 0; X < NPAIRCLASS; X++)
                 if ((rc = upload_class(X, pairs[X]))) return bail(rc);
 
         std::vector<double> h_q((size_t)nbas * nbas, 1e-100);
-        if ((rc = dev_upload(P->qcond, h_q))) return bail(rc);
+        if ((rc = dev_upload(P->qcond, h_q, s))) return bail(rc);
         {
                 auto qcs = quartet_classes();
                 for (int X = 0; X < NPAIRCLASS; X++) {
@@ -1199,10 +1212,10 @@ int b200jk_plan_create(const int32_t *atm, int natm, const int32_t *bas, int nba
                         qa.cart = P->cart;
                         {
                                 std::string err;
-                                if (launch_qcond(P->pc[X].la, P->pc[X].lb, qa, P->stream, err)) return bail(fail(B200JK_ECUDA, err));
+                                if (launch_qcond(P->pc[X].la, P->pc[X].lb, qa, s, err)) return bail(fail(B200JK_ECUDA, err));
                         }
                 }
-                if (cudaStreamSynchronize(P->stream) != cudaSuccess)
+                if (cudaStreamSynchronize(s) != cudaSuccess)
                         return bail(fail(B200JK_ECUDA, std::string("q_cond kernels: ") + cudaGetErrorString(cudaGetLastError())));
                 if (cudaMemcpy(h_q.data(), P->qcond.p, sizeof(double) * h_q.size(), cudaMemcpyDeviceToHost) != cudaSuccess)
                         return bail(fail(B200JK_ECUDA, "q_cond download failed"));
@@ -1266,8 +1279,11 @@ int b200jk_plan_create(const int32_t *atm, int natm, const int32_t *bas, int nba
                 }
                 P->pk_off[NPAIRCLASS] = (long long)src.size();
                 P->pk_total = (long long)src.size();
-                if ((rc = dev_upload(P->pk_src, src))) return bail(rc);
+                if ((rc = dev_upload(P->pk_src, src, s))) return bail(rc);
         }
+        // builds may run on any stream
+        if (cudaStreamSynchronize(s) != cudaSuccess)
+                return bail(fail(B200JK_ECUDA, std::string("plan tables: ") + cudaGetErrorString(cudaGetLastError())));
         memset(&P->st, 0, sizeof(P->st));
         P->st.nao = P->nao; P->st.nao_cart = P->naoc; P->st.nbas = nbas; P->st.nseg = P->nseg;
         P->st.shell_pairs = P->shell_pairs; P->st.prim_pairs = P->prim_pairs;
@@ -1343,13 +1359,15 @@ static int ensure_i1(b200jk_plan *P)
                 hc[t] = P->segl[t].cart_off;
                 ha[t] = P->shell_atom[P->segl[t].parent];
         }
-        if ((rc = dev_upload(P->i1_pair, hp)) || (rc = dev_upload(P->i1_off, off)) || (rc = dev_upload(P->i1_seg, hs)) ||
-            (rc = dev_upload(P->i1_seg_cart, hc)) || (rc = dev_upload(P->i1_seg_atom, ha)) ||
-            (rc = dev_upload(P->i1_atoms, P->h_atoms)) ||
+        cudaStream_t s = P->stream;
+        if ((rc = dev_upload(P->i1_pair, hp, s)) || (rc = dev_upload(P->i1_off, off, s)) ||
+            (rc = dev_upload(P->i1_seg, hs, s)) || (rc = dev_upload(P->i1_seg_cart, hc, s)) ||
+            (rc = dev_upload(P->i1_seg_atom, ha, s)) || (rc = dev_upload(P->i1_atoms, P->h_atoms, s)) ||
             (rc = dev_alloc(P->i1_S, nc)) || (rc = dev_alloc(P->i1_H, nc)) || (rc = dev_alloc(P->i1_zero, nc)) ||
             (rc = dev_alloc(P->i1_out, 2 * nn)))
                 return rc;
-        CUDA_TRY(cudaMemset(P->i1_zero.p, 0, sizeof(double) * nc));
+        CUDA_TRY(cudaMemsetAsync(P->i1_zero.p, 0, sizeof(double) * nc, s));
+        CUDA_TRY(cudaStreamSynchronize(s));   // the integrals may run on any stream
         P->i1_npair = (int)hp.size();
         return B200JK_OK;
 }
@@ -2178,7 +2196,7 @@ static const gq0_launcher_t g_gq0_launch[NPAIRCLASS] = {
         launch_gq0_00, launch_gq0_10, launch_gq0_11, launch_gq0_20, launch_gq0_21,
         launch_gq0_22, launch_gq0_30, launch_gq0_31, launch_gq0_32, launch_gq0_33};
 
-// upload one class of pairs in the given order, q per pair
+// upload one class of pairs in the given order, q per pair, on the plan's stream
 static int upload_pairs(const b200jk_plan *P, PairClassDev &c, int X, const std::vector<PairLite> &hv,
                         const std::vector<double> &q)
 {
@@ -2197,7 +2215,7 @@ static int upload_pairs(const b200jk_plan *P, PairClassDev &c, int X, const std:
                 Av[t] = make_double4(A.R[0], A.R[1], A.R[2], hv[t].i == hv[t].j ? 1.0 : 0.0);
                 ABv[t] = make_double4(A.R[0] - B.R[0], A.R[1] - B.R[1], A.R[2] - B.R[2], 0.0);
         }
-        return c.upload(sh, pr, q, q, Av, ABv);
+        return c.upload(sh, pr, q, q, Av, ABv, P->stream);
 }
 
 // q0 (once per plan) and the gradient pair lists (per screening tolerance)
@@ -2210,7 +2228,7 @@ static int ensure_grad(b200jk_plan *P, double tol)
         if (!g.q0_ready) {
                 if ((rc = ensure_goff(P->device, true))) return rc;
                 std::vector<double> init(n2, 1e-100);
-                if ((rc = dev_upload(g.q0, init))) return rc;
+                if ((rc = dev_upload(g.q0, init, P->stream))) return rc;
                 // (the pair lists of the bounds go where the ket lists go later)
                 for (int X = 0; X < NPAIRCLASS; X++) {
                         const std::vector<PairLite> &hv = P->all_pairs[X];
@@ -2271,6 +2289,7 @@ static int ensure_grad(b200jk_plan *P, double tol)
                 order(hk, qk);
                 if ((rc = upload_pairs(P, g.bra[X], X, hb, qb)) || (rc = upload_pairs(P, g.ket[X], X, hk, qk))) return rc;
         }
+        CUDA_TRY(cudaStreamSynchronize(P->stream));   // the build may run on any stream
         g.tol = tol;
         g.lists_ready = true;
         return B200JK_OK;
@@ -2337,7 +2356,9 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
                 }
         if (nseg_all + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one build");
         const size_t NQ = NPAIRCLASS * NPAIRCLASS;
-        if (fused && ((rc = dev_alloc(g.de, (size_t)3 * P->natm)) || (!g.shell_atom.p && (rc = dev_upload(g.shell_atom, P->shell_atom)))))
+        cudaStream_t s = stream ? (cudaStream_t)stream : P->stream;
+        if (fused && ((rc = dev_alloc(g.de, (size_t)3 * P->natm)) ||
+                      (!g.shell_atom.p && (rc = dev_upload(g.shell_atom, P->shell_atom, s)))))
                 return rc;
         if ((rc = dev_alloc(g.D, nn * n_dm)) || (rc = dev_alloc(g.Dc, nc * n_dm)) || (rc = dev_alloc(g.Ds, nc * n_dm)) ||
             (rc = dev_alloc(g.V, fused ? 1 : 6 * nc * n_dm)) || (rc = dev_alloc(g.out, dev_ptrs || fused ? 1 : 6 * nn * n_dm)) ||
@@ -2354,7 +2375,6 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
         if ((rc = lease.pool.take(lease.fan))) return rc;
         StreamFan &lanes = *lease.fan;
 
-        cudaStream_t s = stream ? (cudaStream_t)stream : P->stream;
         if (!passes.empty()) {
                 std::vector<CountDesc> h;
                 for (const Pass &p : passes) h.push_back(p.d);
@@ -3147,13 +3167,15 @@ static int ensure_fill(b200jk_plan *P)
                 nseg += h2.size() * B2_NBUCKET * (X + 1);
         }
         if (nseg + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one fill");
-        if ((rc = dev_alloc(P->fill_cdesc, 64)) || (rc = dev_alloc(P->fill_next, 64)) || (rc = dev_upload(P->fill_one, std::vector<double>(1, 1.0))) || (rc = dev_alloc(P->fill_nkl, nseg)) ||
-            (rc = dev_alloc(P->fill_kst, nseg)) || (rc = dev_alloc(P->fill_nchunk, nseg + 1)) ||
-            (rc = dev_alloc(P->fill_chunk_off, nseg + 1)))
+        if ((rc = dev_alloc(P->fill_cdesc, 64)) || (rc = dev_alloc(P->fill_next, 64)) ||
+            (rc = dev_upload(P->fill_one, std::vector<double>(1, 1.0), P->stream)) ||
+            (rc = dev_alloc(P->fill_nkl, nseg)) || (rc = dev_alloc(P->fill_kst, nseg)) ||
+            (rc = dev_alloc(P->fill_nchunk, nseg + 1)) || (rc = dev_alloc(P->fill_chunk_off, nseg + 1)))
                 return rc;
         size_t tmp = 0;
         CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp, P->fill_nchunk.p, P->fill_chunk_off.p, (int)nseg + 1));
         if ((rc = dev_alloc(P->fill_cub, std::max<size_t>(tmp, 1)))) return rc;
+        CUDA_TRY(cudaStreamSynchronize(P->stream));   // the fill may run on any stream
         P->fill_ready = true;
         return B200JK_OK;
 }
@@ -3351,7 +3373,7 @@ int b200jk_incore_jk(const double *eri, long long eri_len, int nao, const double
                         W.nf[v] = (int)items[v].size();
                         W.h_items.insert(W.h_items.end(), items[v].begin(), items[v].end());
                 }
-                if ((rc = dev_upload(W.items, W.h_items))) return rc;
+                if ((rc = dev_upload(W.items, W.h_items, s))) return rc;
                 W.items_nao = nao;
                 W.items_s8 = s8;
         }
