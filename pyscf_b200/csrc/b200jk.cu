@@ -76,8 +76,9 @@ static int check_dev_ptr(const void *p, int device, const char *what)
         return B200JK_OK;
 }
 
-// Test hook: when positive, the n-th device allocation from now on fails as
-// an out-of-memory condition would (b200jk_debug_fail_alloc).  0 = off.
+// Test hook: when positive, the n-th device allocation or stream of a build's
+// stream set from now on fails as it would for lack of resources
+// (b200jk_debug_fail_alloc).  0 = off.
 static std::atomic<long long> g_fail_alloc_countdown{0};
 static bool alloc_should_fail()
 {
@@ -233,6 +234,7 @@ struct StreamFan {
                 if (ready) return B200JK_OK;
                 if (!forked) CUDA_TRY(cudaEventCreateWithFlags(&forked, cudaEventDisableTiming));
                 for (int i = 0; i < N; i++) {
+                        if (alloc_should_fail()) return fail(B200JK_ECUDA, "stream creation failed (test hook)");
                         if (!st[i]) CUDA_TRY(cudaStreamCreateWithFlags(&st[i], cudaStreamNonBlocking));
                         if (!done[i]) CUDA_TRY(cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming));
                 }
@@ -306,7 +308,10 @@ struct FanPool {
                 }
                 if (!out) out = new StreamFan();
                 const int rc = out->create();
-                if (rc) give(out);
+                if (rc) {
+                        give(out);       // deletes it: the caller's lease must not give it again
+                        out = nullptr;
+                }
                 return rc;
         }
         void give(StreamFan *f)

@@ -1,0 +1,63 @@
+"""The stream sets builds run on: every allocation and stream creation of a
+first J/K, gradient and fill made to fail in turn.  Each failure is an error
+code, and the next call on the same plan is right."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.join(os.path.dirname(os.path.abspath(__file__)), '..')
+
+# In a process of its own: sets are kept while a device has plans, so only
+# the first build after the last plan has gone creates one.
+SCRIPT = r'''
+import sys
+sys.path[:0] = ['.', 'tests']
+import numpy
+from conftest import load_fixture
+from pyscf_b200 import lib
+f = load_fixture('h2o_631g')
+d = f['dm_rand'] + f['dm_rand'].T
+calls = {
+    'jk': lambda p: numpy.array(p.get_jk(d, hermi=1)),
+    'grad': lambda p: numpy.array(p.grad_jk(d)),
+    'force': lambda p: p.grad_contract(d),
+    'fill': lambda p: p.int2e_s8(device=False),
+}
+call = calls[sys.argv[1]]
+new = lambda: lib.Plan(f['atm'], f['bas'], f['env'], direct_scf_tol=1e-13)
+p = new()
+want = call(p)
+p.close()
+streams = nth = 0
+while True:
+    nth += 1
+    p = new()
+    lib.load().b200jk_debug_fail_alloc(nth)
+    try:
+        got = call(p)
+        failed = False
+    except lib.B200JKError as e:
+        failed = True
+        assert e.code in (lib.B200JK_ENOMEM, lib.B200JK_ECUDA), e
+        assert (e.code == lib.B200JK_ECUDA) == ('stream creation' in str(e)), e
+        streams += 'stream creation' in str(e)
+    lib.load().b200jk_debug_fail_alloc(0)
+    got = call(p)
+    assert abs(got - want).max() < 1e-10 * max(1.0, abs(want).max()), nth
+    p.close()
+    if not failed:
+        break
+assert nth < 200 and streams == 7, (nth, streams)
+print('ok', nth)
+'''
+
+
+@pytest.mark.parametrize('call', ['jk', 'grad', 'force', 'fill'])
+def test_failing_stream_sets(call):
+    r = subprocess.run([sys.executable, '-c', SCRIPT, call], cwd=ROOT, stdout=subprocess.PIPE, stderr=subprocess.STDOUT,
+                       timeout=300)
+    assert r.returncode == 0 and r.stdout.startswith(b'ok'), r.stdout.decode()[-2000:]
