@@ -382,8 +382,8 @@ int b200jk_measure_fp64_peak(int device, double *tflops);
 /* Test hook, no reference counterpart: the nth device allocation made by
  * the library from now on fails as an out-of-memory condition would (the
  * call returns B200JK_ENOMEM and frees what it had taken); the streams a
- * build spreads its classes over count as well (B200JK_ECUDA).  0 turns it
- * off. */
+ * build spreads its classes over and each launch it puts on one count as well
+ * (B200JK_ECUDA).  0 turns it off. */
 int b200jk_debug_fail_alloc(int nth);
 
 /* Host replay of the device integral code for one shell quartet (no GPU is

@@ -76,9 +76,9 @@ static int check_dev_ptr(const void *p, int device, const char *what)
         return B200JK_OK;
 }
 
-// Test hook: when positive, the n-th device allocation or stream of a build's
-// stream set from now on fails as it would for lack of resources
-// (b200jk_debug_fail_alloc).  0 = off.
+// Test hook: when positive, the n-th device allocation, stream of a build's
+// stream set or lane taken from one fails from now on as it would for lack of
+// resources (b200jk_debug_fail_alloc).  0 = off.
 static std::atomic<long long> g_fail_alloc_countdown{0};
 static bool alloc_should_fail()
 {
@@ -251,6 +251,7 @@ struct StreamFan {
         // the next lane in turn (the caller's stream is one of them)
         int take(cudaStream_t s, cudaStream_t &out)
         {
+                if (alloc_should_fail()) return fail(B200JK_ECUDA, "lane of a stream set failed (test hook)");
                 if (lane == N) {
                         lane = 0;
                         out = s;
@@ -286,8 +287,25 @@ struct StreamFan {
         }
 };
 
+// The work a call has put on its stream and, between fork and join, on the
+// lanes of a fan.  A call that returns early waits here: nothing is left
+// running on the plan's buffers, the caller's arrays or lanes that the next
+// build is lent.  A call that has waited by itself says so (ended).
+struct InFlight {
+        cudaStream_t s;
+        StreamFan *fan;
+        bool ended = false;
+        InFlight(cudaStream_t s_, StreamFan *fan_) : s(s_), fan(fan_) {}
+        ~InFlight()
+        {
+                if (ended) return;
+                for (int i = 0; fan && i < fan->used; i++) cudaStreamSynchronize(fan->st[i]);
+                cudaStreamSynchronize(s);
+        }
+};
+
 // The fans of a device, lent to one build at a time (a build returns after
-// its work has ended, so a fan comes back idle).  Builds in several threads
+// its work has ended, also on an error: InFlight; so a fan comes back idle).  Builds in several threads
 // hold one each; at most KEEP idle ones are kept, none once the device has no
 // plan left.  (Seven streams in every plan made creating the next plan 1.5-2
 // ms slower.)
@@ -1392,6 +1410,7 @@ int b200jk_int1e(b200jk_plan *P, double *ovlp, double *hcore, int dev_ptrs, void
         const size_t nc = (size_t)P->naoc * P->naoc, nn = (size_t)P->nao * P->nao;
         if ((rc = ensure_i1(P))) return rc;
         cudaStream_t s = stream ? (cudaStream_t)stream : P->stream;
+        InFlight work(s, nullptr);
         CUDA_TRY(cudaMemsetAsync(P->i1_S.p, 0, sizeof(double) * nc, s));
         CUDA_TRY(cudaMemsetAsync(P->i1_H.p, 0, sizeof(double) * nc, s));
         long long nelem = 0;
@@ -1425,6 +1444,7 @@ int b200jk_int1e(b200jk_plan *P, double *ovlp, double *hcore, int dev_ptrs, void
                 if (hcore) CUDA_TRY(cudaMemcpyAsync(hcore, oh, sizeof(double) * nn, cudaMemcpyDeviceToHost, s));
         }
         CUDA_TRY(cudaStreamSynchronize(s));
+        work.ended = true;
         return B200JK_OK;
 }
 
@@ -1445,6 +1465,7 @@ int b200jk_grad_int1e(b200jk_plan *P, const double *dm, const double *dme, doubl
         const int natm = (int)P->h_atoms.size();
         if ((rc = dev_alloc(P->i1_de, 3 * (size_t)natm))) return rc;
         cudaStream_t s = stream ? (cudaStream_t)stream : P->stream;
+        InFlight work(s, nullptr);
         // the Cartesian D and W live in the overlap/hcore scratch
         const double *dD = dm, *dW = dme;
         if (!dev_ptrs) {
@@ -1482,6 +1503,7 @@ int b200jk_grad_int1e(b200jk_plan *P, const double *dm, const double *dme, doubl
         }
         if (!dev_ptrs) CUDA_TRY(cudaMemcpyAsync(de, out, sizeof(double) * 3 * natm, cudaMemcpyDeviceToHost, s));
         CUDA_TRY(cudaStreamSynchronize(s));
+        work.ended = true;
         return B200JK_OK;
 }
 
@@ -1650,8 +1672,10 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
         long long nseg = 0, nscan = 0;
         const std::vector<ClassPass> passes = class_passes(P, mixed, n_dm, nk, nseg, nscan);
         FanLease lease(P->device);
-        if ((rc = ensure_count(P, passes, nseg, nscan, s)) || (rc = lease.pool.take(lease.fan))) return rc;
+        if ((rc = lease.pool.take(lease.fan))) return rc;
         StreamFan &lanes = *lease.fan;
+        InFlight work(s, lease.fan);
+        if ((rc = ensure_count(P, passes, nseg, nscan, s))) return rc;
         CUDA_TRY(cudaEventRecord(P->ev0, s));
         const double *dD = dms;
         if (!dev_ptrs) {
@@ -1757,11 +1781,9 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
                 a.screen = P->screen;
                 a.omega2 = P->omega2;
                 cudaStream_t cs = s;
-                if (fan && (rc = lanes.take(s, cs))) { lanes.join(s); return rc; }
-                if ((rc = dispatch_jk(P, bra.la, bra.lb, ket.la, ket.lb, a, c.pass, cs, nullptr, nullptr, 0, c.variant))) {
-                        if (fan) lanes.join(s);
+                if (fan && (rc = lanes.take(s, cs))) return rc;
+                if ((rc = dispatch_jk(P, bra.la, bra.lb, ket.la, ket.lb, a, c.pass, cs, nullptr, nullptr, 0, c.variant)))
                         return rc;
-                }
                 launches++;
                 if (P->profiling && (i + 1 == passes.size() || passes[i + 1].t != t))
                         CUDA_TRY(cudaEventRecord(P->cls_ev[2 * t + 1], s));
@@ -1805,6 +1827,7 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
         unsigned long long hs[4 * 64];
         CUDA_TRY(cudaMemcpyAsync(hs, P->stats.p, sizeof(hs), cudaMemcpyDeviceToHost, s));
         CUDA_TRY(cudaStreamSynchronize(s));
+        work.ended = true;
         float ms = 0;
         CUDA_TRY(cudaEventElapsedTime(&ms, P->ev0, P->ev1));
         P->st.quartets = 0;
@@ -2379,6 +2402,7 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
         FanLease lease(P->device);
         if ((rc = lease.pool.take(lease.fan))) return rc;
         StreamFan &lanes = *lease.fan;
+        InFlight work(s, lease.fan);
 
         if (!passes.empty()) {
                 std::vector<CountDesc> h;
@@ -2462,12 +2486,9 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
                 a.shell_atom = fused ? g.shell_atom.p : nullptr;
                 std::string err;
                 cudaStream_t cs = s;
-                if (fan && (rc = lanes.take(s, cs))) { lanes.join(s); return rc; }
+                if (fan && (rc = lanes.take(s, cs))) return rc;
                 if (P->profiling) CUDA_TRY(cudaEventRecord(g.cls_ev[2 * t], s));
-                if (g_grad_launch[p.X](ket.la, ket.lb, a, cs, P->nsm, err)) {
-                        if (fan) lanes.join(s);
-                        return fail(B200JK_ECUDA, err);
-                }
+                if (g_grad_launch[p.X](ket.la, ket.lb, a, cs, P->nsm, err)) return fail(B200JK_ECUDA, err);
                 if (P->profiling) CUDA_TRY(cudaEventRecord(g.cls_ev[2 * t + 1], s));
                 ran[t] = 1;
                 launches++;
@@ -2504,6 +2525,7 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
         std::vector<unsigned long long> hs(2 * NPAIRCLASS * NPAIRCLASS);
         CUDA_TRY(cudaMemcpyAsync(hs.data(), g.stats.p, sizeof(unsigned long long) * hs.size(), cudaMemcpyDeviceToHost, s));
         CUDA_TRY(cudaStreamSynchronize(s));
+        work.ended = true;
         float ms = 0;
         CUDA_TRY(cudaEventElapsedTime(&ms, P->ev0, P->ev1));
         g.quartets = g.prim_quartets = 0;
@@ -2761,6 +2783,9 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                 if ((rc = dev_alloc(B->cub_tmp, cub_bytes + 16))) return rc;
         }
         const b200jk_batch::Staging &h = B->staging[async ? 1 : 0];
+        // (the asynchronous entry never waits: its stream may be capturing)
+        InFlight work(s, &B->fan);
+        work.ended = async;
 
         if (!async) CUDA_TRY(cudaEventRecord(B->ev0, s));
         int64_t launches = 0;
@@ -2922,6 +2947,7 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
         unsigned long long hs[4 * 64];
         CUDA_TRY(cudaMemcpyAsync(hs, B->stats.p, sizeof(hs), cudaMemcpyDeviceToHost, s));
         CUDA_TRY(cudaStreamSynchronize(s));
+        work.ended = true;
         float ms = 0;
         CUDA_TRY(cudaEventElapsedTime(&ms, B->ev0, B->ev1));
         B->quartets = B->prim_quartets = B->fp32_quartets = 0;
@@ -3054,6 +3080,7 @@ extern "C" int b200jk_get_jk_noalloc(b200jk_plan *P, const double *dms, int n_dm
         void *cub_tmp = base + o_cub;
 
         cudaStream_t s = stream ? (cudaStream_t)stream : P->stream;
+        InFlight work(s, nullptr);
         // the array keeps the previous call's contents: clear what accumulates
         CUDA_TRY(cudaMemsetAsync(dmax, 0, sizeof(unsigned long long), s));
         CUDA_TRY(cudaMemsetAsync(stats, 0, 2 * 64 * sizeof(unsigned long long), s));
@@ -3126,6 +3153,7 @@ extern "C" int b200jk_get_jk_noalloc(b200jk_plan *P, const double *dms, int n_dm
                 }
         }
         CUDA_TRY(cudaStreamSynchronize(s));
+        work.ended = true;
         return B200JK_OK;
 }
 
@@ -3240,12 +3268,13 @@ int b200jk_int2e_s8(b200jk_plan *P, double *eri, long long len, int dev_ptr, voi
                 }
         }
         auto run = [&]() -> int {
-                CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * need, s));
                 auto qcs = quartet_classes();
                 FanLease lease(P->device);
                 int rc;
                 if ((rc = lease.pool.take(lease.fan))) return rc;
                 StreamFan &lanes = *lease.fan;
+                InFlight work(s, lease.fan);
+                CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * need, s));
                 if (!passes.empty()) {
                         std::vector<CountDesc> h;
                         for (const Pass &p : passes) h.push_back(p.d);
@@ -3291,15 +3320,13 @@ int b200jk_int2e_s8(b200jk_plan *P, double *eri, long long len, int dev_ptr, voi
                         f.eri = out;
                         std::string err;
                         cudaStream_t cs = s;
-                        if ((rc = lanes.take(s, cs))) { lanes.join(s); return rc; }
-                        if (g_fill_launch[qcs[t].X](ket.la, ket.lb, f, cs, P->nsm, err)) {
-                                lanes.join(s);
-                                return fail(B200JK_ECUDA, err);
-                        }
+                        if ((rc = lanes.take(s, cs))) return rc;
+                        if (g_fill_launch[qcs[t].X](ket.la, ket.lb, f, cs, P->nsm, err)) return fail(B200JK_ECUDA, err);
                 }
                 if ((rc = lanes.join(s))) return rc;
                 if (!dev_ptr) CUDA_TRY(cudaMemcpyAsync(eri, out, sizeof(double) * need, cudaMemcpyDeviceToHost, s));
                 CUDA_TRY(cudaStreamSynchronize(s));
+                work.ended = true;
                 return B200JK_OK;
         };
         rc = run();
@@ -3361,6 +3388,7 @@ int b200jk_incore_jk(const double *eri, long long eri_len, int nao, const double
         const double *E = eri, *Dd = dms;
         double *oj = vj, *ok = vk;
         cudaStream_t s = stream ? (cudaStream_t)stream : 0;
+        InFlight work(s, nullptr);   // (ends before the workspace is unlocked)
         if (!dev_ptrs) {
                 if ((rc = dev_alloc(W.eri, (size_t)eri_len)) || (rc = dev_alloc(W.dms, nn * n_dm)) ||
                     (with_j && (rc = dev_alloc(W.vj, nn * n_dm))) || (with_k && (rc = dev_alloc(W.vk, nn * n_dm))))
@@ -3422,5 +3450,6 @@ int b200jk_incore_jk(const double *eri, long long eri_len, int nao, const double
                 if (with_k) CUDA_TRY(cudaMemcpyAsync(vk, W.vk.p, sizeof(double) * nn * n_dm, cudaMemcpyDeviceToHost, s));
         }
         CUDA_TRY(cudaStreamSynchronize(s));
+        work.ended = true;
         return B200JK_OK;
 }

@@ -1,6 +1,6 @@
-"""The stream sets builds run on: every allocation and stream creation of a
-first J/K, gradient and fill made to fail in turn.  Each failure is an error
-code, and the next call on the same plan is right."""
+"""The stream sets builds run on: every allocation, stream creation and lane of
+a first J/K, gradient and fill made to fail in turn.  Each failure is an error
+code, nothing is left running, and the next call on the same plan is right."""
 import os
 import subprocess
 import sys
@@ -43,7 +43,7 @@ while True:
     except lib.B200JKError as e:
         failed = True
         assert e.code in (lib.B200JK_ENOMEM, lib.B200JK_ECUDA), e
-        assert (e.code == lib.B200JK_ECUDA) == ('stream creation' in str(e)), e
+        assert (e.code == lib.B200JK_ECUDA) == ('(test hook)' in str(e)), e
         streams += 'stream creation' in str(e)
     lib.load().b200jk_debug_fail_alloc(0)
     got = call(p)
@@ -61,3 +61,39 @@ def test_failing_stream_sets(call):
     r = subprocess.run([sys.executable, '-c', SCRIPT, call], cwd=ROOT, stdout=subprocess.PIPE, stderr=subprocess.STDOUT,
                        timeout=300)
     assert r.returncode == 0 and r.stdout.startswith(b'ok'), r.stdout.decode()[-2000:]
+
+
+@pytest.mark.parametrize('op', ['jk', 'grad', 'fill', 'batch'])
+@pytest.mark.parametrize('nth', [2, 8, 17])
+def test_error_between_fork_and_join_waits(op, nth):
+    """A launch that fails with others in flight: the call returns once those
+    have ended (the caller's stream is idle), and the next call is right."""
+    import torch
+    from conftest import load_fixture
+    from pyscf_b200 import lib
+    if lib.device_count() == 0:
+        pytest.skip('no GPU')
+    f = load_fixture('h2o8_vdz')
+    d = torch.from_numpy(f['dm_rand'] + f['dm_rand'].T).cuda()
+    plans = [lib.Plan(f['atm'], f['bas'], f['env'], direct_scf_tol=1e-13) for _ in range(4)]
+    p = plans[0]
+    batch = lib.Batch(plans)
+    call = {'jk': lambda: torch.stack(p.get_jk_device(d, hermi=1)), 'grad': lambda: torch.stack(p.grad_jk_device(d)),
+            'fill': lambda: p.int2e_s8(),
+            'batch': lambda: torch.stack(sum(batch.get_jk_device([d] * 4), []))}[op]
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        want = call()
+        side.synchronize()
+        lib.load().b200jk_debug_fail_alloc(nth)
+        try:
+            with pytest.raises(lib.B200JKError, match='lane of a stream set') as e:
+                call()
+            idle = side.query()
+        finally:
+            lib.load().b200jk_debug_fail_alloc(0)
+        assert e.value.code == lib.B200JK_ECUDA and idle
+        got = call()
+        side.synchronize()
+        assert float((got - want).abs().max()) < 1e-10 * max(1.0, float(want.abs().max()))
