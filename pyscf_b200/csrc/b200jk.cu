@@ -429,6 +429,7 @@ struct PairClassDev {
                 mem.release();
                 sh = nullptr; pr = nullptr; q = qs = nullptr; A = AB = nullptr;
                 n = 0;
+                for (int &b : boff) b = 0;
         }
 };
 
@@ -2224,7 +2225,8 @@ static const gq0_launcher_t g_gq0_launch[NPAIRCLASS] = {
         launch_gq0_00, launch_gq0_10, launch_gq0_11, launch_gq0_20, launch_gq0_21,
         launch_gq0_22, launch_gq0_30, launch_gq0_31, launch_gq0_32, launch_gq0_33};
 
-// upload one class of pairs in the given order, q per pair, on the plan's stream
+// upload one class of pairs in the given order, q per pair, on the plan's
+// stream; on failure the class is left empty
 static int upload_pairs(const b200jk_plan *P, PairClassDev &c, int X, const std::vector<PairLite> &hv,
                         const std::vector<double> &q)
 {
@@ -2243,7 +2245,9 @@ static int upload_pairs(const b200jk_plan *P, PairClassDev &c, int X, const std:
                 Av[t] = make_double4(A.R[0], A.R[1], A.R[2], hv[t].i == hv[t].j ? 1.0 : 0.0);
                 ABv[t] = make_double4(A.R[0] - B.R[0], A.R[1] - B.R[1], A.R[2] - B.R[2], 0.0);
         }
-        return c.upload(sh, pr, q, q, Av, ABv, P->stream);
+        const int rc = c.upload(sh, pr, q, q, Av, ABv, P->stream);
+        if (rc) c.release();
+        return rc;
 }
 
 // q0 (once per plan) and the gradient pair lists (per screening tolerance)
@@ -2285,6 +2289,7 @@ static int ensure_grad(b200jk_plan *P, double tol)
                 g.lists_ready = false;
         }
         if (g.lists_ready && g.tol == tol) return B200JK_OK;
+        g.lists_ready = false;   // until every class holds the new tolerance's lists
         const std::vector<double> &q1 = P->h_qcond, &q0 = g.h_q0;
         double q0max = 0, q1max = 0;
         for (size_t t = 0; t < n2; t++) { q0max = std::max(q0max, q0[t]); q1max = std::max(q1max, q1[t]); }

@@ -93,3 +93,28 @@ def test_nan_density_propagates_and_plan_recovers(b2):
     vj, vk = p.get_jk(f['dm_rand'], hermi=1)
     assert abs(vj - f['vj_rand']).max() < TOL_JK
     assert abs(vk - f['vk_rand']).max() < TOL_JK
+
+
+@pytest.mark.parametrize('nth', [1, 2, 4])
+def test_failed_gradient_replan_is_planned_again(b2, nth):
+    """A tighter gradient tolerance whose longer pair lists cannot be
+    allocated: the call at the first tolerance after it plans its lists again
+    instead of using a mixture of the two."""
+    f = load_fixture('h2o8_vdz')
+    d = f['dm_rand'] + f['dm_rand'].T
+    p = b2.Plan(f['atm'], f['bas'], f['env'], direct_scf_tol=1e-13)
+    want = p.grad_jk(d, direct_scf_tol=1e-3)
+    nq = p.grad_stats()['quartets']
+    tight = b2.Plan(f['atm'], f['bas'], f['env'], direct_scf_tol=1e-13).grad_jk(d, direct_scf_tol=0.0)
+    b2.load().b200jk_debug_fail_alloc(nth)
+    try:
+        with pytest.raises(b2.B200JKError) as e:
+            p.grad_jk(d, direct_scf_tol=0.0)
+        assert e.value.code == b2.B200JK_ENOMEM
+    finally:
+        b2.load().b200jk_debug_fail_alloc(0)
+    for tol, ref in ((1e-3, want), (0.0, tight), (1e-3, want)):
+        got = p.grad_jk(d, direct_scf_tol=tol)
+        for g, r in zip(got, ref):
+            assert abs(g - r).max() < TOL_JK * max(1.0, abs(r).max())
+    assert p.grad_stats()['quartets'] == nq
