@@ -194,6 +194,7 @@ static int dev_upload(DevArr<T> &d, const std::vector<T> &h, cudaStream_t s)
         if (d.n == 0) return B200JK_OK;
         if (alloc_should_fail() || cudaMalloc(&d.p, sizeof(T) * d.n) != cudaSuccess) {
                 d.p = nullptr;
+                d.n = 0;
                 return fail(B200JK_ENOMEM, "cudaMalloc failed for a plan table");
         }
         CUDA_TRY(cudaMemcpyAsync(d.p, h.data(), sizeof(T) * d.n, cudaMemcpyHostToDevice, s));
@@ -3411,6 +3412,7 @@ int b200jk_incore_jk(const double *eri, long long eri_len, int nao, const double
                         W.nf[v] = (int)items[v].size();
                         W.h_items.insert(W.h_items.end(), items[v].begin(), items[v].end());
                 }
+                W.items_nao = -1;   // (no list while the upload may fail)
                 if ((rc = dev_upload(W.items, W.h_items, s))) return rc;
                 W.items_nao = nao;
                 W.items_s8 = s8;

@@ -118,3 +118,30 @@ def test_failed_gradient_replan_is_planned_again(b2, nth):
         for g, r in zip(got, ref):
             assert abs(g - r).max() < TOL_JK * max(1.0, abs(r).max())
     assert p.grad_stats()['quartets'] == nq
+
+
+def test_failed_item_list_of_the_stored_tensor(b2):
+    """The stored-tensor contraction keeps the last basis size's item list per
+    GPU: when the list of another size cannot be allocated, the next call at
+    the first size makes its list again."""
+    import torch
+    from pyscf_b200 import incore
+    rng = numpy.random.default_rng(3)
+    cases = []
+    for nao in (24, 9):
+        npair = nao * (nao + 1) // 2
+        eri = torch.from_numpy(rng.standard_normal(npair * (npair + 1) // 2)).cuda()
+        d = rng.standard_normal((nao, nao))
+        cases.append((eri, torch.from_numpy(d + d.T).cuda()))
+    want = [torch.stack(incore.incore(e, d, hermi=1)) for e, d in reversed(cases)][::-1]
+    incore.incore(*cases[0], hermi=1)      # the list of nao = 24 is there
+    b2.load().b200jk_debug_fail_alloc(1)   # nao = 9 needs no larger workspace, only its list
+    try:
+        with pytest.raises(b2.B200JKError) as e:
+            incore.incore(*cases[1], hermi=1)
+        assert e.value.code == b2.B200JK_ENOMEM
+    finally:
+        b2.load().b200jk_debug_fail_alloc(0)
+    for (eri, d), w in zip(cases, want):
+        got = torch.stack(incore.incore(eri, d, hermi=1))
+        assert float((got - w).abs().max()) < 1e-12 * float(w.abs().max())
