@@ -2631,6 +2631,11 @@ struct b200jk_batch {
                 BatchClass *bc = nullptr;
         } staging[2];
         size_t h_cap = 0;               // entries the staging holds
+        // what the last synchronous build set up completely (every buffer and
+        // stream): the asynchronous entry runs within it or not at all
+        bool ready = false;
+        size_t ready_cap = 0;
+        long long ready_segs = 0;
         // workspace generation of every plan when the last synchronous build
         // sized the buffers; the asynchronous entry refuses to run when a
         // plan's workspace has moved since (its captured graphs would use the
@@ -2717,10 +2722,10 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
         cudaStream_t s = stream ? (cudaStream_t)stream : B->stream;
         const int nk = hermi == 1 ? 1 : 2;
         int rc;
+        if (async && !B->ready)
+                return fail(B200JK_EINVAL, "b200jk_batch_get_jk_async needs one b200jk_batch_get_jk call first");
         for (int m = 0; m < nmol; m++) {
                 if (async) {
-                        if (B->plans[m]->ws_ndm < 1 || B->ws_gen.size() != (size_t)nmol)
-                                return fail(B200JK_EINVAL, "b200jk_batch_get_jk_async needs one b200jk_batch_get_jk call first");
                         if (B->plans[m]->ws_gen != B->ws_gen[m])
                                 return fail(B200JK_EINVAL, "a plan's workspace moved since the last b200jk_batch_get_jk "
                                                            "(a larger build on it); call b200jk_batch_get_jk again");
@@ -2731,10 +2736,6 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                                 return rc;
                         if ((rc = ensure_workspace(B->plans[m], 1))) return rc;
                 }
-        }
-        if (!async) {
-                B->ws_gen.resize(nmol);
-                for (int m = 0; m < nmol; m++) B->ws_gen[m] = B->plans[m]->ws_gen;
         }
         auto qcs = quartet_classes();
         const int nclass = (int)qcs.size();
@@ -2764,9 +2765,10 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
         }
         if (cap_segs + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one batch");
         if (async) {
-                if (cap > B->h_cap || !B->staging[1].args || B->args.n < cap || B->nkl.n < (size_t)cap_segs)
+                if (cap > B->ready_cap || cap_segs > B->ready_segs)
                         return fail(B200JK_EINVAL, "b200jk_batch_get_jk_async needs one b200jk_batch_get_jk call first");
         } else {
+                B->ready = false;
                 if (cap > B->h_cap || !B->staging[1].args) {
                         B->free_staging();
                         for (auto &h : B->staging) {
@@ -2787,6 +2789,11 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                 size_t cub_bytes = 0;
                 cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, B->nchunk.p, B->chunk_off.p, (int)(cap_segs + 1));
                 if ((rc = dev_alloc(B->cub_tmp, cub_bytes + 16))) return rc;
+                B->ws_gen.resize(nmol);
+                for (int m = 0; m < nmol; m++) B->ws_gen[m] = B->plans[m]->ws_gen;
+                B->ready_cap = cap;
+                B->ready_segs = cap_segs;
+                B->ready = true;
         }
         const b200jk_batch::Staging &h = B->staging[async ? 1 : 0];
         // (the asynchronous entry never waits: its stream may be capturing)

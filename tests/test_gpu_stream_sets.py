@@ -97,3 +97,35 @@ def test_error_between_fork_and_join_waits(op, nth):
         got = call()
         side.synchronize()
         assert float((got - want).abs().max()) < 1e-10 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize('nth', [1, 2, 5, 8, 10, 11, 17, 18])
+def test_async_batch_after_a_failed_set_up(nth):
+    """The synchronous batch call's set-up fails at one of its ten buffers, its
+    seven streams or the scan storage: the asynchronous entry is refused on
+    the host until a synchronous call has succeeded."""
+    import torch
+    from conftest import load_fixture
+    from pyscf_b200 import lib
+    if lib.device_count() == 0:
+        pytest.skip('no GPU')
+    f = load_fixture('h2o_vdz')
+    d = torch.from_numpy(f['dm_rand'] + f['dm_rand'].T).cuda()
+    plans = [lib.Plan(f['atm'], f['bas'], f['env'], direct_scf_tol=1e-13) for _ in range(2)]
+    want = [p.get_jk_device(d, hermi=1) for p in plans]      # (their workspaces exist)
+    batch = lib.Batch(plans)
+    vj, vk = [torch.empty_like(d) for _ in plans], [torch.empty_like(d) for _ in plans]
+    lib.load().b200jk_debug_fail_alloc(nth)
+    try:
+        with pytest.raises(lib.B200JKError):
+            batch.get_jk_device([d, d])
+    finally:
+        lib.load().b200jk_debug_fail_alloc(0)
+    with pytest.raises(lib.B200JKError, match='one b200jk_batch_get_jk call first') as e:
+        batch.get_jk_device_async([d, d], vj, vk)
+    assert e.value.code == lib.B200JK_EINVAL
+    batch.get_jk_device([d, d])
+    batch.get_jk_device_async([d, d], vj, vk)
+    torch.cuda.synchronize()
+    for j, k, (rj, rk) in zip(vj, vk, want):
+        assert float((j - rj).abs().max()) < 1e-10 and float((k - rk).abs().max()) < 1e-10
