@@ -550,7 +550,6 @@ struct b200jk_plan {
         DevArr<int4> seg_info;
         DevArr<int> out_seg, out_comp, cart_seg, cart_comp, ao_loc_d;
         // workspace; ws_gen counts the times its buffers moved
-        int ws_ndm = 0;
         long long ws_gen = 0;
         DevArr<double> D, Dc, Ds, Jacc, Kacc, outJ, outK;
         DevArr<unsigned long long> dmax, stats;
@@ -1524,10 +1523,9 @@ static std::vector<const void *> workspace_key(const b200jk_plan *P)
                 P->stats.p, P->Dpk.p, P->Jpk.p};
 }
 
-static int ensure_workspace(b200jk_plan *P, int n_dm)
+static int alloc_workspace(b200jk_plan *P, int n_dm)
 {
         const size_t nn = (size_t)P->nao * P->nao, nc = (size_t)P->naoc * P->naoc;
-        const std::vector<const void *> key0 = workspace_key(P);
         int rc;
         if ((rc = dev_alloc(P->D, nn * n_dm)) || (rc = dev_alloc(P->Dc, nc * n_dm * 2)) ||
             (rc = dev_alloc(P->Ds, nc * n_dm)) || (rc = dev_alloc(P->Jacc, nc * n_dm)) ||
@@ -1537,9 +1535,16 @@ static int ensure_workspace(b200jk_plan *P, int n_dm)
             (rc = dev_alloc(P->Dpk, (size_t)std::max<long long>(1, P->pk_total) * n_dm)) ||
             (rc = dev_alloc(P->Jpk, (size_t)std::max<long long>(1, P->pk_total) * n_dm)))
                 return rc;
-        P->ws_ndm = std::max(P->ws_ndm, n_dm);
-        if (workspace_key(P) != key0) P->ws_gen++;
         return B200JK_OK;
+}
+
+static int ensure_workspace(b200jk_plan *P, int n_dm)
+{
+        const std::vector<const void *> key0 = workspace_key(P);
+        const int rc = alloc_workspace(P, n_dm);
+        // (counted on failure too: buffers may have moved or gone before it)
+        if (workspace_key(P) != key0) P->ws_gen++;
+        return rc;
 }
 
 // One launch of a build: a quartet class in one precision pass.

@@ -129,3 +129,37 @@ def test_async_batch_after_a_failed_set_up(nth):
     torch.cuda.synchronize()
     for j, k, (rj, rk) in zip(vj, vk, want):
         assert float((j - rj).abs().max()) < 1e-10 and float((k - rk).abs().max()) < 1e-10
+
+
+@pytest.mark.parametrize('nth', [1, 3, 6])
+def test_async_batch_after_a_failed_larger_build(nth):
+    """A build of two densities on a plan of the batch fails while its
+    workspace grows: the asynchronous entry sees that the workspace moved."""
+    import numpy
+    import torch
+    from conftest import load_fixture
+    from pyscf_b200 import lib
+    if lib.device_count() == 0:
+        pytest.skip('no GPU')
+    f = load_fixture('h2o_vdz')
+    h = f['dm_rand'] + f['dm_rand'].T
+    d = torch.from_numpy(h).cuda()
+    plans = [lib.Plan(f['atm'], f['bas'], f['env'], direct_scf_tol=1e-13) for _ in range(2)]
+    batch = lib.Batch(plans)
+    rj, rk = batch.get_jk_device([d, d])
+    vj, vk = [torch.empty_like(d) for _ in plans], [torch.empty_like(d) for _ in plans]
+    lib.load().b200jk_debug_fail_alloc(nth)
+    try:
+        with pytest.raises(lib.B200JKError) as e:
+            plans[1].get_jk(numpy.array([h, h]), hermi=1)
+        assert e.value.code == lib.B200JK_ENOMEM
+    finally:
+        lib.load().b200jk_debug_fail_alloc(0)
+    with pytest.raises(lib.B200JKError, match='workspace moved') as e:
+        batch.get_jk_device_async([d, d], vj, vk)
+    assert e.value.code == lib.B200JK_EINVAL
+    batch.get_jk_device([d, d])
+    batch.get_jk_device_async([d, d], vj, vk)
+    torch.cuda.synchronize()
+    for got, want in zip(vj + vk, rj + rk):
+        assert float((got - want).abs().max()) < 1e-10
