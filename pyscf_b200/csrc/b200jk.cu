@@ -2618,11 +2618,13 @@ struct b200jk_batch {
         cudaStream_t stream = nullptr;
         cudaEvent_t ev0 = nullptr, ev1 = nullptr;
         DevArr<JKArgs> args;
-        // per entry (a molecule in a class and pass): first segment and class;
-        // per class and pass: what its entries share
+        // per entry (a molecule in a class and pass): first segment, and class and
+        // pass.  All classes' float64 entries come first, then all their float32
+        // ones, so that an entry's place does not depend on a call's precision or
+        // thresholds: a captured build reads the entries of its pass from the
+        // staging at each replay, whatever calls came between
         DevArr<long long> seg0;
         DevArr<int> cls, nkl, kst;
-        DevArr<BatchClass> bc;
         DevArr<long long> nchunk, chunk_off, mchunk;
         DevArr<unsigned char> cub_tmp;
         DevArr<unsigned long long> stats;
@@ -2633,7 +2635,6 @@ struct b200jk_batch {
                 JKArgs *args = nullptr;
                 long long *seg0 = nullptr;
                 int *cls = nullptr;
-                BatchClass *bc = nullptr;
         } staging[2];
         size_t h_cap = 0;               // entries the staging holds
         // what the last synchronous build set up completely (every buffer and
@@ -2656,14 +2657,13 @@ struct b200jk_batch {
                         if (h.args) cudaFreeHost(h.args);
                         if (h.seg0) cudaFreeHost(h.seg0);
                         if (h.cls) cudaFreeHost(h.cls);
-                        if (h.bc) cudaFreeHost(h.bc);
                         h = Staging();
                 }
                 h_cap = 0;
         }
         ~b200jk_batch()
         {
-                args.release(); seg0.release(); cls.release(); bc.release(); nkl.release(); kst.release();
+                args.release(); seg0.release(); cls.release(); nkl.release(); kst.release();
                 nchunk.release(); chunk_off.release(); mchunk.release(); cub_tmp.release(); stats.release();
                 fan.release();
                 free_staging();
@@ -2744,30 +2744,26 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
         }
         auto qcs = quartet_classes();
         const int nclass = (int)qcs.size();
-        // the entries, class-major: the molecules with work in each class, for
-        // the float64 pass and (mixed) the float32 pass.  Buffers are sized for
-        // both passes whatever this call's precision
+        // the entries: the molecules with work in each class, in the float64 pass
+        // and (used by mixed builds) in the float32 pass
         std::vector<size_t> at(2 * nclass, 0);
         std::vector<int> ncnt(nclass, 0);
-        size_t cap = 0, nent = 0;
-        long long cap_segs = 0, nseg = 0;
+        size_t half = 0;
+        long long half_segs = 0;
         for (int t = 0; t < nclass; t++) {
-                long long segs = 0;
+                at[2 * t] = half;
                 for (int m = 0; m < nmol; m++) {
                         const PairClassDev &bra = B->plans[m]->pc[qcs[t].X], &ket = B->plans[m]->pc[qcs[t].Y];
                         if (bra.n == 0 || ket.n == 0) continue;
                         ncnt[t]++;
-                        segs += (long long)bra.n * B2_NBUCKET;
+                        half_segs += (long long)bra.n * B2_NBUCKET;
                 }
-                cap += 2 * (size_t)ncnt[t];
-                cap_segs += 2 * segs;
-                const int np = mixed && class_tau(B->plans[0], t) > 0 ? 2 : 1;
-                for (int pass = 0; pass < np; pass++) {
-                        at[2 * t + pass] = nent;
-                        nent += ncnt[t];
-                        nseg += segs;
-                }
+                half += ncnt[t];
         }
+        for (int t = 0; t < nclass; t++) at[2 * t + 1] = half + at[2 * t];
+        // buffers are sized for both passes whatever this call's precision
+        const size_t cap = 2 * half, nent = mixed ? cap : half;
+        const long long cap_segs = 2 * half_segs, nseg = mixed ? cap_segs : half_segs;
         if (cap_segs + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one batch");
         if (async) {
                 if (cap > B->ready_cap || cap_segs > B->ready_segs)
@@ -2780,13 +2776,12 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                                 CUDA_TRY(cudaMallocHost(&h.args, sizeof(JKArgs) * std::max<size_t>(1, cap)));
                                 CUDA_TRY(cudaMallocHost(&h.seg0, sizeof(long long) * (cap + 1)));
                                 CUDA_TRY(cudaMallocHost(&h.cls, sizeof(int) * std::max<size_t>(1, cap)));
-                                CUDA_TRY(cudaMallocHost(&h.bc, sizeof(BatchClass) * 2 * nclass));
                         }
                         B->h_cap = cap;
                 }
                 const size_t ns = (size_t)std::max(1ll, cap_segs);
                 if ((rc = dev_alloc(B->args, std::max<size_t>(1, cap))) || (rc = dev_alloc(B->seg0, cap + 1)) ||
-                    (rc = dev_alloc(B->cls, std::max<size_t>(1, cap))) || (rc = dev_alloc(B->bc, 2 * nclass)) ||
+                    (rc = dev_alloc(B->cls, std::max<size_t>(1, cap))) ||
                     (rc = dev_alloc(B->nkl, ns)) || (rc = dev_alloc(B->kst, ns)) || (rc = dev_alloc(B->nchunk, ns + 1)) ||
                     (rc = dev_alloc(B->chunk_off, ns + 1)) || (rc = dev_alloc(B->mchunk, cap + 1)) ||
                     (rc = dev_alloc(B->stats, 6 * 64)) || (rc = B->fan.create()))
@@ -2838,70 +2833,68 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
         const double *tbl = B->tbl;
         const float *tbl_f = B->tbl_f;
         // the entries (pointers only depend on the workspaces): fill and upload
-        {
-                long long seg = 0;
+        BatchClasses bc;
+        static_assert(sizeof(bc.c) / sizeof(bc.c[0]) == NPAIRCLASS * (NPAIRCLASS + 1), "an entry per class and pass");
+        memset(&bc, 0, sizeof(bc));
+        long long seg = 0;
+        for (int pass = 0; pass < (mixed ? 2 : 1); pass++)
                 for (int t = 0; t < nclass; t++) {
                         int la, lb, lc, ld;
                         class_l(qcs[t].X, la, lb);
                         class_l(qcs[t].Y, lc, ld);
                         const double tau = mixed ? class_tau(B->plans[0], t) : 0.0;
-                        for (int pass = 0; pass < (tau > 0 ? 2 : 1); pass++) {
-                                // bra runs (variant 2) need the tiled pass of one plan: a batch
-                                // runs those classes as variant 0
-                                int variant = class_variant(B->plans[0], t, pass);
-                                if (variant == 2) variant = 0;
-                                BatchClass &c = h.bc[2 * t + pass];
-                                c.chunk = family_chunk(la, lb, lc, ld, variant);
-                                c.most = family_is_thread(la, lb, lc, ld) ? (variant == 0 ? 5 : 0) : 3;
-                                c.pass = pass;
-                                c.pad = 0;
-                                c.tau = tau;
-                                size_t e = at[2 * t + pass];
-                                for (int m = 0; m < nmol; m++) {
-                                        b200jk_plan *P = B->plans[m];
-                                        const PairClassDev &bra = P->pc[qcs[t].X], &ket = P->pc[qcs[t].Y];
-                                        if (bra.n == 0 || ket.n == 0) continue;
-                                        JKArgs a{};
-                                        a.bra = bra.view();
-                                        a.ket = ket.view();
-                                        a.PP = P->PP.p; a.PK = P->PK.p;
-                                        a.chunk_off = B->chunk_off.p + seg;
-                                        a.nkl = B->nkl.p + seg;
-                                        a.kst = B->kst.p + seg;
-                                        a.dm_cond = P->dm_cond.p;
-                                        a.table = tbl;
-                                        a.table_f = tbl_f;
-                                        a.goff = goff_ptr(t);
-                                        a.Jacc = P->Jacc.p; a.Kacc = P->Kacc.p;
-                                        a.Ds = P->Ds.p; a.Dk = P->Dc.p;
-                                        a.Dpk = P->Dpk.p + P->pk_off[qcs[t].Y];
-                                        a.Jpk = P->Jpk.p + P->pk_off[qcs[t].Y];
-                                        a.pk_stride = P->pk_total;
-                                        a.stats = B->stats.p + 2 * (64 * pass + t);
-                                        a.next = B->stats.p + 4 * 64 + 64 * pass + t;
-                                        a.dmax4 = (const double *)P->dmax.p;
-                                        a.tol = P->tol > 0 ? P->tol : -1.0;
-                                        a.nbas = P->nbas; a.naoc = P->naoc; a.n_dm = 1; a.nk = nk;
-                                        a.with_j = with_j; a.with_k = with_k; a.same = qcs[t].X == qcs[t].Y;
-                                        a.screen = P->screen;
-                                        a.omega2 = P->omega2;
-                                        a.split = 1;
-                                        h.args[e] = a;
-                                        h.seg0[e] = seg;
-                                        h.cls[e] = 2 * t + pass;
-                                        e++;
-                                        seg += (long long)bra.n * B2_NBUCKET;
-                                }
+                        // bra runs (variant 2) need the tiled pass of one plan: a batch
+                        // runs those classes as variant 0
+                        int variant = class_variant(B->plans[0], t, pass);
+                        if (variant == 2) variant = 0;
+                        BatchClass &c = bc.c[2 * t + pass];
+                        c.chunk = pass == 0 || tau > 0 ? family_chunk(la, lb, lc, ld, variant) : 0;
+                        c.most = family_is_thread(la, lb, lc, ld) ? (variant == 0 ? 5 : 0) : 3;
+                        c.pass = pass;
+                        c.tau = tau;
+                        size_t e = at[2 * t + pass];
+                        for (int m = 0; m < nmol; m++) {
+                                b200jk_plan *P = B->plans[m];
+                                const PairClassDev &bra = P->pc[qcs[t].X], &ket = P->pc[qcs[t].Y];
+                                if (bra.n == 0 || ket.n == 0) continue;
+                                JKArgs a{};
+                                a.bra = bra.view();
+                                a.ket = ket.view();
+                                a.PP = P->PP.p; a.PK = P->PK.p;
+                                a.chunk_off = B->chunk_off.p + seg;
+                                a.nkl = B->nkl.p + seg;
+                                a.kst = B->kst.p + seg;
+                                a.dm_cond = P->dm_cond.p;
+                                a.table = tbl;
+                                a.table_f = tbl_f;
+                                a.goff = goff_ptr(t);
+                                a.Jacc = P->Jacc.p; a.Kacc = P->Kacc.p;
+                                a.Ds = P->Ds.p; a.Dk = P->Dc.p;
+                                a.Dpk = P->Dpk.p + P->pk_off[qcs[t].Y];
+                                a.Jpk = P->Jpk.p + P->pk_off[qcs[t].Y];
+                                a.pk_stride = P->pk_total;
+                                a.stats = B->stats.p + 2 * (64 * pass + t);
+                                a.next = B->stats.p + 4 * 64 + 64 * pass + t;
+                                a.dmax4 = (const double *)P->dmax.p;
+                                a.tol = P->tol > 0 ? P->tol : -1.0;
+                                a.nbas = P->nbas; a.naoc = P->naoc; a.n_dm = 1; a.nk = nk;
+                                a.with_j = with_j; a.with_k = with_k; a.same = qcs[t].X == qcs[t].Y;
+                                a.screen = P->screen;
+                                a.omega2 = P->omega2;
+                                a.split = 1;
+                                h.args[e] = a;
+                                h.seg0[e] = seg;
+                                h.cls[e] = 2 * t + pass;
+                                e++;
+                                seg += (long long)bra.n * B2_NBUCKET;
                         }
                 }
-                h.seg0[nent] = seg;
-        }
+        h.seg0[nent] = seg;
         if (nent > 0) {
                 CUDA_TRY(cudaMemcpyAsync(B->args.p, h.args, sizeof(JKArgs) * nent, cudaMemcpyHostToDevice, s));
                 CUDA_TRY(cudaMemcpyAsync(B->seg0.p, h.seg0, sizeof(long long) * (nent + 1), cudaMemcpyHostToDevice, s));
                 CUDA_TRY(cudaMemcpyAsync(B->cls.p, h.cls, sizeof(int) * nent, cudaMemcpyHostToDevice, s));
-                CUDA_TRY(cudaMemcpyAsync(B->bc.p, h.bc, sizeof(BatchClass) * 2 * nclass, cudaMemcpyHostToDevice, s));
-                count_kernel_multi<<<grid_for(nseg, 256), 256, 0, s>>>(B->args.p, B->seg0.p, B->cls.p, B->bc.p, (int)nent,
+                count_kernel_multi<<<grid_for(nseg, 256), 256, 0, s>>>(B->args.p, B->seg0.p, B->cls.p, bc, (int)nent,
                                                                       B->nkl.p, B->kst.p, B->nchunk.p);
                 CUDA_TRY(cudaGetLastError());
                 CUDA_TRY(cudaMemsetAsync(B->nchunk.p + nseg, 0, sizeof(long long), s));

@@ -324,18 +324,23 @@ static __global__ void count_kernel(PairView bra, PairView ket, int same, double
         count_segment(bra, ket, same, tol, *dmax4, chunk, tau32, pass, shard, nshard, t, nkl[t], kst[t], nchunk[t]);
 }
 
-// What one class and pass of a batch shares: chunk length, cut limit of its
-// segments, precision pass, float32 threshold.
+// What one class and pass of a batch shares: chunk length (0: the pass does
+// not run, its segments are empty), cut limit of its segments, precision pass,
+// float32 threshold.  The table travels as a kernel argument, so that a
+// captured build keeps the thresholds it was captured with.
 struct BatchClass {
         int chunk, most, pass, pad;
         double tau;
+};
+struct BatchClasses {
+        BatchClass c[2 * 55];   // [2 * class + pass]
 };
 
 // Count kernel of a batch of molecules, all classes and passes in one launch:
 // entry e (a molecule in a class and pass) owns segments [seg0[e],
 // seg0[e + 1]) of the concatenated nkl/kst/nchunk arrays.
 static __global__ void count_kernel_multi(const JKArgs *__restrict__ margs, const long long *__restrict__ seg0,
-                                          const int *__restrict__ cls, const BatchClass *__restrict__ bc, int nent,
+                                          const int *__restrict__ cls, const __grid_constant__ BatchClasses bc, int nent,
                                           int *nkl, int *kst, long long *nchunk)
 {
         const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -347,8 +352,13 @@ static __global__ void count_kernel_multi(const JKArgs *__restrict__ margs, cons
                 else hi = mid;
         }
         const JKArgs &a = margs[lo];
-        const BatchClass c = bc[cls[lo]];
+        const BatchClass &c = bc.c[cls[lo]];
         const int sgi = (int)(t - seg0[lo]);
+        if (c.chunk == 0) {
+                nkl[t] = kst[t] = 0;
+                nchunk[t] = 0;
+                return;
+        }
         count_segment(a.bra, a.ket, a.same, a.tol > 0 ? a.tol : 0.0, *a.dmax4,
                       c.chunk >> segment_split(a, sgi, c.most), c.tau, c.pass, 0, 1, sgi, nkl[t], kst[t], nchunk[t]);
 }

@@ -95,6 +95,49 @@ def test_batch_cuda_graph(b2):
             assert abs(k.cpu().numpy() - f['vk_' + key]).max() < TOL_JK
 
 
+def test_batch_graph_between_other_calls(b2):
+    """A captured float64 build replays unchanged after an asynchronous mixed
+    build and changed thresholds (both use the same argument staging), and a
+    captured mixed build keeps the thresholds of its capture."""
+    import torch
+    names = ['h2o_vdz', 'h2o8_vdz', 'h2o2_vtz']
+    fs, plans = _plans(b2, names)
+    batch = b2.Batch(plans)
+    dms = [torch.tensor(f['dm_rand'], device='cuda:0') for f in fs]
+    batch.get_jk_device(dms, hermi=1)
+    for captured, other in ((b2.PREC_FP64, b2.PREC_MIXED), (b2.PREC_MIXED, b2.PREC_FP64)):
+        for p in plans:
+            p.set_mixed_threshold(1e-6)
+        vj, vk = [torch.empty_like(d) for d in dms], [torch.empty_like(d) for d in dms]
+        uj, uk = [torch.empty_like(d) for d in dms], [torch.empty_like(d) for d in dms]
+        batch.get_jk_device(dms, hermi=1, precision=captured)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            batch.get_jk_device_async(dms, vj, vk, hermi=1, precision=captured)
+        tau = numpy.zeros(55)
+        tau[::2] = 1e30                    # every other class wholly in float32, the rest not at all
+        for p in plans:
+            p.set_class_thresholds(tau)
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            batch.get_jk_device_async(dms, uj, uk, hermi=1, precision=other)
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        # mixed at 1e-6: the bound of the float32 pass on these molecules
+        tol = TOL_JK if captured == b2.PREC_FP64 else 1e-7
+        for f, j, k in zip(fs, vj, vk):
+            assert abs(j.cpu().numpy() - f['vj_rand']).max() < tol
+            assert abs(k.cpu().numpy() - f['vk_rand']).max() < tol
+        for f, j, k in zip(fs, uj, uk):
+            tol = TOL_JK if other == b2.PREC_FP64 else 2e-5 * abs(f['vj_rand']).max()
+            assert abs(j.cpu().numpy() - f['vj_rand']).max() < tol
+            assert abs(k.cpu().numpy() - f['vk_rand']).max() < tol
+        del g
+
+
 def test_batch512_sample_matches_reference(b2):
     """The 512-molecule batch workload (bench's batch line), built in one
     batched build: 16 sampled molecules against the reference drivers' J/K of
