@@ -134,6 +134,18 @@ def _ptr(a):
     return a.ctypes.data_as(ctypes.c_void_p)
 
 
+# CUDA's handle of the legacy default stream (cudaStreamLegacy)
+_STREAM_LEGACY = 1
+
+
+def _stream(device):
+    """PyTorch's current stream on `device` as the library takes it.  The
+    default stream's handle is NULL, which the C entry points take as the
+    plan's own stream: that one does not wait for the caller's tensors."""
+    import torch
+    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream or _STREAM_LEGACY)
+
+
 class Plan:
     """One molecule/basis on one GPU: shell pairs, primitive pairs and q_cond.
 
@@ -207,8 +219,8 @@ class Plan:
             is_dev = False
         if is_dev:
             d = dm.contiguous()
-            stream = torch.cuda.current_stream(d.device).cuda_stream
-            check(load().b200jk_autotune(self._h, ctypes.c_void_p(d.data_ptr()), 1, ctypes.c_void_p(stream)))
+            stream = _stream(d.device)
+            check(load().b200jk_autotune(self._h, ctypes.c_void_p(d.data_ptr()), 1, stream))
         else:
             d = numpy.ascontiguousarray(dm, dtype=numpy.double)
             check(load().b200jk_autotune(self._h, _ptr(d), 0, None))
@@ -248,9 +260,9 @@ class Plan:
             dev = torch.device('cuda', self.device)
             S = torch.empty((self.nao, self.nao), dtype=torch.float64, device=dev)
             H = torch.empty_like(S)
-            stream = torch.cuda.current_stream(dev).cuda_stream
+            stream = _stream(dev)
             check(load().b200jk_int1e(self._h, ctypes.c_void_p(S.data_ptr()), ctypes.c_void_p(H.data_ptr()), 1,
-                                      ctypes.c_void_p(stream)))
+                                      stream))
             return S, H
         S = numpy.empty((self.nao, self.nao))
         H = numpy.empty((self.nao, self.nao))
@@ -279,8 +291,8 @@ class Plan:
             import torch
             dev = torch.device('cuda', self.device)
             eri = torch.empty(n, dtype=torch.float64, device=dev)
-            stream = torch.cuda.current_stream(dev).cuda_stream
-            check(load().b200jk_int2e_s8(self._h, ctypes.c_void_p(eri.data_ptr()), n, 1, ctypes.c_void_p(stream)))
+            stream = _stream(dev)
+            check(load().b200jk_int2e_s8(self._h, ctypes.c_void_p(eri.data_ptr()), n, 1, stream))
             return eri
         eri = numpy.empty(n)
         check(load().b200jk_int2e_s8(self._h, _ptr(eri), n, 0, None))
@@ -312,9 +324,9 @@ class Plan:
             is_dev = False
         if is_dev:
             d = dm.contiguous()
-            stream = torch.cuda.current_stream(d.device).cuda_stream
+            stream = _stream(d.device)
             check(load().b200jk_autotune_mixed(self._h, ctypes.c_void_p(d.data_ptr()), 1, float(budget), _ptr(res),
-                                               ctypes.c_void_p(stream)))
+                                               stream))
         else:
             d = numpy.ascontiguousarray(dm, dtype=numpy.double)
             check(load().b200jk_autotune_mixed(self._h, _ptr(d), 0, float(budget), _ptr(res), None))
@@ -361,12 +373,12 @@ class Plan:
         n_dm = d.shape[0]
         vj = torch.empty_like(d) if with_j else None
         vk = torch.empty_like(d) if with_k else None
-        stream = torch.cuda.current_stream(d.device).cuda_stream
+        stream = _stream(d.device)
         check(load().b200jk_get_jk(self._h, ctypes.c_void_p(d.data_ptr()), n_dm, int(hermi),
                                    int(bool(with_j)), int(bool(with_k)),
                                    ctypes.c_void_p(vj.data_ptr()) if with_j else None,
                                    ctypes.c_void_p(vk.data_ptr()) if with_k else None,
-                                   1, int(precision), ctypes.c_void_p(stream)))
+                                   1, int(precision), stream))
         return (vj.reshape(shape) if with_j else None), (vk.reshape(shape) if with_k else None)
 
     def grad_jk(self, dms, with_j=True, with_k=True, direct_scf_tol=1e-14):
@@ -396,11 +408,11 @@ class Plan:
         n_dm = d.shape[0]
         vj = torch.empty((n_dm, 3, nao, nao), dtype=torch.float64, device=d.device) if with_j else None
         vk = torch.empty((n_dm, 3, nao, nao), dtype=torch.float64, device=d.device) if with_k else None
-        stream = torch.cuda.current_stream(d.device).cuda_stream
+        stream = _stream(d.device)
         check(load().b200jk_grad_jk(self._h, ctypes.c_void_p(d.data_ptr()), n_dm, int(bool(with_j)),
                                     int(bool(with_k)), ctypes.c_void_p(vj.data_ptr()) if with_j else None,
                                     ctypes.c_void_p(vk.data_ptr()) if with_k else None, 1,
-                                    float(direct_scf_tol), ctypes.c_void_p(stream)))
+                                    float(direct_scf_tol), stream))
         shape = tuple(dms.shape[:-2]) + (3, nao, nao)
         return (vj.reshape(shape) if with_j else None), (vk.reshape(shape) if with_k else None)
 
@@ -419,9 +431,9 @@ class Plan:
             if tuple(d.shape) != (self.nao, self.nao) or d.dtype != torch.float64:
                 raise ValueError('dm must be a float64 (nao, nao) tensor')
             de = torch.empty((natm, 3), dtype=torch.float64, device=d.device)
-            stream = torch.cuda.current_stream(d.device).cuda_stream
+            stream = _stream(d.device)
             check(load().b200jk_grad_contract(self._h, ctypes.c_void_p(d.data_ptr()), ctypes.c_void_p(de.data_ptr()),
-                                              1, float(direct_scf_tol), ctypes.c_void_p(stream)))
+                                              1, float(direct_scf_tol), stream))
             return de
         d = numpy.ascontiguousarray(dm, dtype=numpy.double)
         if d.shape != (self.nao, self.nao):
@@ -482,9 +494,9 @@ class Batch:
         pd = P(*[d.data_ptr() for d in ds])
         pj = P(*[t.data_ptr() for t in vj]) if with_j else None
         pk = P(*[t.data_ptr() for t in vk]) if with_k else None
-        stream = torch.cuda.current_stream(ds[0].device).cuda_stream
+        stream = _stream(ds[0].device)
         check(load().b200jk_batch_get_jk(self._h, pd, int(hermi), int(bool(with_j)), int(bool(with_k)),
-                                         pj, pk, int(precision), ctypes.c_void_p(stream)))
+                                         pj, pk, int(precision), stream))
         return vj, vk
 
     def get_jk_device_async(self, dms, vj, vk, hermi=1, precision=PREC_FP64):
@@ -496,9 +508,9 @@ class Batch:
         pd = P(*[d.data_ptr() for d in dms])
         pj = P(*[t.data_ptr() for t in vj])
         pk = P(*[t.data_ptr() for t in vk])
-        stream = torch.cuda.current_stream(dms[0].device).cuda_stream
+        stream = _stream(dms[0].device)
         check(load().b200jk_batch_get_jk_async(self._h, pd, int(hermi), 1, 1, pj, pk, int(precision),
-                                               ctypes.c_void_p(stream)))
+                                               stream))
 
     def stats(self):
         q, q32, n = ctypes.c_int64(0), ctypes.c_int64(0), ctypes.c_int64(0)
