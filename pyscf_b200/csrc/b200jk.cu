@@ -2853,6 +2853,7 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                         c.pass = pass;
                         c.tau = tau;
                         size_t e = at[2 * t + pass];
+                        const int *goff = goff_ptr(t);   // (a runtime call: once per class, not per molecule)
                         for (int m = 0; m < nmol; m++) {
                                 b200jk_plan *P = B->plans[m];
                                 const PairClassDev &bra = P->pc[qcs[t].X], &ket = P->pc[qcs[t].Y];
@@ -2867,7 +2868,7 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                                 a.dm_cond = P->dm_cond.p;
                                 a.table = tbl;
                                 a.table_f = tbl_f;
-                                a.goff = goff_ptr(t);
+                                a.goff = goff;
                                 a.Jacc = P->Jacc.p; a.Kacc = P->Kacc.p;
                                 a.Ds = P->Ds.p; a.Dk = P->Dc.p;
                                 a.Dpk = P->Dpk.p + P->pk_off[qcs[t].Y];
