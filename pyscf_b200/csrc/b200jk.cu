@@ -17,7 +17,6 @@
 #include <string.h>
 #include <stdio.h>
 #include <math.h>
-#include <limits.h>
 #include <string>
 #include <vector>
 #include <algorithm>
@@ -1632,12 +1631,12 @@ static int ensure_count(b200jk_plan *P, const std::vector<ClassPass> &passes, lo
                         cudaStream_t s)
 {
         int rc;
-        if (nscan + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one build");
-        // (lengths, then starts)
+        // (lengths, then starts; the scans take 64-bit counts: the segments of all
+        // classes may exceed 2^31 where those of each class do not)
         if ((rc = dev_alloc(P->nkl, 2 * (size_t)std::max(1ll, nseg))) || (rc = dev_alloc(P->nchunk, (size_t)nscan + 1)) || (rc = dev_alloc(P->chunk_off, (size_t)nscan + 1)))
                 return rc;
         size_t tmp = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, tmp, P->nchunk.p, P->chunk_off.p, (int)(nscan + 1));
+        cub::DeviceScan::ExclusiveSum(nullptr, tmp, P->nchunk.p, P->chunk_off.p, nscan + 1);
         if ((rc = dev_alloc(P->cub_tmp, tmp + 16))) return rc;
         const bool there = P->cdesc.p && P->h_cdesc.size() == passes.size();
         bool same = there;
@@ -1747,7 +1746,7 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
                         P->shard, P->nshard, P->nkl.p, P->nkl.p + nseg, (unsigned long long *)P->nchunk.p);
                 CUDA_TRY(cudaGetLastError());
                 size_t tmp = P->cub_tmp.n;
-                CUDA_TRY(cub::DeviceScan::ExclusiveSum(P->cub_tmp.p, tmp, P->nchunk.p, P->chunk_off.p, (int)(nscan + 1), s));
+                CUDA_TRY(cub::DeviceScan::ExclusiveSum(P->cub_tmp.p, tmp, P->nchunk.p, P->chunk_off.p, nscan + 1, s));
                 launches++;
         }
         // with class timing on, the classes run one after the other
@@ -2393,7 +2392,6 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
                         nseg_all += (long long)bra.n * B2_NBUCKET;
                         passes.push_back(p);
                 }
-        if (nseg_all + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one build");
         const size_t NQ = NPAIRCLASS * NPAIRCLASS;
         cudaStream_t s = stream ? (cudaStream_t)stream : P->stream;
         if (fused && ((rc = dev_alloc(g.de, (size_t)3 * P->natm)) ||
@@ -2408,7 +2406,7 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
             (rc = dev_alloc(g.cdesc, std::max<size_t>(1, passes.size()))))
                 return rc;
         size_t cub_bytes = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, g.nchunk.p, g.chunk_off.p, (int)(nseg_all + 1));
+        cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, g.nchunk.p, g.chunk_off.p, nseg_all + 1);
         if ((rc = dev_alloc(g.cub_tmp, cub_bytes + 16))) return rc;
         FanLease lease(P->device);
         if ((rc = lease.pool.take(lease.fan))) return rc;
@@ -2462,7 +2460,7 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
                                                                         (unsigned long long *)g.nchunk.p);
                 CUDA_TRY(cudaGetLastError());
                 size_t tmp = g.cub_tmp.n;
-                CUDA_TRY(cub::DeviceScan::ExclusiveSum(g.cub_tmp.p, tmp, g.nchunk.p, g.chunk_off.p, (int)(nseg_all + 1), s));
+                CUDA_TRY(cub::DeviceScan::ExclusiveSum(g.cub_tmp.p, tmp, g.nchunk.p, g.chunk_off.p, nseg_all + 1, s));
                 launches++;
         }
         // with class timing on, the classes run one after the other
@@ -2764,7 +2762,6 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
         // buffers are sized for both passes whatever this call's precision
         const size_t cap = 2 * half, nent = mixed ? cap : half;
         const long long cap_segs = 2 * half_segs, nseg = mixed ? cap_segs : half_segs;
-        if (cap_segs + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one batch");
         if (async) {
                 if (cap > B->ready_cap || cap_segs > B->ready_segs)
                         return fail(B200JK_EINVAL, "b200jk_batch_get_jk_async needs one b200jk_batch_get_jk call first");
@@ -2787,7 +2784,7 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                     (rc = dev_alloc(B->stats, 6 * 64)) || (rc = B->fan.create()))
                         return rc;
                 size_t cub_bytes = 0;
-                cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, B->nchunk.p, B->chunk_off.p, (int)(cap_segs + 1));
+                cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, B->nchunk.p, B->chunk_off.p, cap_segs + 1);
                 if ((rc = dev_alloc(B->cub_tmp, cub_bytes + 16))) return rc;
                 B->ws_gen.resize(nmol);
                 for (int m = 0; m < nmol; m++) B->ws_gen[m] = B->plans[m]->ws_gen;
@@ -2900,7 +2897,7 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                 CUDA_TRY(cudaGetLastError());
                 CUDA_TRY(cudaMemsetAsync(B->nchunk.p + nseg, 0, sizeof(long long), s));
                 size_t tmp = B->cub_tmp.n;
-                CUDA_TRY(cub::DeviceScan::ExclusiveSum(B->cub_tmp.p, tmp, B->nchunk.p, B->chunk_off.p, (int)(nseg + 1), s));
+                CUDA_TRY(cub::DeviceScan::ExclusiveSum(B->cub_tmp.p, tmp, B->nchunk.p, B->chunk_off.p, nseg + 1, s));
                 batch_chunk_starts<<<grid_for((long long)nent + 1, 128), 128, 0, s>>>(B->chunk_off.p, B->seg0.p, (int)nent,
                                                                                     B->mchunk.p);
                 CUDA_TRY(cudaGetLastError());
@@ -3211,14 +3208,13 @@ static int ensure_fill(b200jk_plan *P)
                 if ((rc = upload_pairs(P, P->fill_pc[X], X, h2, q2))) return rc;
                 nseg += h2.size() * B2_NBUCKET * (X + 1);
         }
-        if (nseg + 1 > INT_MAX) return fail(B200JK_EUNSUPPORTED, "too many shell pairs for one fill");
         if ((rc = dev_alloc(P->fill_cdesc, 64)) || (rc = dev_alloc(P->fill_next, 64)) ||
             (rc = dev_upload(P->fill_one, std::vector<double>(1, 1.0), P->stream)) ||
             (rc = dev_alloc(P->fill_nkl, nseg)) || (rc = dev_alloc(P->fill_kst, nseg)) ||
             (rc = dev_alloc(P->fill_nchunk, nseg + 1)) || (rc = dev_alloc(P->fill_chunk_off, nseg + 1)))
                 return rc;
         size_t tmp = 0;
-        CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp, P->fill_nchunk.p, P->fill_chunk_off.p, (int)nseg + 1));
+        CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp, P->fill_nchunk.p, P->fill_chunk_off.p, (long long)nseg + 1));
         if ((rc = dev_alloc(P->fill_cub, std::max<size_t>(tmp, 1)))) return rc;
         CUDA_TRY(cudaStreamSynchronize(P->stream));   // the fill may run on any stream
         P->fill_ready = true;
@@ -3301,7 +3297,7 @@ int b200jk_int2e_s8(b200jk_plan *P, double *eri, long long len, int dev_ptr, voi
                         CUDA_TRY(cudaGetLastError());
                         size_t tb = P->fill_cub.n;
                         CUDA_TRY(cub::DeviceScan::ExclusiveSum(P->fill_cub.p, tb, P->fill_nchunk.p, P->fill_chunk_off.p,
-                                                               (int)(nseg + 1), s));
+                                                               nseg + 1, s));
                 }
                 if ((rc = lanes.fork(s))) return rc;
                 for (const Pass &p : passes) {
