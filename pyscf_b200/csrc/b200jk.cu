@@ -3408,7 +3408,9 @@ int b200jk_incore_jk(const double *eri, long long eri_len, int nao, const double
         const int B = incore_block(nao);
         if (W.items_nao != nao || W.items_s8 != s8) {
                 std::vector<int4> items[4];
-                incore_items(nao, s8, B, items);
+                int nsm = 0;
+                CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+                incore_items(nao, s8, B, nsm, items);
                 W.h_items.clear();
                 for (int v = 0; v < 4; v++) {
                         W.nf[v] = (int)items[v].size();

@@ -345,10 +345,16 @@ int check(const char *what, std::string &err)
         return 1;
 }
 
+// shared memory of a block: two density slabs, the row weights, the ring
+constexpr size_t pass_smem(int B, int nao)
+{
+        return sizeof(double) * (2 * (size_t)B * nao + B * B + (size_t)STAGES * B * NT);
+}
+
 template <int B, bool S8>
 int launch_pass(const IncoreArgs &a, cudaStream_t s, std::string &err)
 {
-        const size_t smem = sizeof(double) * (2 * (size_t)B * a.nao + B * B + (size_t)STAGES * B * NT);
+        const size_t smem = pass_smem(B, a.nao);
         cudaError_t e = cudaFuncSetAttribute(incore_fast_kernel<B, S8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) {
@@ -367,14 +373,16 @@ int launch_pass(const IncoreArgs &a, cudaStream_t s, std::string &err)
 
 // 8 AO rows per block: a lane keeps 4 x B doubles in registers (its J-row
 // image sums and density rows), which B = 8 keeps under the 128 registers of
-// two resident blocks.  nao up to 906 (two density slabs of B x nao doubles
-// beside the 64 KB ring of entries).
+// two resident blocks.  The entry point takes bases of up to 906 functions (a
+// tensor of 675 GB in s8: memory ends earlier); their two density slabs fit a
+// block beside the ring of entries.
+static_assert(pass_smem(8, 906) <= 227 * 1024, "the largest basis fits a block");
 int incore_block(int nao)
 {
         return nao <= 906 ? 8 : 0;
 }
 
-void incore_items(int nao, int s8, int B, std::vector<int4> (&items)[4])
+void incore_items(int nao, int s8, int B, int nsm, std::vector<int4> (&items)[4])
 {
         for (auto &v : items) v.clear();
         const long long npair = (long long)nao * (nao + 1) / 2;
@@ -387,7 +395,7 @@ void incore_items(int nao, int s8, int B, std::vector<int4> (&items)[4])
                         const long long i1 = std::min(nao, (I + 1) * B) - 1;
                         total += s8 ? i1 * (i1 + 1) / 2 + 1 : npair;
                 }
-        const long long want = total / (4 * 148 * NT) * NT;
+        const long long want = total / (4ll * nsm * NT) * NT;
         const long long window = std::min<long long>(2048, std::max<long long>(NT, want));
         auto split = [&](std::vector<int4> &v, int I, int J, long long c0, long long c1) {
                 for (long long c = c0; c < c1; c += window)

@@ -33,8 +33,9 @@ int incore_block(int nao);
 // EDGE + 2 DIAG (DIAG: I == J, else I > J): for s8 the columns before the
 // block's first row (EDGE = 0: no entry there needs a validity test) and the
 // rest (EDGE = 1: q <= p tested per entry, half weight on q == p); for s4
-// every window (EDGE = 0).
-void incore_items(int nao, int s8, int B, std::vector<int4> (&items)[4]);
+// every window (EDGE = 0).  nsm: the device's SM count, which the windows of a
+// small tensor are sized by.
+void incore_items(int nao, int s8, int B, int nsm, std::vector<int4> (&items)[4]);
 
 int launch_incore_pass(const IncoreArgs &a, cudaStream_t s, std::string &err);
 // t = packed D + D^T (diagonal once) of a nao x nao density

@@ -102,7 +102,7 @@ def incore_fits(nao, device=0):
     npair = nao * (nao + 1) // 2
     need = 8 * npair * (npair + 1) // 2
     total = torch.cuda.get_device_properties(device).total_memory
-    return nao <= 880 and need <= INCORE_FRACTION * total
+    return nao <= 906 and need <= INCORE_FRACTION * total
 
 
 def _mol_key(mol):
