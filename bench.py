@@ -718,7 +718,7 @@ def run_gpu(args):
             'quartets_per_build': q_per_build, 'prim_quartets_per_build': _sum_over_ranks(tot['prim_quartets'], dist, dev) / args.steps,
             'fp64_tflops_build': build_flops / (t_total / args.steps) / 1e12 if world == 1 else None,
             'roofline': {'bound': 'fp64', 'kernel': 'jk_%s_kernel<%d,%d,%d,%d>' % (
-                             'thread' if dom['family'] == 0 else 'warp', dom['la'], dom['lb'], dom['lc'], dom['ld']),
+                             ('thread', 'warp', 'row')[dom['family']], dom['la'], dom['lb'], dom['lc'], dom['ld']),
                          'achieved': achieved, 'peak': fp64_peak, 'unit': 'TFLOP/s', 'frac': achieved / fp64_peak,
                          'peak_source': 'measured FP64 FMA loop on this GPU (b200jk_measure_fp64_peak)',
                          'share': dom_ms * 1e-3 / (sum(times) / args.steps), 'traffic': traffic},
@@ -732,7 +732,7 @@ def run_gpu(args):
                     'd2h_bytes_per_step': int(2 * nao * nao * 8),
                     'timing': 'wall clock around pyscf_b200._vhf.direct with pinned host arrays'},
             'classes': [{'class': '(%d%d|%d%d)' % (c['la'], c['lb'], c['lc'], c['ld']),
-                         'family': 'thread' if c['family'] == 0 else 'group',
+                         'family': ('thread', 'group', 'row')[c['family']],
                          'ms_per_build': c['ms'],
                          'share': c['ms'] * 1e-3 / (sum(times) / args.steps),
                          'quartets_per_build': c['quartets'],

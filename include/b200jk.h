@@ -77,7 +77,8 @@ typedef struct {
     int64_t quartets;            /* shell quartets evaluated in the last build */
     int64_t prim_quartets;       /* primitive quartets evaluated in the last build */
     double  ms;                  /* kernel time of the class (profiling on), else 0 */
-    int32_t family;              /* 0 thread-per-quartet, 1 warp-per-quartet */
+    int32_t family;              /* 0 a lane per quartet, 1 lane groups with the block in shared
+                                  * memory, 2 rows (a lane per first index; J/K builds only) */
     int32_t pad;
     int64_t fp32_quartets;       /* of quartets, those evaluated in float32 */
 } b200jk_class_stat_t;

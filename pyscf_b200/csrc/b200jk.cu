@@ -1730,7 +1730,7 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
                         class_l(qcs[t].X, la, lb);
                         class_l(qcs[t].Y, lc, ld);
                         P->cls[t].la = la; P->cls[t].lb = lb; P->cls[t].lc = lc; P->cls[t].ld = ld;
-                        P->cls[t].family = family_is_thread(la, lb, lc, ld) ? 0 : 1;
+                        P->cls[t].family = family_is_thread(la, lb, lc, ld) ? 0 : (family_row_groups(la, lb, lc, ld) ? 2 : 1);
                 }
         }
         if (P->profiling && P->cls_ev.empty()) {

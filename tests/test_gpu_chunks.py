@@ -189,3 +189,19 @@ def test_row_family(b2, nprims, l_of, ncopy, omega):
     for s in range(2):
         rj, rk, _ = oracle.get_jk(d[s], atm, bas, env, hermi=0)
         assert abs(vj[s] - rj).max() < tol and abs(vk[s] - rk).max() < tol
+
+
+def test_class_families(b2):
+    """The class statistics tell the three kernel families apart: by the
+    block's size, lanes (0), rows (2), and shared memory (1) for the six
+    largest classes."""
+    atm, bas, env = contracted_molecule((1, 1, 1, 1), (3, 2, 1, 0), ncopy=2)
+    plan = b2.Plan(atm, bas, env, direct_scf_tol=1e-13)
+    d = densities(plan.nao, 1)[0]
+    plan.get_jk(d + d.T, hermi=1)
+    fam = {(c['la'], c['lb'], c['lc'], c['ld']): c['family'] for c in plan.class_stats()}
+    assert len(fam) == 55
+    assert [fam[k] for k in ((0, 0, 0, 0), (1, 0, 0, 0), (2, 0, 1, 0), (3, 1, 0, 0))] == [0] * 4
+    assert [fam[k] for k in ((1, 1, 1, 1), (2, 1, 2, 0), (2, 2, 2, 1), (3, 2, 2, 2))] == [2] * 4
+    assert sorted(k for k in fam if fam[k] == 1) == [(3, 2, 3, 1), (3, 2, 3, 2), (3, 3, 2, 2), (3, 3, 3, 1),
+                                                      (3, 3, 3, 2), (3, 3, 3, 3)]
