@@ -67,21 +67,30 @@ def test_long_contractions(b2, nprims, l_of, nctr, hermi, n_dm):
 
 
 @pytest.mark.parametrize('tile', [0, 1, 5, 64])
-@pytest.mark.parametrize('precision', [0, 1])
-def test_chunk_orders(b2, tile, precision):
-    """Every tile size, both precisions and a J-only / K-only build give the
-    default order's J and K (mixed: every quartet in float64, tau = 0)."""
+@pytest.mark.parametrize('tau', [0.0, 1e-3, 1e30])
+def test_chunk_orders(b2, tile, tau):
+    """Every tile size, with all quartets in float64, about half of them (by
+    bound) or all in float32 (tau = 0, 1e-3, 1e30), J and K together and
+    alone, against the oracle.  The float32 passes are held to 2e-5 of the
+    largest element, as elsewhere."""
     atm, bas, env = contracted_molecule((1, 3, 9, 1), (1, 0, 0, 2), ncopy=6)
     plan = b2.Plan(atm, bas, env, direct_scf_tol=1e-13)
     d = densities(plan.nao, 1)[0]
     d = d + d.T
-    rj, rk = plan.get_jk(d, hermi=1)
+    rj, rk, _ = oracle.get_jk(d, atm, bas, env, hermi=1)
+    plan.get_jk(d, hermi=1)
     nq = plan.stats()['quartets']
     plan.set_tile(tile)
-    plan.set_mixed_threshold(0.0)
+    plan.set_mixed_threshold(tau)
     for kw in ({}, {'with_k': False}, {'with_j': False}):
-        vj, vk = plan.get_jk(d, hermi=1, precision=precision, **kw)
-        assert plan.stats()['quartets'] == nq
+        vj, vk = plan.get_jk(d, hermi=1, precision=b2.PREC_MIXED, **kw)
+        st = plan.stats()
+        assert st['quartets'] == nq
+        assert (st['fp32_quartets'] == 0) if tau == 0.0 else (st['fp32_quartets'] == nq) if tau > 1.0 \
+            else (nq // 4 < st['fp32_quartets'] < nq - nq // 4)
+        for v, r in ((vj, rj), (vk, rk)):
+            assert v is None or abs(v - r).max() < (TOL if tau == 0.0 else 2e-5 * abs(r).max())
+        vj, vk = plan.get_jk(d, hermi=1, **kw)
         assert vj is None or abs(vj - rj).max() < TOL
         assert vk is None or abs(vk - rk).max() < TOL
 
