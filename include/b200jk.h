@@ -219,7 +219,7 @@ int b200jk_set_profiling(b200jk_plan *plan, int on);
 /* Autotuner: for every quartet class with more than one launch variant (the
  * register family with one or several kets per lane, or bra runs; the shared-memory
  * family with full- or half-width lane groups per quartet; classes of the row
- * family run the same launch as 0 and 1), time each variant
+ * family run the same launch as 0 and 1 and stay at 0), time each variant
  * on FP64 J/K builds of the density dm (nao x nao, symmetric; host array, or
  * device array with dev_ptrs = 1), then the float32 pass's variants on mixed
  * builds at the plan's threshold, and keep the faster for later builds of

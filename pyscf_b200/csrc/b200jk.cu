@@ -2087,6 +2087,7 @@ int b200jk_autotune(b200jk_plan *P, const double *dm, int dev_ptrs, void *stream
                                 class_l(qcs[t].X, la, lb);
                                 class_l(qcs[t].Y, lc, ld);
                                 if (!family_has_variant_n(la, lb, lc, ld, v)) continue;   // no such variant
+                                if (v > 0 && family_row_groups(la, lb, lc, ld) > 0) continue;   // the launch of 0
                                 if (P->cls[t].ms < best_ms[t]) { best_ms[t] = P->cls[t].ms; best[t] = v; }
                         }
                 }

@@ -214,3 +214,16 @@ def test_class_families(b2):
     assert [fam[k] for k in ((1, 1, 1, 1), (2, 1, 2, 0), (2, 2, 2, 1), (3, 2, 2, 2))] == [2] * 4
     assert sorted(k for k in fam if fam[k] == 1) == [(3, 2, 3, 1), (3, 2, 3, 2), (3, 3, 2, 2), (3, 3, 3, 1),
                                                       (3, 3, 3, 2), (3, 3, 3, 3)]
+
+
+def test_autotuner_leaves_rows(b2):
+    """Variants 0 and 1 of a row class are the same launch: the autotuner does
+    not choose between them."""
+    atm, bas, env = contracted_molecule((1, 2, 1, 1), (2, 1, 0, 0), ncopy=4)
+    plan = b2.Plan(atm, bas, env, direct_scf_tol=1e-13)
+    d = densities(plan.nao, 1)[0]
+    for _ in range(3):
+        plan.autotune(d + d.T)
+        for precision in (b2.PREC_FP64, b2.PREC_MIXED):
+            rows = [v for v, c in zip(plan.tuning(precision), plan.class_stats()) if c['family'] == 2]
+            assert len(rows) == 28 and not any(rows)
