@@ -718,7 +718,8 @@ def run_gpu(args):
             'quartets_per_build': q_per_build, 'prim_quartets_per_build': _sum_over_ranks(tot['prim_quartets'], dist, dev) / args.steps,
             'fp64_tflops_build': build_flops / (t_total / args.steps) / 1e12 if world == 1 else None,
             'roofline': {'bound': 'fp64', 'kernel': 'jk_%s_kernel<%d,%d,%d,%d>' % (
-                             ('thread', 'warp', 'row')[dom['family']], dom['la'], dom['lb'], dom['lc'], dom['ld']),
+                             ('thread_run' if tuning[cls.index(dom)] == 2 else 'thread', 'warp', 'row')[dom['family']],
+                             dom['la'], dom['lb'], dom['lc'], dom['ld']),
                          'achieved': achieved, 'peak': fp64_peak, 'unit': 'TFLOP/s', 'frac': achieved / fp64_peak,
                          'peak_source': 'measured FP64 FMA loop on this GPU (b200jk_measure_fp64_peak)',
                          'share': dom_ms * 1e-3 / (sum(times) / args.steps), 'traffic': traffic},

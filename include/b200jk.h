@@ -5,7 +5,10 @@
  * b200jk_last_error() gives a message for the calling thread.  No torch or
  * CUDA types appear in the signatures: densities and outputs are plain
  * double arrays, either host memory or device memory of the plan's GPU
- * (flag dev_ptrs), and a stream is passed as void* (NULL = the plan's own).
+ * (flag dev_ptrs), and a stream is passed as void* (NULL = the plan's own,
+ * which does not wait for work on the legacy default stream: a caller whose
+ * device arrays are written there passes that stream's handle,
+ * cudaStreamLegacy).
  *
  * The entry points replace PySCF 2.12.1's direct-SCF path:
  *

@@ -82,11 +82,13 @@ def _stale(obj, src, flags_file):
 
 
 # blocks per SM the register-family kernels of a quartet class are compiled
-# for (absent: 0, the compiler's own allocation): 4 caps a thread at 128
-# registers, 3 at 168.  Each entry is the faster build of the class on the
-# FP64 build of (H2O)64/cc-pVTZ (class CUDA events, builds compiled with 0,
-# 3 and 4 for every class, launch variants 0 and 2 each, with the part
-# counts below): a few spills buy 12 or 16 resident warps instead of 8.
+# for (absent: 0, the compiler's own allocation): 6 caps a thread at 80
+# registers, 5 at 96, 4 at 128, 3 at 168.  The five classes of RUN_MINB were
+# chosen on the FP64 build of (H2O)16/cc-pVTZ, below; the other entries, and
+# RUN_MINB's, are the faster build of the class on that of (H2O)64/cc-pVTZ
+# (class CUDA events, builds compiled with 0, 3 and 4 for every class, launch
+# variants 0 and 2 each, with the part counts below): a few spills buy 12 or
+# 16 resident warps instead of 8.
 # B2_THREAD_MINB=<n> (every class) or "la lb lc ld:n,..." in the environment
 # overrides it.
 THREAD_MINB = {
@@ -201,8 +203,8 @@ def _source_of(cmd):
 
 
 def _weight(obj):
-    """Rough compile time of a unit: gradient, fill and class units by the
-    angular momenta in their names."""
+    """Rough compile time of a unit, for the order of compilation alone:
+    gradient, fill and class units by the angular momenta in their names."""
     l = sum(int(c) for c in obj if c.isdigit())
     return {'grad': 1000, 'fill': 100, 'b200': 500}.get(obj[:4], 0) + l
 

@@ -611,13 +611,14 @@ static void class_l(int X, int &la, int &lb)
 typedef int (*jk_launcher_t)(const JKArgs &, cudaStream_t, int, int, int, const JKArgs *, const long long *, int,
                              std::string &);
 
-// the launch variant of class t in precision pass `pass` (1: float32 quartets)
 // Launch variant of a float64 pass in a plan the autotuner has not timed:
-// the autotuner's choices on the FP64 build of (H2O)64/cc-pVTZ, where each
-// won by 15-25% per class -- bra runs (2) for eight register-family
+// the autotuner's choices on the FP64 build of (H2O)64/cc-pVTZ before the Rys
+// table was staged free of bank conflicts and classes ran side by side, where
+// each won by 15-25% per class -- bra runs (2) for eight register-family
 // classes of s and p kets, and 1 for (21|20) and (22|10), which chose half-width
 // groups before the row family took them (there 0 and 1 are the same launch).
-// Of (H2O)27/cc-pVTZ the defaults take 946 ms, variant 0 everywhere 975 ms.
+// Of (H2O)27/cc-pVTZ the defaults take 946 ms, variant 0 everywhere 975 ms with
+// the present kernels; of (H2O)64/cc-pVTZ 7.19 s, tuned 7.12 s.
 // Callers that never tune (a drop-in SCF, whose first builds would pay for
 // the timing) get them on plans of DEFAULT_VARIANT_MIN_NAO or more AOs.
 // Smaller plans keep variant 0: bra runs give a warp four bra pairs, too
@@ -1555,8 +1556,8 @@ struct ClassPass {
 };
 
 // How finely the long contractions of a class are cut (split_log2): level 2
-// where the class has fewer quartets than about four per resident lane (2048
-// lanes or 64 lane groups an SM), level 1 otherwise.
+// where the class has fewer quartets than one per resident lane (2048 an SM)
+// or four per lane group (64 an SM), level 1 otherwise.
 static int split_level(const PairClassDev &bra, const PairClassDev &ket, int same, bool thread, int nsm)
 {
         const double nq = same ? 0.5 * bra.n * (bra.n + 1.0) : (double)bra.n * ket.n;
@@ -1633,7 +1634,8 @@ static int ensure_count(b200jk_plan *P, const std::vector<ClassPass> &passes, lo
         int rc;
         // (lengths, then starts; the scans take 64-bit counts: the segments of all
         // classes may exceed 2^31 where those of each class do not)
-        if ((rc = dev_alloc(P->nkl, 2 * (size_t)std::max(1ll, nseg))) || (rc = dev_alloc(P->nchunk, (size_t)nscan + 1)) || (rc = dev_alloc(P->chunk_off, (size_t)nscan + 1)))
+        if ((rc = dev_alloc(P->nkl, 2 * (size_t)std::max(1ll, nseg))) || (rc = dev_alloc(P->nchunk, (size_t)nscan + 1)) ||
+            (rc = dev_alloc(P->chunk_off, (size_t)nscan + 1)))
                 return rc;
         size_t tmp = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, tmp, P->nchunk.p, P->chunk_off.p, nscan + 1);

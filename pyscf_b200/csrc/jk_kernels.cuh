@@ -244,12 +244,12 @@ struct ChunkLoop {
 // every quartet in FP64.  Same-class quartets keep kl <= ij in the
 // (bucket, rank) order.  Sharded over nshard GPUs, rank `shard` takes the bra
 // pairs ij = shard (mod nshard): pairs are sorted by their bound inside a
-// bucket, so striding spreads the cost evenly.
-// Tiled chunk order: tile t gets tile_b x (the most chunks of its bra pairs)
-// chunk slots; slots past a bra pair's own chunks stay idle.
+// bucket, so striding spreads the cost evenly (count_segment, below).
 
 // chunk -> (segment, chunk of the segment, log2 of the segment's cut); the
-// segment's chunks hold chunk_len >> lg quartets.  false for an idle slot.
+// segment's chunks hold chunk_len >> lg quartets.  In the tiled order a tile has
+// tile_b x (the most chunks of its bra pairs) chunk slots; slots past a bra
+// pair's own chunks stay idle: false.
 __device__ __forceinline__ bool map_chunk(const JKArgs &a, long long chunk, int chunk_len, int most, int &sgi, int &kc,
                                           int &lg)
 {

@@ -18,9 +18,10 @@
 //
 // Measured on the FP64 build of (H2O)16/cc-pVTZ against groups with the block
 // in shared memory: (21|20) 25.6 -> 13.2 ms, (21|11) 17.1 -> 7.9, (21|21) 13.4 ->
-// 5.8, (31|21) 10.7 -> 4.3, (22|21) 10.3 -> 5.7, (32|22) 4.5 -> 1.4 ms.  What bounds it now is latency at 8-12 warps per SM: the chain
-// of one primitive quartet (division, root polynomial, recurrence, two passes
-// through shared memory) and the loads of its data.
+// 5.8, (31|21) 10.7 -> 4.3, (22|21) 10.3 -> 5.7, (32|22) 4.5 -> 1.4 ms.  What
+// bounds it now is still the L1 data pipe, 90 % busy in (21|20) on
+// (H2O)9/cc-pVTZ (2.09 ms): shared memory takes 442 M wavefronts, 160 M of them
+// bank conflicts, of the 2D slices and the sums over lanes; FP64 35 %.
 //
 // A warp walks a chunk of one bra pair's kets: its 32 lanes screen 32 kets at
 // once and the groups take the survivors in turn, in step (every loop of the
