@@ -216,18 +216,19 @@ static int dev_alloc(DevArr<T> &d, size_t n)
 
 // Streams the class kernels of one build are spread over: a class of few
 // quartets leaves most SMs idle until its longest chunk ends, so the classes
-// run side by side between a fork from and a join to the caller's stream.
+// run side by side between a fork from and a join to the caller's stream (after
+// the classes that fill the GPU for longer, which run alone: ALONE_US).
 // Kernels of different classes only add to the same accumulators.
 // With one count and scan for all classes and the longest chunks drawn first
 // (ChunkLoop) a build of H2O/cc-pVDZ went from 3.66 to 0.34 ms, (H2O)8/cc-pVDZ
-// 11.5 -> 5.5 ms, (H2O)3/cc-pVTZ with two general densities 22.2 -> 7.3 ms,
-// (H2O)16/cc-pVTZ, which fills the GPU class by class, 405 -> 380 ms.
+// 11.5 -> 5.5 ms, (H2O)3/cc-pVTZ with two general densities 22.2 -> 7.3 ms.
 struct StreamFan {
         static const int N = 7;     // besides the caller's stream
         cudaStream_t st[N] = {};
         cudaEvent_t forked = nullptr, done[N] = {};
         int used = 0;               // lanes of st with work since the fork
         int lane = 0;
+        bool forked_now = false;    // in this build
         bool ready = false;
         int create()
         {
@@ -241,20 +242,21 @@ struct StreamFan {
                 ready = true;
                 return B200JK_OK;
         }
-        int fork(cudaStream_t s)
-        {
-                CUDA_TRY(cudaEventRecord(forked, s));
-                used = 0;
-                lane = 0;
-                return B200JK_OK;
-        }
-        // the next lane in turn (the caller's stream is one of them)
-        int take(cudaStream_t s, cudaStream_t &out)
+        void begin() { used = lane = 0; forked_now = false; }
+        // the stream of the next launch: the caller's for a class that runs alone
+        // (those come first), else the next lane in turn (the caller's stream is
+        // one of them); the first of these forks
+        int next(cudaStream_t s, bool alone, cudaStream_t &out)
         {
                 if (alloc_should_fail()) return fail(B200JK_ECUDA, "lane of a stream set failed (test hook)");
+                out = s;
+                if (alone) return B200JK_OK;
+                if (!forked_now) {
+                        CUDA_TRY(cudaEventRecord(forked, s));
+                        forked_now = true;
+                }
                 if (lane == N) {
                         lane = 0;
-                        out = s;
                         return B200JK_OK;
                 }
                 out = st[lane++];
@@ -1553,6 +1555,7 @@ struct ClassPass {
         int pass, variant;
         CountDesc d;
         long long nscan, max_chunk;
+        bool alone;                // by ALONE_US
 };
 
 // How finely the long contractions of a class are cut (split_log2): level 2
@@ -1562,6 +1565,51 @@ static int split_level(const PairClassDev &bra, const PairClassDev &ket, int sam
 {
         const double nq = same ? 0.5 * bra.n * (bra.n + 1.0) : (double)bra.n * ket.n;
         return nq < 4.0 * nsm * (thread ? 512 : 64) ? 2 : 1;
+}
+
+// A class's time on the whole GPU in microseconds, from its pairs before
+// screening: (8 + 1.2 NR NG) ps per primitive quartet, measured within a factor
+// of 1.6 over the classes of (H2O)16/cc-pVDZ in FP64 (NR roots, NG Cartesian
+// components), with the buckets' typical primitive pairs.
+static double class_us(const PairClassDev &bra, const PairClassDev &ket, int same, int nsm)
+{
+        static const double prims[B2_NBUCKET] = {1, 3, 9, 30};
+        double pb = 0, pk = 0;
+        for (int b = 0; b < B2_NBUCKET; b++) {
+                pb += prims[b] * (bra.boff[b + 1] - bra.boff[b]);
+                pk += prims[b] * (ket.boff[b + 1] - ket.boff[b]);
+        }
+        const int nr = (bra.la + bra.lb + ket.la + ket.lb) / 2 + 1;
+        const double ng = (double)ncart(bra.la) * ncart(bra.lb) * ncart(ket.la) * ncart(ket.lb);
+        return (same ? 0.5 : 1.0) * pb * pk * (8.0 + 1.2 * nr * ng) * 1e-6 * 148 / nsm;
+}
+
+// Classes of at least this estimate run alone, one after the other, before the
+// others run side by side.  A class's grid is sized for the whole GPU and its
+// blocks hold their SMs until the class's queue is empty: classes that start
+// together each get a part of the SMs, and the last of them end on a part of
+// the GPU.  With classes of a millisecond and more that costs more than the
+// tails it fills.  Measured, this line / all side by side / all one after the
+// other (ms): (H2O)8/cc-pVDZ 4.2 / 4.2 / 4.8 (no class reaches it),
+// (H2O)13/cc-pVDZ 10.2 / 11.5 / 10.9, (H2O)20/cc-pVDZ 36.2 / 41.4 / 36.3,
+// (H2O)8/cc-pVTZ 39.8 / 40.1 / 40.8, (H2O)16/cc-pVTZ 227 / 239 / 228,
+// (H2O)27/cc-pVTZ 945 / 964-1005 / 945; with the line at 500, (H2O)5/cc-pVTZ
+// takes 9.9 instead of 9.5.  A batch's classes count over its molecules: 30
+// molecules of up to 16 waters in cc-pVDZ 179 / 213 ms.  The gradient's classes
+// cost more per primitive quartet: gradient J/K of (H2O)9/cc-pVDZ 46.3 / 46.7 /
+// 48.1, (H2O)16/cc-pVDZ 278 / 286 / 280, (H2O)24/cc-pVDZ 875 / 908.  The fill,
+// of small groups with their own chunk rows, gains nothing by it (14 waters
+// in cc-pVDZ 72.6 / 73.3 / 72.8).
+static constexpr double ALONE_US = 2000, GRAD_ALONE_US = 1000;
+
+// the order a build launches its passes in: as listed, or (fan) the ones that
+// run alone first
+static std::vector<size_t> launch_order(const std::vector<char> &alone, bool fan)
+{
+        std::vector<size_t> v(alone.size());
+        std::iota(v.begin(), v.end(), 0);
+        if (fan) std::stable_partition(v.begin(), v.end(), [&](size_t i) { return alone[i] != 0; });
+        return v;
 }
 
 // The passes of a build with work, their segment ranges and chunk bounds.
@@ -1609,6 +1657,7 @@ static std::vector<ClassPass> class_passes(const b200jk_plan *P, int mixed, int 
                         d.tile_b = P->tile_b;
                         d.ntb = (bra.n + P->tile_b - 1) / std::max(1, P->tile_b);
                         d.nslot = c.variant == 2 ? P->tile_b / brun : P->tile_b;
+                        c.alone = class_us(bra, ket, d.same, P->nsm) >= ALONE_US;
                         d.seg0 = nseg;
                         d.scan0 = nscan;
                         c.nscan = tiled ? (long long)B2_NBUCKET * d.ntb : (long long)bra.n * B2_NBUCKET;
@@ -1753,8 +1802,10 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
         }
         // with class timing on, the classes run one after the other
         const bool fan = !P->profiling;
-        if (fan && (rc = lanes.fork(s))) return rc;
-        for (size_t i = 0; i < passes.size(); i++) {
+        std::vector<char> alone;
+        for (const ClassPass &c : passes) alone.push_back(c.alone);
+        lanes.begin();
+        for (size_t i : launch_order(alone, fan)) {
                 const ClassPass &c = passes[i];
                 const size_t t = c.t;
                 const PairClassDev &bra = P->pc[qcs[t].X], &ket = P->pc[qcs[t].Y];
@@ -1789,7 +1840,7 @@ int b200jk_get_jk(b200jk_plan *P, const double *dms, int n_dm, int hermi, int wi
                 a.screen = P->screen;
                 a.omega2 = P->omega2;
                 cudaStream_t cs = s;
-                if (fan && (rc = lanes.take(s, cs))) return rc;
+                if (fan && (rc = lanes.next(s, c.alone, cs))) return rc;
                 if ((rc = dispatch_jk(P, bra.la, bra.lb, ket.la, ket.lb, a, c.pass, cs, nullptr, nullptr, 0, c.variant)))
                         return rc;
                 launches++;
@@ -2369,6 +2420,7 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
                 long long max_chunk;
         };
         std::vector<Pass> passes;
+        std::vector<char> alone;
         long long nseg_all = 0;
         for (int X = 0; X < NPAIRCLASS; X++)
                 for (int Y = 0; Y < NPAIRCLASS; Y++) {
@@ -2377,6 +2429,7 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
                         Pass p;
                         p.X = X;
                         p.Y = Y;
+                        alone.push_back(class_us(bra, ket, 0, P->nsm) >= GRAD_ALONE_US);
                         CountDesc &d = p.d;
                         memset(&d, 0, sizeof(d));
                         d.bra = bra.view();
@@ -2468,8 +2521,9 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
         }
         // with class timing on, the classes run one after the other
         const bool fan = !P->profiling;
-        if (fan && (rc = lanes.fork(s))) return rc;
-        for (const Pass &p : passes) {
+        lanes.begin();
+        for (size_t i : launch_order(alone, fan)) {
+                const Pass &p = passes[i];
                 const PairClassDev &bra = g.bra[p.X], &ket = g.ket[p.Y];
                 const int t = p.X * NPAIRCLASS + p.Y;
                 GradArgs a;
@@ -2498,7 +2552,7 @@ static int grad_build(b200jk_plan *P, const double *dms, int n_dm, int with_j, i
                 a.shell_atom = fused ? g.shell_atom.p : nullptr;
                 std::string err;
                 cudaStream_t cs = s;
-                if (fan && (rc = lanes.take(s, cs))) return rc;
+                if (fan && (rc = lanes.next(s, alone[i], cs))) return rc;
                 if (P->profiling) CUDA_TRY(cudaEventRecord(g.cls_ev[2 * t], s));
                 if (g_grad_launch[p.X](ket.la, ket.lb, a, cs, P->nsm, err)) return fail(B200JK_ECUDA, err);
                 if (P->profiling) CUDA_TRY(cudaEventRecord(g.cls_ev[2 * t + 1], s));
@@ -2905,26 +2959,39 @@ static int batch_build(b200jk_batch *B, const double *const *dms, int hermi, int
                                                                                     B->mchunk.p);
                 CUDA_TRY(cudaGetLastError());
                 launches += 2;
-                if ((rc = B->fan.fork(s))) return rc;
+                struct Pass {
+                        int t, pass;
+                };
+                std::vector<Pass> passes;
+                std::vector<char> alone;
                 for (int t = 0; t < nclass; t++) {
                         if (ncnt[t] == 0) continue;
-                        int la, lb, lc, ld;
-                        class_l(qcs[t].X, la, lb);
-                        class_l(qcs[t].Y, lc, ld);
-                        const double tau = mixed ? class_tau(B->plans[0], t) : 0.0;
-                        for (int pass = 0; pass < (tau > 0 ? 2 : 1); pass++) {
-                                int variant = class_variant(B->plans[0], t, pass);
-                                if (variant == 2) variant = 0;
-                                const size_t e = at[2 * t + pass];
-                                cudaStream_t cs = s;
-                                if ((rc = B->fan.take(s, cs)) ||
-                                    (rc = dispatch_jk(B->plans[0], la, lb, lc, ld, h.args[e], pass, cs, B->args.p + e,
-                                                      B->mchunk.p + e, ncnt[t], variant))) {
-                                        B->fan.join(s);
-                                        return rc;
-                                }
-                                launches++;
+                        double us = 0;
+                        for (const b200jk_plan *P : B->plans)
+                                us += class_us(P->pc[qcs[t].X], P->pc[qcs[t].Y], qcs[t].X == qcs[t].Y, B->nsm);
+                        const int np = mixed && class_tau(B->plans[0], t) > 0 ? 2 : 1;
+                        for (int pass = 0; pass < np; pass++) {
+                                passes.push_back({t, pass});
+                                alone.push_back(us >= ALONE_US);
                         }
+                }
+                B->fan.begin();
+                for (size_t i : launch_order(alone, true)) {
+                        const Pass &p = passes[i];
+                        int la, lb, lc, ld;
+                        class_l(qcs[p.t].X, la, lb);
+                        class_l(qcs[p.t].Y, lc, ld);
+                        int variant = class_variant(B->plans[0], p.t, p.pass);
+                        if (variant == 2) variant = 0;
+                        const size_t e = at[2 * p.t + p.pass];
+                        cudaStream_t cs = s;
+                        if ((rc = B->fan.next(s, alone[i], cs)) ||
+                            (rc = dispatch_jk(B->plans[0], la, lb, lc, ld, h.args[e], p.pass, cs, B->args.p + e,
+                                              B->mchunk.p + e, ncnt[p.t], variant))) {
+                                B->fan.join(s);
+                                return rc;
+                        }
+                        launches++;
                 }
                 if ((rc = B->fan.join(s))) return rc;
         }
@@ -3302,7 +3369,7 @@ int b200jk_int2e_s8(b200jk_plan *P, double *eri, long long len, int dev_ptr, voi
                         CUDA_TRY(cub::DeviceScan::ExclusiveSum(P->fill_cub.p, tb, P->fill_nchunk.p, P->fill_chunk_off.p,
                                                                nseg + 1, s));
                 }
-                if ((rc = lanes.fork(s))) return rc;
+                lanes.begin();
                 for (const Pass &p : passes) {
                         const size_t t = p.t;
                         const PairClassDev &bra = P->fill_pc[qcs[t].X], &ket = P->fill_pc[qcs[t].Y];
@@ -3331,7 +3398,7 @@ int b200jk_int2e_s8(b200jk_plan *P, double *eri, long long len, int dev_ptr, voi
                         f.eri = out;
                         std::string err;
                         cudaStream_t cs = s;
-                        if ((rc = lanes.take(s, cs))) return rc;
+                        if ((rc = lanes.next(s, false, cs))) return rc;
                         if (g_fill_launch[qcs[t].X](ket.la, ket.lb, f, cs, P->nsm, err)) return fail(B200JK_ECUDA, err);
                 }
                 if ((rc = lanes.join(s))) return rc;

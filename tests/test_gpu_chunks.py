@@ -227,3 +227,36 @@ def test_autotuner_leaves_rows(b2):
         for precision in (b2.PREC_FP64, b2.PREC_MIXED):
             rows = [v for v, c in zip(plan.tuning(precision), plan.class_stats()) if c['family'] == 2]
             assert len(rows) == 28 and not any(rows)
+
+
+def test_classes_alone_and_side_by_side(b2):
+    """A molecule of which some classes run alone, before the others run side
+    by side, against all of them one after the other (class timing on): J/K,
+    mixed, general densities, the gradient, the force, and in a batch with a
+    small molecule.  The same sums in another order: 1e-12 of the largest."""
+    import torch
+    from conftest import load_fixture
+    f, small = load_fixture('c20h42_vdz'), load_fixture('h2o_vdz')
+    p = b2.Plan(f['atm'], f['bas'], f['env'], direct_scf_tol=1e-13)
+    h = densities(p.nao, 1)[0]
+    d, ds = torch.from_numpy(h).cuda(), torch.from_numpy(h + h.T).cuda()
+    calls = [lambda: torch.stack(p.get_jk_device(ds, hermi=1)), lambda: torch.stack(p.get_jk_device(d, hermi=0)),
+             lambda: torch.stack(p.grad_jk_device(ds)), lambda: p.grad_contract(ds)]
+    for call in calls:
+        p.set_profiling(True)
+        want = call()
+        nq = p.stats()['quartets'], p.grad_stats()['quartets']
+        p.set_profiling(False)
+        got = call()
+        assert (p.stats()['quartets'], p.grad_stats()['quartets']) == nq
+        assert float((got - want).abs().max()) < 1e-12 * max(1.0, float(want.abs().max()))
+    q = b2.Plan(small['atm'], small['bas'], small['env'], direct_scf_tol=1e-13)
+    e = densities(q.nao, 1)[0]
+    e = torch.from_numpy(e + e.T).cuda()
+    batch = b2.Batch([p, q])
+    for precision in (b2.PREC_FP64, b2.PREC_MIXED):
+        vj, vk = batch.get_jk_device([ds, e], hermi=1, precision=precision)
+        for m, x, j, k in ((p, ds, vj[0], vk[0]), (q, e, vj[1], vk[1])):
+            rj, rk = m.get_jk_device(x, hermi=1, precision=precision)
+            for got, want in ((j, rj), (k, rk)):
+                assert float((got - want).abs().max()) < 1e-12 * max(1.0, float(want.abs().max()))
