@@ -620,7 +620,7 @@ typedef int (*jk_launcher_t)(const JKArgs &, cudaStream_t, int, int, int, const 
 // classes of s and p kets, and 1 for (21|20) and (22|10), which chose half-width
 // groups before the row family took them (there 0 and 1 are the same launch).
 // Of (H2O)27/cc-pVTZ the defaults take 946 ms, variant 0 everywhere 975 ms with
-// the present kernels; of (H2O)64/cc-pVTZ 7.19 s, tuned 7.12 s.
+// the present kernels; of (H2O)64/cc-pVTZ 7.17 s, tuned 7.12 s.
 // Callers that never tune (a drop-in SCF, whose first builds would pay for
 // the timing) get them on plans of DEFAULT_VARIANT_MIN_NAO or more AOs.
 // Smaller plans keep variant 0: bra runs give a warp four bra pairs, too
