@@ -192,6 +192,7 @@ static int dev_upload(DevArr<T> &d, const std::vector<T> &h, cudaStream_t s)
         d.n = h.size();
         if (d.n == 0) return B200JK_OK;
         if (alloc_should_fail() || cudaMalloc(&d.p, sizeof(T) * d.n) != cudaSuccess) {
+                cudaGetLastError();   // (else the next launch's check would report it)
                 d.p = nullptr;
                 d.n = 0;
                 return fail(B200JK_ENOMEM, "cudaMalloc failed for a plan table");
@@ -207,6 +208,7 @@ static int dev_alloc(DevArr<T> &d, size_t n)
         d.release();
         if (n == 0) return B200JK_OK;
         if (alloc_should_fail() || cudaMalloc(&d.p, sizeof(T) * n) != cudaSuccess) {
+                cudaGetLastError();   // (else the next launch's check would report it)
                 d.p = nullptr;
                 return fail(B200JK_ENOMEM, "cudaMalloc failed for a workspace buffer");
         }

@@ -145,3 +145,31 @@ def test_failed_item_list_of_the_stored_tensor(b2):
     for (eri, d), w in zip(cases, want):
         got = torch.stack(incore.incore(eri, d, hermi=1))
         assert float((got - w).abs().max()) < 1e-12 * float(w.abs().max())
+
+
+def test_refused_allocation_does_not_fail_the_next_call(b2):
+    """An allocation larger than the GPU (the s8 tensor of 760 functions, 335
+    GB, into a host array that is never reached) is B200JK_ENOMEM, and the
+    next build on another plan is not told of it."""
+    import torch
+    n = 760
+    need = (n * (n + 1) // 2) * (n * (n + 1) // 2 + 1) // 2
+    assert 8 * need > torch.cuda.get_device_properties(0).total_memory
+    env = [0.0] * 20
+    atm, bas = [], []
+    for k in range(n):
+        atm.append([1, len(env), 1, len(env) + 3, 0, 0])
+        env += [20.0 * (k % 10), 20.0 * (k // 10 % 10), 20.0 * (k // 100), 0.0]
+    for k in range(n):
+        bas.append([k, 0, 1, 1, 0, len(env), len(env) + 1, 0])
+    env += [1.0, 1.0]
+    big = b2.Plan(numpy.array(atm, dtype=numpy.int32), numpy.array(bas, dtype=numpy.int32), numpy.array(env),
+                  direct_scf_tol=1e-13)
+    f = load_fixture('h2o_vdz')
+    p = b2.Plan(f['atm'], f['bas'], f['env'], direct_scf_tol=1e-13)
+    out = numpy.empty(1)
+    rc = b2.load().b200jk_int2e_s8(big._h, out.ctypes.data_as(ctypes.c_void_p), need, 0, None)
+    assert rc == b2.B200JK_ENOMEM
+    vj, vk = p.get_jk(f['dm_rand'], hermi=1)
+    assert abs(vj - f['vj_rand']).max() < TOL_JK
+    assert abs(vk - f['vk_rand']).max() < TOL_JK
